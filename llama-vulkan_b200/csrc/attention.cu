@@ -112,13 +112,16 @@ __global__ void __launch_bounds__(kAttnThreads) attn_values_kernel(float* __rest
 
 // ---- fused ---------------------------------------------------------------------------------
 
-// Scratch layout (floats): for each (z, h, chunk): kRot partial outputs, then
-// the chunk's running maximum and exp-sum; after all of those one u32 arrival
-// counter per (z, h).
-struct AttnScratch {
-    float* partial;      // [batch][heads][nchunks][kRot + 2]
-    uint32_t* counters;  // [batch][heads]
-};
+// Scratch layout: one u32 arrival counter per (z, h), then (floats) for each (z, h, chunk) kRot partial
+// outputs and the chunk's running maximum and exp-sum.  A session uses one scratch for launches of many batch
+// sizes and contexts and clears it once, so the counters of any launch must never lie where the partial outputs of
+// another one went: they come first, in an area that does not depend on the context and is the same for all
+// batches of up to kCounterBatch rows.
+constexpr uint32_t kCounterBatch = 64;
+
+__host__ __device__ inline size_t attn_counter_words(uint32_t heads, uint32_t batch) {
+    return size_t(heads) * (batch > kCounterBatch ? batch : kCounterBatch);
+}
 
 __host__ __device__ inline size_t attn_partial_floats(uint32_t heads, uint32_t nchunks, uint32_t batch) {
     return size_t(batch) * heads * nchunks * (kRot + 2);
@@ -519,7 +522,7 @@ extern "C" int lv_attn_values(lv_ctx* ctx, float* v_out, const void* v_cache, co
 extern "C" size_t lv_attention_scratch_bytes(uint32_t heads, uint32_t rot, uint32_t max_ctx, uint32_t batch) {
     if (rot != uint32_t(kRot) || heads == 0 || max_ctx == 0 || batch == 0) return 0;
     const uint32_t nchunks = (max_ctx + kAttnChunk - 1) / kAttnChunk;
-    return attn_partial_floats(heads, nchunks, batch) * sizeof(float) + size_t(batch) * heads * sizeof(uint32_t);
+    return attn_partial_floats(heads, nchunks, batch) * sizeof(float) + attn_counter_words(heads, batch) * sizeof(uint32_t);
 }
 
 extern "C" int lv_attention_fused(lv_ctx* ctx, float* out, const float* q, const void* k_cache, const void* v_cache,
@@ -529,8 +532,8 @@ extern "C" int lv_attention_fused(lv_ctx* ctx, float* out, const float* q, const
     LV_REQUIRE(out && q && k_cache && v_cache && pos && rope_table && scratch, "null argument");
     if (int rc = check_attn_shape(max_ctx, heads, rot, batch)) return rc;
     const uint32_t nchunks = (max_ctx + kAttnChunk - 1) / kAttnChunk;
-    float* partial = static_cast<float*>(scratch);
-    uint32_t* counters = reinterpret_cast<uint32_t*>(partial + attn_partial_floats(heads, nchunks, batch));
+    uint32_t* counters = static_cast<uint32_t*>(scratch);
+    float* partial = static_cast<float*>(scratch) + attn_counter_words(heads, batch);
     dim3 grid(heads, nchunks, batch);
     if (int rc = launch_attention_fused(ctx, grid, out, q, k_cache, v_cache, pos, rope_table, partial, counters, heads, nchunks, max_ctx, rot)) return rc;
     return LV_OK;
@@ -542,8 +545,8 @@ extern "C" int lv_attention_fused_group(lv_ctx* ctx, float* out, const float* q,
     LV_REQUIRE(out && q && members && rope_table && scratch, "null argument");
     if (int rc = check_attn_shape(max_ctx, heads, rot, n)) return rc;
     const uint32_t nchunks = (max_ctx + kAttnChunk - 1) / kAttnChunk;
-    float* partial = static_cast<float*>(scratch);
-    uint32_t* counters = reinterpret_cast<uint32_t*>(partial + attn_partial_floats(heads, nchunks, n));
+    uint32_t* counters = static_cast<uint32_t*>(scratch);
+    float* partial = static_cast<float*>(scratch) + attn_counter_words(heads, n);
     dim3 grid(heads, nchunks, n);
     return launch_attention_fused(ctx, grid, out, q, nullptr, nullptr, nullptr, rope_table, partial, counters, heads, nchunks, max_ctx, rot, members);
 }
@@ -556,8 +559,9 @@ extern "C" int lv_attention_fused_static(lv_ctx* ctx, float* out, const float* q
     LV_ENTER(ctx);
     LV_REQUIRE(out && q && k_cache && v_cache && pos && rope_table, "null argument");
     if (int rc = check_attn_shape(max_ctx, heads, rot, batch)) return rc;
-    const size_t need = lv_attention_scratch_bytes(heads, rot, max_ctx, batch);
-    if (need == 0 || need > kStaticScratchBytes)
+    // (this buffer's counters are cleared before every launch and follow the partial outputs: no room is kept for other batches)
+    const size_t need = attn_partial_floats(heads, (max_ctx + kAttnChunk - 1) / kAttnChunk, batch) * sizeof(float) + size_t(batch) * heads * sizeof(uint32_t);
+    if (need > kStaticScratchBytes)
         return fail(LV_ERR_BAD_ARGUMENTS, "lv_attention_fused_static: heads x context x batch needs " + std::to_string(need) +
                                               " bytes of scratch, the built-in buffer holds " + std::to_string(kStaticScratchBytes) +
                                               "; use lv_attention_fused with caller-provided scratch");

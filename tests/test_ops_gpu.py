@@ -376,6 +376,31 @@ def test_fused_attention_batch_is_causal(gpu, pkg, rope_table):
         close(got[z], ob.attention(k, v, q[z], pos + z, 128, HEADS, ROT), rel_l2=5e-6, max_abs_frac=2e-5)
 
 
+def test_fused_attention_shares_one_scratch_between_batches_and_contexts(gpu, pkg, rope_table):
+    """A session clears its scratch once and then launches prompt steps of several sizes, single tokens and growing backlogs on it:
+    what the launches with more than one chunk leave there must not reach the arrival counters of the others."""
+    rng = np.random.default_rng(33)
+    k, v = _caches(rng, 1100, 2048)
+    dk, dv = gpu.upload(k), gpu.upload(v)
+    shared = gpu.zeros(gpu.lib.lv_attention_scratch_bytes(HEADS, ROT, 2048, 64))
+    for batch, pos, max_ctx in ((64, 300, 512), (37, 364, 512), (1, 401, 512), (64, 512, 1024), (8, 576, 1024), (5, 584, 1024), (1, 1024, 2048), (2, 1030, 2048)):
+        dq = gpu.upload(rng.standard_normal((batch, DIM)).astype(np.float32))
+        own = gpu.zeros(gpu.lib.lv_attention_scratch_bytes(HEADS, ROT, max_ctx, batch))
+        got = []
+        for scratch in (shared, own):
+            d_out = gpu.alloc(batch * DIM * 4)
+            pkg.check(gpu.lib.lv_memset(gpu.handle, d_out, 0xFF, batch * DIM * 4))
+            pkg.check(gpu.lib.lv_attention_fused(gpu.handle, d_out, dq, dk, dv, u32_dev(gpu, pos), rope_table, scratch, HEADS, ROT, max_ctx, batch))
+            gpu.sync()
+            got.append(gpu.download(d_out, np.float32, batch * DIM))
+            gpu.free(d_out)
+        assert np.array_equal(got[0], got[1]), (batch, pos)
+        gpu.free(dq)
+        gpu.free(own)
+    for d in (dk, dv, shared):
+        gpu.free(d)
+
+
 def test_qkv_fused_writes_cache_rows_and_query(gpu, pkg):
     rng = np.random.default_rng(32)
     ctx_rows, pos, batch = 8, 3, 2
