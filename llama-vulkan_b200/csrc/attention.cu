@@ -406,6 +406,15 @@ int attention_configure(lv_ctx* ctx) {
     return LV_OK;
 }
 
+// Whether lv_attention_fused takes the matrix products of attention_prompt.cu.  Measured on the heads of LLaMA-7B, in a chain of launches,
+// one CTA per row, head and 256 positions here / products there, us:
+//   rows    context 200 of 512    500 of 512    1000 of 1024    1950 of 2048
+//      8           9.4 / 13.8     20.5 / 14.0      36.9 / 15.7      64.1 / 27.3
+//     12          14.2 / 13.9     28.7 / 14.1      50.6 / 16.1      92.3 / 27.9
+//     64          65.7 / 20.8    124.6 / 21.7     237.2 / 24.5     459.6 / 38.0
+// (contexts of up to 128: 8 rows 7.0 / 7.1, 12 rows 10.5 / 7.2, 64 rows 45.6 / 11.7)
+static bool use_prompt_attention(uint32_t batch, uint32_t max_ctx) { return batch >= 12 || (batch >= 8 && max_ctx > 512); }
+
 // Grids of at most one CTA per SM stage key rows and the exact table rows in shared memory; larger
 // ones (context beyond ~1280 rows, batches) stage key rows and the compact table, two CTAs per SM.
 static int launch_attention_fused(lv_ctx* ctx, dim3 grid, float* out, const float* q, const void* k_cache, const void* v_cache,
@@ -531,6 +540,7 @@ extern "C" int lv_attention_fused(lv_ctx* ctx, float* out, const float* q, const
     LV_ENTER(ctx);
     LV_REQUIRE(out && q && k_cache && v_cache && pos && rope_table && scratch, "null argument");
     if (int rc = check_attn_shape(max_ctx, heads, rot, batch)) return rc;
+    if (use_prompt_attention(batch, max_ctx)) return launch_attention_prompt(ctx, out, q, k_cache, v_cache, pos, rope_table, heads, max_ctx, batch);
     const uint32_t nchunks = (max_ctx + kAttnChunk - 1) / kAttnChunk;
     uint32_t* counters = static_cast<uint32_t*>(scratch);
     float* partial = static_cast<float*>(scratch) + attn_counter_words(heads, batch);

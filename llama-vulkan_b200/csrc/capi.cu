@@ -66,6 +66,7 @@ extern "C" int lv_ctx_create(int device, lv_ctx** out) {
     *ctx->h_err = 0;
     int rc = gemv_configure(ctx);
     if (rc == LV_OK) rc = attention_configure(ctx);
+    if (rc == LV_OK) rc = attention_prompt_configure(ctx);
     if (rc == LV_OK) rc = gemm_tc_configure(ctx);
     if (rc == LV_OK) rc = gemm_bf16_configure(ctx);
     if (rc != LV_OK) {

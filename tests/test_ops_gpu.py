@@ -376,6 +376,49 @@ def test_fused_attention_batch_is_causal(gpu, pkg, rope_table):
         close(got[z], ob.attention(k, v, q[z], pos + z, 128, HEADS, ROT), rel_l2=5e-6, max_abs_frac=2e-5)
 
 
+@pytest.mark.parametrize("batch,pos,max_ctx", [(12, 0, 128), (64, 0, 128), (16, 120, 256), (17, 111, 128), (64, 64, 128), (33, 300, 512), (64, 512, 1024), (50, 974, 1024),
+                                               (9, 1015, 2048), (64, 1984, 2048), (63, 1985, 2048), (70, 90, 256), (130, 640, 1024), (12, 19, 31)])
+def test_prompt_attention(gpu, pkg, rope_table, batch, pos, max_ctx):
+    """Steps of many rows go through the matrix products of attention_prompt.cu: chunks of 128 keys that end inside a block of 16, one or
+    several CTAs and passes per head, one or several tiles of 64 rows.  Bounds as for the compact table of test_fused_attention: the angle of
+    a distance of 2000 is an f32 with half an ulp of 2^-14, and the sum of two angles rounds elsewhere than the angle of the sum, which
+    for queries of at most unit size moves scores by about 1e-5."""
+    rng = np.random.default_rng(500 + batch + pos)
+    k, v = _caches(rng, pos + batch, max_ctx)
+    q = (rng.standard_normal((batch, DIM)) * np.exp2(rng.integers(-12, 1, (batch, 1)))).astype(np.float32)
+    q[0, :ROT] = 0                                          # a head's query of zeros weighs its keys equally
+    dk, dv, dq = gpu.upload(k), gpu.upload(v), gpu.upload(q)
+    d_out, scratch = gpu.alloc((batch + 1) * DIM * 4), gpu.zeros(gpu.lib.lv_attention_scratch_bytes(HEADS, ROT, max_ctx, batch))
+    pkg.check(gpu.lib.lv_memset(gpu.handle, d_out, 0xFF, (batch + 1) * DIM * 4))
+    pkg.check(gpu.lib.lv_attention_fused(gpu.handle, d_out, dq, dk, dv, u32_dev(gpu, pos), rope_table, scratch, HEADS, ROT, max_ctx, batch))
+    gpu.sync()
+    got = gpu.download(d_out, np.float32, (batch + 1) * DIM).reshape(batch + 1, DIM)
+    assert np.all(got[batch].view(np.uint32) == 0xFFFFFFFF)
+    backlog = 128
+    while backlog < pos + batch:
+        backlog *= 2
+    for z in sorted({0, 1, 7, min(15, batch - 1), batch // 2, batch - 2, batch - 1}):
+        close(got[z], ob.attention(k, v, q[z], pos + z, backlog, HEADS, ROT), rel_l2=1e-5, max_abs_frac=2e-5)
+    for d in (dk, dv, dq, d_out, scratch):
+        gpu.free(d)
+
+
+def test_prompt_attention_leaves_out_rows_outside_the_cache(gpu, pkg, rope_table):
+    rng = np.random.default_rng(34)
+    batch, pos, max_ctx = 20, 245, 256                      # rows 0 .. 10 lie inside
+    k, v = _caches(rng, max_ctx, max_ctx)
+    q = rng.standard_normal((batch, DIM)).astype(np.float32)
+    d_out, scratch = gpu.alloc(batch * DIM * 4), gpu.zeros(gpu.lib.lv_attention_scratch_bytes(HEADS, ROT, max_ctx, batch))
+    pkg.check(gpu.lib.lv_memset(gpu.handle, d_out, 0xA5, batch * DIM * 4))
+    pkg.check(gpu.lib.lv_attention_fused(gpu.handle, d_out, gpu.upload(q), gpu.upload(k), gpu.upload(v), u32_dev(gpu, pos), rope_table, scratch, HEADS, ROT, max_ctx, batch))
+    with pytest.raises(pkg.LvError) as e:
+        gpu.sync()
+    assert e.value.code == pkg.LV_ERR_DEVICE_WAIT
+    got = gpu.download(d_out, np.float32, batch * DIM).reshape(batch, DIM)
+    close(got[10], ob.attention(k, v, q[10], pos + 10, max_ctx, HEADS, ROT), rel_l2=1e-5, max_abs_frac=2e-5)
+    assert np.all(got[11:].view(np.uint8) == 0xA5)
+
+
 def test_fused_attention_shares_one_scratch_between_batches_and_contexts(gpu, pkg, rope_table):
     """A session clears its scratch once and then launches prompt steps of several sizes, single tokens and growing backlogs on it:
     what the launches with more than one chunk leave there must not reach the arrival counters of the others."""
