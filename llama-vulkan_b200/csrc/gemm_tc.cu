@@ -26,17 +26,16 @@
 // in a scratch buffer; the last to arrive adds them in split order (deterministic) and applies
 // the epilogue.
 //
-// Three forms of the A operand (template parameter FORM; 1 for q4_0 only):
+// Two forms of the A operand here (template parameter FORM; 1 for q4_0 only); the form that is used by default is the
+// kernel of gemm_tc_stream.cu:
 //   exact (FORM = 0)      the hi/lo pair described above, one 64-column tile per producer step;
-//   fast  (FORM = 1, 2)   hi = fp16(w) alone: a weight is rounded to 11 significant bits (relative error <= 2^-12, none
+//   fast  (FORM = 1)      hi = fp16(w) alone: a weight is rounded to 11 significant bits (relative error <= 2^-12, none
 //                         for q4_0 weights with q - 8 in {0, +-1, +-2, +-4, -8}); the activations keep both planes.
 //                         One producer step covers four tiles of K (a whole raw stage): a warp handles 8 rows x 4 tiles,
 //                         so that its 32-bit loads of the 144-byte raw rows and its 16-byte tile stores are free of bank
 //                         conflicts, a thread dequantises the two blocks of one tile of one row, and one MMA per K step
 //                         (W_hi x [x_hi; x_lo]) replaces two.  Any matrix is split along K so that the CTAs fill the SMs
-//                         in whole waves.  Form 1 keeps the tile in shared memory as described; form 2 (the default)
-//                         stores it from the producers' registers into tensor memory and gives it to the MMA as its
-//                         TMEM operand (see the producer branch below).
+//                         in whole waves.
 //
 // Every wait is bounded (common.cuh); a lost wait sets the context's error word, the CTA
 // drains and frees its tensor memory.
@@ -47,16 +46,12 @@
 
 #include "common.cuh"
 #include "ctx.h"
-#include "gemv_stream.cuh"
+#include "gemm_tc.cuh"
 #include "tcgen05.cuh"
 #include "tmap.h"
 
 namespace lv {
 
-constexpr int kTcRows = 128;                   // rows of W per CTA = M of the MMA
-constexpr int kTcMaxZ = 64;                    // tokens per launch = N of the MMA (padded to 16)
-constexpr int kTcChunkK = 64;                  // K per A/B tile: 64 fp16 = one 128-byte swizzle row
-constexpr int kTcRawBlocks = 8;                // q-blocks of a row per raw stage (4 tiles of K)
 constexpr int kTcRawStages = 2;
 constexpr int kTcSlots = 3;
 constexpr int kTcTileBytes = kTcRows * kTcChunkK * 2;                 // 16384: one fp16 plane of A
@@ -65,58 +60,25 @@ constexpr int kTcMaxBStages = 16;
 constexpr int kTcBanks = 2;                    // accumulator sets used in turn, to halve the length of each fp32 chain
 constexpr int kTcProducerWarps = 16;           // two groups of 8: even and odd tiles of K
 constexpr int kTcGroupWarps = 8;
-constexpr int kTcThreads = (kTcProducerWarps + 3) * 32;               // + TMA warp + two MMA warps (the second issues in form 2 only)
+constexpr int kTcThreads = (kTcProducerWarps + 2) * 32;               // + TMA warp + MMA warp
 
-template <int QT> struct TcTraits;
-template <> struct TcTraits<T_Q4_0> {
-    static constexpr int kBlockBytes = kQ4BlockBytes;
-    static constexpr int kBRingBytes = 65536;  // ring of B tiles (hi and lo planes, 2 zpad rows of 128 bytes each)
-};
-template <> struct TcTraits<T_Q8_0> {
-    static constexpr int kBlockBytes = kQ8BlockBytes;
-    static constexpr int kBRingBytes = 49152;  // the raw ring is larger, the B ring shorter
-};
-template <int QT> __host__ __device__ constexpr int tc_raw_row_bytes() { return kTcRawBlocks * TcTraits<QT>::kBlockBytes; }       // 144 / 272
-template <int QT> __host__ __device__ constexpr int tc_raw_stage() { return kTcRows * tc_raw_row_bytes<QT>(); }                   // 18432 / 34816
+template <int QT> struct TcBRing;            // ring of B tiles (hi and lo planes, 2 zpad rows of 128 bytes each)
+template <> struct TcBRing<T_Q4_0> { static constexpr int kBytes = 65536; };
+template <> struct TcBRing<T_Q8_0> { static constexpr int kBytes = 49152; };      // the raw ring is larger, the B ring shorter
 constexpr int kTcFastGroup = 4;                // fast form: tiles of K per producer step (= one raw stage)
 constexpr int kTcFastBufs = 2;
 constexpr int kTcFastBufBytes = kTcFastGroup * kTcTileBytes;          // 65536
 constexpr int kTcFastBRingBytes = 49152;
-// FORM: 0 exact (hi/lo tiles in shared memory), 1 fast (one fp16 plane in shared memory), 2 fast with the weight tile in
-// tensor memory (written by the producers with tcgen05.st and read by the MMA as its TMEM operand: the tile never passes
-// through shared memory, which is what bounds forms 0 and 1; the freed 128 KB hold eight activation stages)
-constexpr int kTcTmemBRingBytes = 131072;
-constexpr int kTcTmemScratchBytes = 8192;      // the epilogue's gate exchange
+// FORM: 0 exact (hi/lo tiles), 1 fast (one fp16 plane)
 template <int QT, int FORM> __host__ __device__ constexpr int tc_a_bytes() {
-    return FORM == 2 ? kTcTmemScratchBytes : (FORM == 1 ? kTcFastBufs * kTcFastBufBytes : kTcSlots * kTcSlotBytes);
+    return FORM == 1 ? kTcFastBufs * kTcFastBufBytes : kTcSlots * kTcSlotBytes;
 }
 template <int QT, int FORM> __host__ __device__ constexpr int tc_b_ring_bytes() {
-    return FORM == 2 ? kTcTmemBRingBytes : (FORM == 1 ? kTcFastBRingBytes : TcTraits<QT>::kBRingBytes);
+    return FORM == 1 ? kTcFastBRingBytes : TcBRing<QT>::kBytes;
 }
 template <int QT, int FORM = 0> __host__ __device__ constexpr size_t tc_smem_bytes() {
     return 1024 /* alignment slack */ + size_t(tc_a_bytes<QT, FORM>()) + tc_b_ring_bytes<QT, FORM>() + size_t(kTcRawStages) * tc_raw_stage<QT>() + 512;
 }
-
-struct GemmTcParams {
-    GemvMatrix m[3];         // same meaning as in the GEMV; w_gate set = SiLU pair (64 + 64 rows per CTA)
-    int n_mat;
-    const uint32_t* pos;     // device word for EPI_STORE_F16_AT_POS
-    uint32_t K;
-    uint32_t Z;              // tokens (columns actually written)
-    uint32_t zpad;           // Z rounded up to 16 = N of the MMA
-    uint32_t ctx_rows;
-    const __half* xh;        // split activations, one contiguous pre-swizzled B tile per 64 columns of K (act_split_kernel)
-    uint32_t splits;         // CTAs that share one tile of rows, each taking a contiguous range of K
-    float* scratch;          // splits > 1: partial accumulators [tile][split][zpad][128]
-    uint32_t* counters;      // splits > 1: arrivals per tile (zero between launches)
-    uint32_t* err;
-    const lv_group_member* group;   // non-null: token z is member z of a group step; cache rows go to its own caches at its own position
-};
-
-struct GemmTcMaps {
-    CUtensorMap w[3];
-    CUtensorMap gate;
-};
 
 // Where the 16-byte chunk `c` (0..7) of row `r` lives inside a swizzled tile.
 __device__ __forceinline__ uint32_t tc_swizzled(uint32_t r, uint32_t c) {
@@ -138,19 +100,6 @@ __device__ __forceinline__ void dequant_word(uint32_t w, __half2 d2, __half2 (&h
     }
 }
 
-// Eight nibbles of one word -> fp16((q - 8) * d), same output order as dequant_word.
-__device__ __forceinline__ void dequant_word_hi(uint32_t w, __half2 d2, uint32_t (&hi)[4]) {
-    const uint32_t v01 = __byte_perm(w, 0u, 0x4140), v23 = __byte_perm(w, 0u, 0x4342);
-    const uint32_t raw[4] = {(v01 & 0x000f000fu) | 0x64006400u, (v23 & 0x000f000fu) | 0x64006400u,
-                             ((v01 >> 4) & 0x000f000fu) | 0x64006400u, ((v23 >> 4) & 0x000f000fu) | 0x64006400u};
-    const __half2 off = __floats2half2_rn(1032.0f, 1032.0f);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const __half2 h = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&raw[i]), off), d2);
-        hi[i] = *reinterpret_cast<const uint32_t*>(&h);
-    }
-}
-
 // Four int8 of one word -> exact (hi, lo) fp16 pairs of q * d: e[0] = elements (4k, 4k+1), e[1] = (4k+2, 4k+3).
 __device__ __forceinline__ void dequant_word_q8(uint32_t w, __half2 d2, __half2 (&hi)[2], __half2 (&lo)[2]) {
     const uint32_t u = w ^ 0x80808080u;                                       // q + 128 as unsigned bytes
@@ -164,21 +113,9 @@ __device__ __forceinline__ void dequant_word_q8(uint32_t w, __half2 d2, __half2 
     }
 }
 
-// Four int8 of one word -> fp16(q * d): out[0] = elements (4k, 4k+1), out[1] = (4k+2, 4k+3).
-__device__ __forceinline__ void dequant_word_q8_hi(uint32_t w, __half2 d2, uint32_t (&out)[2]) {
-    const uint32_t u = w ^ 0x80808080u;                                       // q + 128 as unsigned bytes
-    const uint32_t raw[2] = {__byte_perm(u, 0x64646464u, 0x4140), __byte_perm(u, 0x64646464u, 0x4342)};   // 1024 + 128 + q
-    const __half2 off = __floats2half2_rn(1152.0f, 1152.0f);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const __half2 h = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&raw[i]), off), d2);
-        out[i] = *reinterpret_cast<const uint32_t*>(&h);
-    }
-}
-
 template <int QT, int FORM>
 __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcParams p, const __grid_constant__ GemmTcMaps maps) {
-    constexpr bool FAST = FORM != 0, TMEMA = FORM == 2;
+    constexpr bool FAST = FORM != 0;
     static_assert(FORM != 1 || QT == T_Q4_0, "the shared-memory fast form exists for q4_0 only");
     pdl_launch_dependents();
     extern __shared__ uint8_t smem_raw[];
@@ -222,14 +159,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
     const uint32_t n_chunks = 4 * n_groups;
     const uint32_t b_bytes = 2u * p.zpad * kTcChunkK * 2u;
     uint32_t nb = min(uint32_t(kTcMaxBStages), uint32_t(kBRingBytes) / b_bytes);               // B stages: 3-4 (zpad 64) .. 16
-    if constexpr (FORM == 2) nb &= ~1u;                   // 8 (zpad 64) .. 16, even: see the MMA warps
     // accumulator columns of a bank: [0, zpad) hi*hi, [zpad, 2 zpad) hi*lo, [2 zpad, 3 zpad) lo*hi; two banks;
     // the allocation is a power of two >= 32
     const uint32_t bank_cols = (FAST ? 2u : 3u) * p.zpad;
-    // form 2: accumulators in columns [0, 256), the two weight buffers (4 tiles x 32 columns each) in [256, 512)
-    constexpr uint32_t kTmemABase = 256, kTmemTileCols = kTcChunkK / 2;
-    const uint32_t tmem_cols = TMEMA ? 512u
-                               : (FAST ? (p.zpad <= 16 ? 64u : (p.zpad <= 32 ? 128u : 256u)) : (p.zpad <= 16 ? 128u : (p.zpad <= 32 ? 256u : 512u)));
+    const uint32_t tmem_cols = FAST ? (p.zpad <= 16 ? 64u : (p.zpad <= 32 ? 128u : 256u)) : (p.zpad <= 16 ? 128u : (p.zpad <= 32 ? 256u : 512u));
 
     // one barrier per thread (a single thread takes about a microsecond for all of them)
     if (threadIdx.x < 44) {
@@ -237,7 +170,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
         uint32_t count = 1;                                             // raw_full, slot_empty, acc_full, b_full, b_empty
         if (i >= 2 && i < 4) count = kTcProducerWarps;                  // raw_empty
         else if (i >= 4 && i < 7) count = FAST ? kTcProducerWarps : kTcGroupWarps;      // slot_full
-        else if (TMEMA && i >= 7 && i <= 10) count = 2;                 // slot_empty, acc_full: both MMA-issuing lanes commit
         mbar_init(&bars[i], count);
         fence_mbar_init();
     }
@@ -302,47 +234,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
                 }
             }
         }
-    } else if (warp == kTcProducerWarps + 1 || warp == kTcProducerWarps + 2) {
-        // ---------------- MMA warps: one lane each issues tensor-core work ------------------------
-        // Forms 0 and 1: the first warp issues everything.  Form 2: the issue loop of a single in-order thread (barrier
-        // wait, four MMAs, commit: ~0.25 us per tile) is longer than the producers' step, so two lanes share it: lane 0 of
-        // the first warp takes the even tiles of K into accumulator bank 0, lane 0 of the second the odd ones into bank 1.
-        // That needs an EVEN number of activation stages, so that a stage is always consumed by the same lane: with an odd
-        // number the two lanes would use a stage in turn, and a lane that runs ahead would find its barrier showing the
-        // completed phase of the same parity two uses earlier and take stale data for its tile.
-        const uint32_t issuer = uint32_t(warp) - (kTcProducerWarps + 1);
-        if (lane == 0 && (TMEMA || issuer == 0)) {
+    } else if (warp == kTcProducerWarps + 1) {
+        // ---------------- MMA warp: one lane issues all tensor-core work ---------------------------
+        if (lane == 0) {
             // instruction descriptors: fp32 accumulator, fp16 A and B, both K-major, M = 128, N = 2 zpad / zpad
             const uint32_t idesc_common = (1u << 4) | ((uint32_t(kTcRows) >> 4) << 24);
             const uint32_t idesc_wide = idesc_common | (((2u * p.zpad) >> 3) << 17);
             const uint32_t idesc_narrow = idesc_common | ((p.zpad >> 3) << 17);
             const uint64_t a_desc0 = tc_smem_desc(smem_u32(slots)), b_desc0 = tc_smem_desc(smem_u32(bring));
-            if constexpr (TMEMA) {
-                static_assert(kTcBanks == 2 && kTcFastGroup % 2 == 0, "two issuing lanes, one accumulator bank each");
-                uint32_t bs = issuer, b_phase = 0;             // stage and phase of this lane's next tile (nb is even and >= 2)
-                const uint32_t bank = tmem_base + issuer * bank_cols;
-                bool first = true;
-                for (uint32_t g = 0; g < n_groups && ok; ++g) {
-                    const uint32_t ab = g % kTcFastBufs;
-                    ok = mbar_wait(&slot_full[ab], (g / kTcFastBufs) & 1u, p.err);
-                    uint32_t a_tmem = tmem_base + kTmemABase + (ab * kTcFastGroup + issuer) * kTmemTileCols;
-                    for (uint32_t t = issuer; t < uint32_t(kTcFastGroup) && ok; t += 2) {
-                        ok = mbar_wait(&b_full[bs], b_phase, p.err);
-                        if (!ok) break;
-                        tc_fence_after_sync();
-                        const uint64_t b_desc = b_desc0 + ((bs * b_bytes) >> 4);
-#pragma unroll
-                        for (int k = 0; k < kTcChunkK / 16; ++k)          // 16 fp16 along K = 2 address units of B = 8 TMEM columns of A
-                            tc_mma_f16_ta(bank, a_tmem + 8u * k, b_desc + 2u * k, idesc_wide, (!first || k != 0) ? 1u : 0u);
-                        first = false;
-                        tc_commit(&b_empty[bs]);
-                        a_tmem += 2u * kTmemTileCols;
-                        bs += 2;
-                        if (bs >= nb) { bs -= nb; b_phase ^= 1u; }
-                    }
-                    if (ok) tc_commit(&slot_empty[ab]);
-                }
-            } else
             if constexpr (FAST) {
                 uint32_t bs = 0, b_phase = 0;                  // B stage and its phase, advanced without divisions
                 for (uint32_t g = 0; g < n_groups && ok; ++g) {
@@ -351,7 +250,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
                     // descriptors differ from the first tile's only in the address field (units of 16 bytes; the whole
                     // shared memory stays below the field's 256 KB)
                     uint64_t a_desc = a_desc0 + ((ab * uint32_t(kTcFastBufBytes)) >> 4);
-                    uint32_t a_tmem = tmem_base + kTmemABase + ab * (kTcFastGroup * kTmemTileCols);
                     for (uint32_t t = 0; t < uint32_t(kTcFastGroup) && ok; ++t) {
                         const uint32_t c = g * kTcFastGroup + t;
                         ok = mbar_wait(&b_full[bs], b_phase, p.err);
@@ -360,14 +258,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
                         const uint64_t b_desc = b_desc0 + ((bs * b_bytes) >> 4);
                         const uint32_t bank = tmem_base + (c % kTcBanks) * bank_cols;
 #pragma unroll
-                        for (int k = 0; k < kTcChunkK / 16; ++k) {        // 16 fp16 along K = 32 bytes = 2 address units = 8 TMEM columns
+                        for (int k = 0; k < kTcChunkK / 16; ++k) {        // 16 fp16 along K = 32 bytes = 2 address units
                             const uint32_t acc = (c >= uint32_t(kTcBanks) || k != 0) ? 1u : 0u;
-                            if constexpr (TMEMA) tc_mma_f16_ta(bank, a_tmem + 8u * k, b_desc + 2u * k, idesc_wide, acc);
-                            else tc_mma_f16(bank, a_desc + 2u * k, b_desc + 2u * k, idesc_wide, acc);
+                            tc_mma_f16(bank, a_desc + 2u * k, b_desc + 2u * k, idesc_wide, acc);
                         }
                         tc_commit(&b_empty[bs]);
                         a_desc += uint32_t(kTcTileBytes) >> 4;
-                        a_tmem += kTmemTileCols;
                         if (++bs == nb) { bs = 0; b_phase ^= 1u; }
                     }
                     if (ok) tc_commit(&slot_empty[ab]);
@@ -397,104 +293,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
         }
     } else {
         // ---------------- producer warps: q4_0 blocks -> swizzled fp16 hi/lo tiles ---------------
-        if constexpr (TMEMA) {
-            // A warp can reach only its own quarter of the tensor memory's lanes (32 (warp % 4) ..): lane = tile row.  Warp w
-            // handles rows 32 (w % 4) .. + 31 of tile w / 4 of every raw stage; a thread dequantises the two blocks of its row
-            // into 32 registers (two fp16 each, in element order) and stores them as 32 columns of its lane.
-            const uint32_t tr_row = (uint32_t(warp) & 3u) * 32u + uint32_t(lane), tt = uint32_t(warp) >> 2;
-            for (uint32_t g = 0; g < n_groups && ok; ++g) {
-                const int rs = int(g % kTcRawStages);
-                ok = mbar_wait(&raw_full[rs], (g / kTcRawStages) & 1u, p.err);
-                if (!ok) break;
-                // the tile's two blocks (36 / 68 bytes) start at byte 36 t / 68 t of the raw row: 16-byte loads from the chunk
-                // that holds the first byte (rows are 9 / 17 chunks apart, so a quarter warp's loads fall into different
-                // banks); the tile then starts t words into the loaded words
-                constexpr int kTileWordsQ = kRawRowBytes / 16;                 // words of a tile: 9 / 17
-                constexpr int kLoadChunks = (kTileWordsQ + 3 + 3) / 4;          // 3 / 5
-                uint32_t L[4 * kLoadChunks];
-                {
-                    const uint4* src = reinterpret_cast<const uint4*>(rawring + rs * kRawStage + tr_row * kRawRowBytes) +
-                                       (QT == T_Q4_0 ? 2u : 4u) * tt;
-#pragma unroll
-                    for (int i = 0; i < kLoadChunks; ++i) {
-                        const uint4 v = src[i];
-                        L[4 * i] = v.x; L[4 * i + 1] = v.y; L[4 * i + 2] = v.z; L[4 * i + 3] = v.w;
-                    }
-                }
-                uint32_t w[kTileWordsQ];
-                switch (tt) {                      // (t is the same for the whole warp)
-                    case 0:
-#pragma unroll
-                        for (int i = 0; i < kTileWordsQ; ++i) w[i] = L[i];
-                        break;
-                    case 1:
-#pragma unroll
-                        for (int i = 0; i < kTileWordsQ; ++i) w[i] = L[i + 1];
-                        break;
-                    case 2:
-#pragma unroll
-                        for (int i = 0; i < kTileWordsQ; ++i) w[i] = L[i + 2];
-                        break;
-                    default:
-#pragma unroll
-                        for (int i = 0; i < kTileWordsQ; ++i) w[i] = L[i + 3];
-                        break;
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&raw_empty[rs]);
-                // registers of the row: column j of the tile = elements 2j, 2j + 1 (block 0: columns 0..15, block 1: 16..31)
-                uint32_t cols[32];
-                constexpr int kQW = (kTileWordsQ - 1) / 2;                      // payload words of a block: 4 / 8
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    // block 0: scale in the low half of word 0, payload shifted by two bytes; block 1: scale in the high half
-                    // of the middle word, payload word-aligned
-                    uint32_t q[kQW];
-#pragma unroll
-                    for (int k = 0; k < kQW; ++k) q[k] = b == 0 ? __funnelshift_r(w[k], w[k + 1], 16) : w[kQW + 1 + k];
-                    const uint32_t dbits = b == 0 ? (w[0] & 0xffffu) : (w[kQW] >> 16);
-                    const __half2 d2 = __half2half2(__ushort_as_half(static_cast<unsigned short>(dbits)));
-                    if constexpr (QT == T_Q4_0) {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            uint32_t hi[4];
-                            dequant_word_hi(q[k], d2, hi);          // (4k, 4k+1), (4k+2, 4k+3), (16+4k, 17+4k), (18+4k, 19+4k)
-                            cols[16 * b + 2 * k] = hi[0];
-                            cols[16 * b + 2 * k + 1] = hi[1];
-                            cols[16 * b + 8 + 2 * k] = hi[2];
-                            cols[16 * b + 8 + 2 * k + 1] = hi[3];
-                        }
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) {
-                            uint32_t hi[2];
-                            dequant_word_q8_hi(q[k], d2, hi);       // int8 payload in element order: (4k, 4k+1), (4k+2, 4k+3)
-                            cols[16 * b + 2 * k] = hi[0];
-                            cols[16 * b + 2 * k + 1] = hi[1];
-                        }
-                    }
-                }
-                const uint32_t ab = g % kTcFastBufs;
-                if (g >= uint32_t(kTcFastBufs)) {
-                    ok = mbar_wait(&slot_empty[ab], ((g / kTcFastBufs) - 1) & 1u, p.err);
-                    if (!ok) break;
-                }
-                tc_fence_after_sync();
-                const uint32_t taddr = tmem_base + ((uint32_t(warp) & 3u) * 32u << 16) + kTmemABase + (ab * kTcFastGroup + tt) * kTmemTileCols;
-                asm volatile(
-                    "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-                    "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-                    ::"r"(taddr), "r"(cols[0]), "r"(cols[1]), "r"(cols[2]), "r"(cols[3]), "r"(cols[4]), "r"(cols[5]), "r"(cols[6]), "r"(cols[7]),
-                      "r"(cols[8]), "r"(cols[9]), "r"(cols[10]), "r"(cols[11]), "r"(cols[12]), "r"(cols[13]), "r"(cols[14]), "r"(cols[15]),
-                      "r"(cols[16]), "r"(cols[17]), "r"(cols[18]), "r"(cols[19]), "r"(cols[20]), "r"(cols[21]), "r"(cols[22]), "r"(cols[23]),
-                      "r"(cols[24]), "r"(cols[25]), "r"(cols[26]), "r"(cols[27]), "r"(cols[28]), "r"(cols[29]), "r"(cols[30]), "r"(cols[31])
-                    : "memory");
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&slot_full[ab]);
-            }
-        } else if constexpr (FAST) {
+        if constexpr (FAST) {
             // a warp: 8 rows x the 4 tiles of a raw stage; the word offsets 36 r + 9 t of its lanes fall into 32 different banks
             const uint32_t fr = uint32_t(warp) * 8u + (uint32_t(lane) & 7u), ft = uint32_t(lane) >> 3;
             for (uint32_t g = 0; g < n_groups && ok; ++g) {
@@ -859,9 +658,6 @@ __global__ void __launch_bounds__(512) act_split_kernel(__half* __restrict__ xh,
     }
 }
 
-constexpr size_t kTcScratchBytes = size_t(32) << 20;
-constexpr uint32_t kTcMaxTiles = 1024;
-
 void gemm_tc_release(lv_ctx* ctx) {
     cudaFree(ctx->tc_scratch);
     cudaFree(ctx->tc_counters);
@@ -879,16 +675,10 @@ int gemm_tc_configure(lv_ctx* ctx) {
     LV_REQUIRE(size_t(ctx->max_smem_optin) >= kFastSmem, "device has too little shared memory for the batched product");
     LV_CUDA((cudaFuncSetAttribute(gemm_tc_kernel<T_Q4_0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tc_smem_bytes<T_Q4_0>()))));
     LV_CUDA((cudaFuncSetAttribute(gemm_tc_kernel<T_Q4_0, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFastSmem))));
-    constexpr size_t kTmemSmem = tc_smem_bytes<T_Q4_0, 2>();
-    LV_REQUIRE(size_t(ctx->max_smem_optin) >= kTmemSmem, "device has too little shared memory for the batched product");
-    LV_CUDA((cudaFuncSetAttribute(gemm_tc_kernel<T_Q4_0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmemSmem))));
-    constexpr size_t kTmemSmem8 = tc_smem_bytes<T_Q8_0, 2>();
-    LV_REQUIRE(size_t(ctx->max_smem_optin) >= kTmemSmem8, "device has too little shared memory for the batched product");
-    LV_CUDA((cudaFuncSetAttribute(gemm_tc_kernel<T_Q8_0, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTmemSmem8))));
     LV_CUDA((cudaFuncSetAttribute(gemm_tc_kernel<T_Q8_0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tc_smem_bytes<T_Q8_0>()))));
     const char* exact = getenv("LV_GEMM_TC_EXACT");
     ctx->tc_exact = exact != nullptr && exact[0] == '1';
-    return LV_OK;
+    return gemm_tc_stream_configure(ctx);
 }
 
 template <int QT>
@@ -913,8 +703,13 @@ static int launch_gemm_tc_typed(lv_ctx* ctx, GemmTcParams& p, const __half* xh) 
         if (int rc = make_weight_map(&maps.gate, p.m[0].w_gate, p.m[0].rows, row_bytes, rows_per_cta, tc_raw_row_bytes<QT>())) return rc;
     }
     p.xh = xh;
-    const uint32_t groups_all = p.K / (4 * kTcChunkK);
+    p.scratch = static_cast<float*>(ctx->tc_scratch);
+    p.counters = static_cast<uint32_t*>(ctx->tc_counters);
     const bool fast = !ctx->tc_exact;
+    static const char* smem_tiles = getenv("LV_GEMM_TC_SMEM_TILES");
+    const bool in_smem = QT == T_Q4_0 && smem_tiles != nullptr && smem_tiles[0] == '1';
+    if (fast && !in_smem) return launch_gemm_tc_stream(ctx, p, maps, QT, tiles);
+    const uint32_t groups_all = p.K / (4 * kTcChunkK);
     uint32_t splits = 1;
     auto fits = [&](uint32_t s) {
         return groups_all / s >= 2 && tiles <= kTcMaxTiles && size_t(tiles) * s * p.zpad * kTcRows * sizeof(float) <= kTcScratchBytes;
@@ -935,21 +730,13 @@ static int launch_gemm_tc_typed(lv_ctx* ctx, GemmTcParams& p, const __half* xh) 
     static const char* no_split = getenv("LV_GEMM_TC_NO_SPLIT");
     if (no_split != nullptr && no_split[0] == '1') splits = 1;
     p.splits = splits;
-    p.scratch = static_cast<float*>(ctx->tc_scratch);
-    p.counters = static_cast<uint32_t*>(ctx->tc_counters);
     tiles *= splits;
-    if (fast) {
-        static const char* smem_tiles = getenv("LV_GEMM_TC_SMEM_TILES");
-        if constexpr (QT == T_Q4_0) {
-            if (smem_tiles != nullptr && smem_tiles[0] == '1') {
-                constexpr size_t kFastSmem = tc_smem_bytes<T_Q4_0, 1>();
-                LV_CUDA((launch_pdl(ctx, gemm_tc_kernel<T_Q4_0, 1>, dim3(tiles), dim3(kTcThreads), kFastSmem, p, maps)));
-                return LV_OK;
-            }
+    if constexpr (QT == T_Q4_0) {
+        if (fast) {
+            constexpr size_t kFastSmem = tc_smem_bytes<T_Q4_0, 1>();
+            LV_CUDA((launch_pdl(ctx, gemm_tc_kernel<T_Q4_0, 1>, dim3(tiles), dim3(kTcThreads), kFastSmem, p, maps)));
+            return LV_OK;
         }
-        constexpr size_t kTmemSmem = tc_smem_bytes<QT, 2>();
-        LV_CUDA((launch_pdl(ctx, gemm_tc_kernel<QT, 2>, dim3(tiles), dim3(kTcThreads), kTmemSmem, p, maps)));
-        return LV_OK;
     }
     LV_CUDA((launch_pdl(ctx, gemm_tc_kernel<QT, 0>, dim3(tiles), dim3(kTcThreads), tc_smem_bytes<QT>(), p, maps)));
     return LV_OK;

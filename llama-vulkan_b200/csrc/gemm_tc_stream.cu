@@ -1,0 +1,553 @@
+// Batched products over quantised weights with the weight tiles in tensor memory (the default form of lv_gemm_tc*).
+//
+//   out[z][r] = sum_k W[r][k] * x[z][k]        z < Z <= 64
+//
+// The work is a list of units: tiles of 128 rows (64 + 64 of a SiLU pair) times groups of 256 columns, tile by tile.  A persistent
+// launch of at most one CTA per SM gives every CTA an equal run of consecutive units, wherever tiles begin and end in it: a run is cut
+// into segments, one per tile that it touches.  A segment that covers a whole tile is finished by its CTA; of the others the partial
+// accumulators go to scratch, every CTA reports all of its tiles once at its end, and the last one to report a tile adds the parts
+// in the order of K (deterministic) and applies the epilogue.
+//
+// What bounds it: one CTA per row tile and share of K ran in waves that were filled to 60-80 %, and paid set-up, ring filling and the
+// pass over the parts in every wave; within a wave two raw stages and one barrier hand-over per 64 columns made a group take 1.2 us
+// where the tensor pipe needs 0.5 us (Z = 64) and HBM 0.4 us.  Here those costs are paid once per launch, the weights arrive through four or
+// more raw stages, and activations are handed over 128 columns at a time.
+//
+// Roles (20 warps):
+//   0..15  producers.  A warp reaches only its own quarter of the tensor memory's lanes (= tile rows), so warp w dequantises rows
+//          32 (w % 4) .. + 31 of tile w / 4 of each group: two blocks of a row per thread into 32 registers (fp16 pairs of hi = fp16(w),
+//          11 significant bits), stored with tcgen05.st.  Two such buffers of four 64-column tiles.  The same warps read finished
+//          accumulators back, one unit after the segment's end, so that the last products run while the next unit is prepared.
+//   16     raw ring: 2-D tensor-map loads of q4_0 / q8_0 rows.
+//   17, 18 one lane each issues tcgen05.mma: tiles 0 and 1 of a group into accumulator bank 0, tiles 2 and 3 into bank 1 (two fp32
+//          chains of half the length); N = 2 zpad columns: the activations' hi and lo planes.
+//   19     activation ring: one bulk copy per two tiles of K (q8_0, whose raw stages are larger: one).  The number of stages is even, so that a stage always belongs to one
+//          issuing lane (a parity wait cannot tell a phase from the one two uses later).
+//
+// Every wait is bounded (common.cuh); a lost wait sets the context's error word, the CTA drains and frees its tensor memory.
+#include <cstdlib>
+
+#include "gemm_tc.cuh"
+#include "tcgen05.cuh"
+#include "tmap.h"
+
+namespace lv {
+
+constexpr int kTsProducers = 16;
+constexpr int kTsThreads = (kTsProducers + 4) * 32;
+constexpr int kTsMaxRaw = 8, kTsMaxB = 16;
+constexpr uint32_t kTsABase = 256, kTsTileCols = kTcChunkK / 2;      // tensor memory: accumulators in columns 0..255, weights from 256 on
+constexpr uint32_t kTsGateBytes = kTcMaxZ * 64 * sizeof(float);      // the epilogue's gate exchange
+constexpr uint32_t kTsBarBytes = 512;
+constexpr uint32_t kTsSmemBytes = 227 * 1024;
+// Tiles of K per activation stage: two, where the raw stages leave room for four stages of 64 tokens (32 KB each).
+template <int QT> __host__ __device__ constexpr uint32_t ts_b_tiles() { return QT == T_Q4_0 ? 2u : 1u; }
+
+struct TsPlan {
+    uint32_t units, per;       // units of the launch and of a CTA
+    uint32_t groups;           // units of a tile
+    uint32_t n_raw, n_b;       // stages of the two rings
+};
+
+__device__ __forceinline__ float ts_silu(float up, float gate) { return up * gate / (expf(-gate) + 1.0f); }      // matmul_silu_ff.comp:95
+
+// Where row 0 of token z goes in the f16 cache of matrix mi, or null (reported) beyond its end.
+__device__ __forceinline__ __half* ts_cache_row(const GemmTcParams& p, const GemvMatrix& M, int mi, uint32_t z) {
+    __half* cache = static_cast<__half*>(M.out);
+    uint32_t at;
+    if (p.group != nullptr) {                // matrix 0 is wk, matrix 2 is wv (lv_gemm_tc_qkv_kvappend_group)
+        const lv_group_member& m = p.group[z];
+        cache = static_cast<__half*>(mi == 0 ? m.k_cache : m.v_cache);
+        at = *m.pos;
+    } else {
+        at = *p.pos + z;
+    }
+    if (at < p.ctx_rows) return cache + size_t(at) * M.rows;
+    atomicOr(p.err, ERR_BAD_INDEX);
+    return nullptr;
+}
+
+// Stores one value / four consecutive rows of a token.  (mi: matrix of the launch)
+__device__ __forceinline__ void ts_store(const GemmTcParams& p, const GemvMatrix& M, int mi, uint32_t row, uint32_t z, float v) {
+    if (M.epilogue == EPI_STORE_F16_AT_POS) {
+        if (__half* to = ts_cache_row(p, M, mi, z)) to[row] = __float2half_rn(v);
+    } else {
+        float* o = static_cast<float*>(M.out) + size_t(z) * M.rows + row;
+        *o = (M.epilogue == EPI_ADD) ? (*o + v) : v;                                   // matmul.glsl:68-72
+    }
+}
+__device__ __forceinline__ void ts_store4(const GemmTcParams& p, const GemvMatrix& M, int mi, uint32_t row, uint32_t z, float4 v) {
+    if (M.epilogue == EPI_STORE_F16_AT_POS) {
+        __half* to = ts_cache_row(p, M, mi, z);
+        if (to == nullptr) return;
+        to += row;
+        const __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
+        if ((reinterpret_cast<uintptr_t>(to) & 7u) == 0) {
+            *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        } else {
+            to[0] = a.x; to[1] = a.y; to[2] = b.x; to[3] = b.y;
+        }
+        return;
+    }
+    float* o = static_cast<float*>(M.out) + size_t(z) * M.rows + row;
+    if ((reinterpret_cast<uintptr_t>(o) & 15u) == 0) {
+        float4* o4 = reinterpret_cast<float4*>(o);
+        if (M.epilogue == EPI_ADD) {
+            const float4 x = *o4;
+            v = make_float4(x.x + v.x, x.y + v.y, x.z + v.z, x.w + v.w);
+        }
+        *o4 = v;
+    } else {
+        const float x[4] = {v.x, v.y, v.z, v.w};
+        for (int i = 0; i < 4; ++i) o[i] = (M.epilogue == EPI_ADD) ? (o[i] + x[i]) : x[i];
+    }
+}
+
+// The words of a raw row that tile TT of its group needs, in 16-byte loads: the tile's two blocks (36 / 68 bytes) start at byte 36 TT /
+// 68 TT, in chunk 2 TT / 4 TT and TT words into it.
+template <int QT> __host__ __device__ constexpr int ts_tile_words() { return tc_raw_row_bytes<QT>() / 16; }          // 9 / 17
+template <int QT> __host__ __device__ constexpr int ts_load_chunks() { return (ts_tile_words<QT>() + 3 + 3) / 4; }    // 3 / 5
+
+// Two blocks of a row -> 32 registers in element order (column j = elements 2j, 2j + 1), each fp16(w) with w = (q - 8) d or q d: the
+// quants are widened by placing them in the mantissa of a power of two whose last place is their unit (1024 for the low nibble, 64 for
+// the high one, which so needs no shift), the offset is subtracted exactly and the product rounded once.
+// Block 0: scale in the low half of word 0, payload shifted by two bytes; block 1: scale in the high half of the middle word, payload
+// word-aligned.
+template <int QT, int TT>
+__device__ __forceinline__ void ts_dequant(const uint32_t (&L)[4 * ts_load_chunks<QT>()], uint32_t (&cols)[32]) {
+    constexpr int kQW = (ts_tile_words<QT>() - 1) / 2;                    // payload words of a block: 4 / 8
+    auto product = [](uint32_t bits, __half2 off, __half2 d2) {
+        const __half2 v = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&bits), off), d2);
+        return *reinterpret_cast<const uint32_t*>(&v);
+    };
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+        const uint32_t dbits = b == 0 ? __byte_perm(L[TT], 0u, 0x1010) : __byte_perm(L[TT + kQW], 0u, 0x3232);
+        const __half2 d2 = *reinterpret_cast<const __half2*>(&dbits);
+#pragma unroll
+        for (int k = 0; k < kQW; ++k) {
+            // bytes 0, 1 and 2, 3 of payload word k
+            const uint32_t lo = b == 0 ? L[TT + k] : L[TT + kQW + 1 + k], hi = b == 0 ? L[TT + k + 1] : lo;
+            if constexpr (QT == T_Q4_0) {
+                // low nibbles = elements 4k .. 4k+3, high nibbles = 16 + 4k .. 19 + 4k
+                const uint32_t v01 = __byte_perm(lo, 0u, b == 0 ? 0x4342 : 0x4140), v23 = __byte_perm(hi, 0u, b == 0 ? 0x4140 : 0x4342);
+                const __half2 off_lo = __floats2half2_rn(1032.0f, 1032.0f), off_hi = __floats2half2_rn(72.0f, 72.0f);
+                cols[16 * b + 2 * k] = product((v01 & 0x000f000fu) | 0x64006400u, off_lo, d2);
+                cols[16 * b + 2 * k + 1] = product((v23 & 0x000f000fu) | 0x64006400u, off_lo, d2);
+                cols[16 * b + 8 + 2 * k] = product((v01 & 0x00f000f0u) | 0x54005400u, off_hi, d2);
+                cols[16 * b + 8 + 2 * k + 1] = product((v23 & 0x00f000f0u) | 0x54005400u, off_hi, d2);
+            } else {
+                // int8 in element order; the sign bit is flipped (q + 128) on the way into the mantissa of 1024
+                const uint32_t u01 = __byte_perm(lo, 0x64646464u, b == 0 ? 0x4342 : 0x4140), u23 = __byte_perm(hi, 0x64646464u, b == 0 ? 0x4140 : 0x4342);
+                const __half2 off = __floats2half2_rn(1152.0f, 1152.0f);
+                cols[16 * b + 2 * k] = product(u01 ^ 0x00800080u, off, d2);
+                cols[16 * b + 2 * k + 1] = product(u23 ^ 0x00800080u, off, d2);
+            }
+        }
+    }
+}
+
+template <int QT>
+__global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const GemmTcParams p, const TsPlan plan, const __grid_constant__ GemmTcMaps maps) {
+    pdl_launch_dependents();
+    extern __shared__ uint8_t smem_raw[];
+    // swizzled tiles need 1024-byte alignment
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
+    constexpr int kRawRowBytes = tc_raw_row_bytes<QT>(), kRawStage = tc_raw_stage<QT>();
+    const uint32_t b_tile = 2u * p.zpad * kTcChunkK * 2u;        // bytes of 64 columns of both planes
+    constexpr uint32_t kBT = ts_b_tiles<QT>();
+    const uint32_t b_stage = kBT * b_tile;
+    uint8_t* bring = smem;
+    uint8_t* rawring = bring + plan.n_b * b_stage;
+    float* gate_s = reinterpret_cast<float*>(rawring + plan.n_raw * kRawStage);          // [64 tokens][64 rows]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(gate_s) + kTsGateBytes);
+    uint64_t* raw_full = bars;                              // [8]
+    uint64_t* raw_empty = raw_full + kTsMaxRaw;             // [8]
+    uint64_t* b_full = raw_empty + kTsMaxRaw;               // [16]
+    uint64_t* b_empty = b_full + kTsMaxB;                   // [16]
+    uint64_t* a_full = b_empty + kTsMaxB;                   // [buffer][half]
+    uint64_t* a_empty = a_full + 4;                         // [buffer][half]
+    uint64_t* acc_full = a_empty + 4;
+    uint64_t* acc_empty = acc_full + 1;
+    uint64_t* gate_full = acc_empty + 1;
+    uint64_t* gate_empty = gate_full + 1;
+    constexpr int kBars = 2 * kTsMaxRaw + 2 * kTsMaxB + 12;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kBars);
+    uint32_t* s_last = tmem_slot + 1;                       // [2]
+    static_assert(kBars * 8 + 12 <= int(kTsBarBytes), "barrier area");
+
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool pair = p.m[0].w_gate != nullptr;
+    const uint32_t rows_per_tile = pair ? kTcRows / 2 : kTcRows;
+    const uint32_t t0 = (p.m[0].rows + rows_per_tile - 1) / rows_per_tile;
+    const uint32_t t1 = t0 + (p.n_mat > 1 ? (p.m[1].rows + rows_per_tile - 1) / rows_per_tile : 0);
+    // which matrix a tile belongs to, and its first row there (a last tile may reach past the matrix: the tensor map fills the
+    // missing rows with zero blocks and the epilogue leaves them out)
+    auto matrix_of = [&](uint32_t tile, uint32_t& row0) {
+        const int mi = (p.n_mat > 1 && tile >= t1) ? 2 : (tile >= t0 ? 1 : 0);
+        row0 = (tile - (mi == 2 ? t1 : (mi == 1 ? t0 : 0))) * rows_per_tile;
+        return mi;
+    };
+    const uint32_t G = plan.groups, u0 = blockIdx.x * plan.per, n_units = min(plan.units, u0 + plan.per) - u0;
+    const uint32_t tile0 = u0 / G, g0 = u0 - tile0 * G;     // where this CTA's run begins
+    const uint32_t bank_cols = 2u * p.zpad;
+
+    // one barrier per thread (a single thread takes about a microsecond for all of them)
+    if (threadIdx.x < kBars) {
+        const int i = int(threadIdx.x);
+        uint32_t count = 1;                                                            // raw_full, b_full, b_empty, a_empty
+        if (i >= kTsMaxRaw && i < 2 * kTsMaxRaw) count = kTsProducers;                  // raw_empty
+        else if (i >= 2 * kTsMaxRaw + 2 * kTsMaxB) {
+            const int j = i - 2 * kTsMaxRaw - 2 * kTsMaxB;
+            if (j < 4) count = kTsProducers / 2;                                        // a_full: the eight warps of a half
+            else if (j == 8) count = 2;                                                 // acc_full: both issuing lanes
+            else if (j == 9) count = kTsProducers;                                      // acc_empty
+            else if (j >= 10) count = kTsProducers / 2;                                 // gate_full, gate_empty
+        }
+        mbar_init(&bars[i], count);
+        fence_mbar_init();
+    }
+    if (warp == kTsProducers + 1) tc_alloc(tmem_slot, 512);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    constexpr uint32_t tmem_base = 0;                       // the allocation is all of the tensor memory
+
+    bool ok = true;
+
+    if (warp == kTsProducers) {
+        // ---------------- raw ring: weights do not depend on the previous kernel ----------------
+        if (lane == 0) {
+            uint32_t tile = tile0, g = g0, row0, rs = 0, phase = 1;
+            int mi = matrix_of(tile, row0);
+            for (uint32_t i = 0; i < n_units && ok; ++i) {
+                if (i >= plan.n_raw) ok = mbar_wait(&raw_empty[rs], phase, p.err);
+                if (!ok) break;
+                uint8_t* dst = rawring + rs * kRawStage;
+                const int x = int(g * (kRawRowBytes / 8));
+                mbar_expect_tx(&raw_full[rs], kRawStage);
+                if (pair) {
+                    tma_load_2d_plain(dst, &maps.w[0], x, int(row0), &raw_full[rs]);                                      // w3 rows -> tile rows 0..63
+                    tma_load_2d_plain(dst + (kTcRows / 2) * kRawRowBytes, &maps.gate, x, int(row0), &raw_full[rs]);      // w1 rows -> 64..127
+                } else {
+                    tma_load_2d_plain(dst, mi == 0 ? &maps.w[0] : (mi == 1 ? &maps.w[1] : &maps.w[2]), x, int(row0), &raw_full[rs]);
+                }
+                if (++rs == plan.n_raw) { rs = 0; phase ^= 1u; }
+                if (++g == G) { g = 0; mi = matrix_of(++tile, row0); }
+            }
+        }
+    } else if (warp == kTsProducers + 3) {
+        // ---------------- activation ring -------------------------------------------------------
+        if (lane == 0) {
+            pdl_wait();                                        // the activations come from the previous kernel
+            const uint8_t* xh = reinterpret_cast<const uint8_t*>(p.xh);
+            uint32_t g = g0, bs = 0, phase = 1;
+            constexpr uint32_t kStages = 4 / kBT;              // stages of a unit; consecutive ones belong to the two MMA lanes in turn
+            for (uint32_t i = 0; i < kStages * n_units && ok; ++i) {
+                if (i >= plan.n_b) ok = mbar_wait(&b_empty[bs], phase, p.err);
+                if (!ok) break;
+                const uint32_t j = i % kStages, t = kBT == 2 ? 2 * j : 2 * (j & 1u) + (j >> 1);       // first tile of the stage
+                mbar_expect_tx(&b_full[bs], b_stage);
+                bulk_g2s(bring + bs * b_stage, xh + size_t(4 * g + t) * b_tile, b_stage, &b_full[bs]);
+                if (++bs == plan.n_b) { bs = 0; phase ^= 1u; }
+                if (j + 1 == kStages && ++g == G) g = 0;
+            }
+        }
+    } else if (warp > kTsProducers) {
+        // ---------------- MMA lanes ---------------------------------------------------------------
+        // (the whole warp runs the loop and one elected lane issues: operands that the compiler knows to be the same for the warp
+        // go to the tensor core without a detour through the lanes)
+        const uint32_t h = uint32_t(__shfl_sync(0xffffffffu, warp, 0)) - (kTsProducers + 1);
+        // fp32 accumulator, fp16 A and B, both K-major, M = 128, N = 2 zpad
+        const uint32_t idesc = (1u << 4) | ((uint32_t(kTcRows) >> 4) << 24) | (((2u * p.zpad) >> 3) << 17);
+        const uint64_t b_desc0 = tc_smem_desc(smem_u32(bring));
+        const uint32_t bank = tmem_base + h * bank_cols;
+        uint32_t g = g0, bs = h, b_phase = 0, seg = 0;
+        bool first = true;
+        for (uint32_t i = 0; i < n_units && ok; ++i) {
+            const uint32_t ab = i & 1u;
+            // the accumulators of the previous segment have been read
+            if (first && seg > 0) ok = mbar_wait_warp(acc_empty, (seg - 1) & 1u, p.err);
+            ok = ok && mbar_wait_warp(&a_full[2 * ab + h], (i >> 1) & 1u, p.err);
+            const uint32_t a_tmem = tmem_base + kTsABase + (4u * ab + 2u * h) * kTsTileCols;
+#pragma unroll
+            for (uint32_t st = 0; st < 2 / kBT; ++st) {
+                ok = ok && mbar_wait_warp(&b_full[bs], b_phase, p.err);
+                if (!ok) break;
+                tc_fence_after_sync();
+                const uint64_t b_desc = b_desc0 + ((bs * b_stage) >> 4);
+                if (tc_elect()) {
+#pragma unroll
+                    for (uint32_t t = 0; t < kBT; ++t)
+#pragma unroll
+                        for (int k = 0; k < kTcChunkK / 16; ++k)          // 16 fp16 along K = 2 address units of B = 8 TMEM columns of A
+                            tc_mma_f16_ta(bank, a_tmem + (st + t) * kTsTileCols + 8u * k, b_desc + t * (b_tile >> 4) + 2u * k, idesc,
+                                          (!first || st + t != 0 || k != 0) ? 1u : 0u);
+                    tc_commit(&b_empty[bs]);
+                }
+                __syncwarp();
+                bs += 2;
+                if (bs >= plan.n_b) { bs -= plan.n_b; b_phase ^= 1u; }
+            }
+            if (!ok) break;
+            first = ++g == G || i + 1 == n_units;
+            if (tc_elect()) {
+                tc_commit(&a_empty[2 * ab + h]);
+                if (first) tc_commit(acc_full);
+            }
+            __syncwarp();
+            if (first) {
+                g = 0;
+                ++seg;
+            }
+        }
+    } else {
+        // ---------------- producers ---------------------------------------------------------------
+        const uint32_t quarter = uint32_t(warp) & 3u, tt = uint32_t(warp) >> 2, half = tt >> 1;
+        const uint32_t tr = quarter * 32u + uint32_t(lane);             // tile row
+        const uint32_t lanes_at = (quarter * 32u) << 16;
+
+        uint32_t n_pairs = 0;
+        // reads the accumulators of segment `seg` (16 tokens per warp) and stores or parks them
+        auto drain = [&](uint32_t seg, uint32_t tile, bool whole, uint32_t slot) {
+            ok = mbar_wait_warp(acc_full, seg & 1u, p.err);
+            if (!ok) return;
+            tc_fence_after_sync();
+            const uint32_t z0 = 16u * tt;
+            float v[16];
+            if (z0 < p.zpad) {
+                uint32_t a[16], b[16];
+                tc_load16(a, tmem_base + lanes_at + z0);
+                tc_load16(b, tmem_base + lanes_at + p.zpad + z0);
+                tc_wait_load();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(b[i]) + __uint_as_float(a[i]);      // the small terms first
+                tc_load16(a, tmem_base + lanes_at + bank_cols + z0);
+                tc_load16(b, tmem_base + lanes_at + bank_cols + p.zpad + z0);
+                tc_wait_load();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] += __uint_as_float(b[i]) + __uint_as_float(a[i]);
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty);
+            pdl_wait();                                        // (outputs may still be read by the previous kernel)
+            if (!whole) {
+                if (z0 < p.zpad) {
+                    float* part = p.scratch + (size_t(2 * blockIdx.x + slot) * p.zpad + z0) * kTcRows + tr;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) __stcg(part + size_t(i) * kTcRows, v[i]);
+                }
+                return;
+            }
+            uint32_t row0;
+            const int mi = matrix_of(tile, row0);
+            const GemvMatrix& M = p.m[mi];
+            if (pair) {
+                // tile rows 64..127 carry the gate (w1) of rows 0..63
+                if (quarter >= 2 && n_pairs > 0) ok = mbar_wait_warp(gate_empty, (n_pairs - 1) & 1u, p.err);
+                if (tr >= 64 && z0 < p.zpad) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) gate_s[(z0 + i) * 64 + tr - 64] = v[i];
+                }
+                if (quarter < 2) {
+                    ok = mbar_wait_warp(gate_full, n_pairs & 1u, p.err);
+                    if (ok && z0 < p.zpad && row0 + tr < M.rows) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            if (z0 + i < p.Z) ts_store(p, M, mi, row0 + tr, z0 + i, ts_silu(v[i], gate_s[(z0 + i) * 64 + tr]));
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(gate_empty);
+                } else {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(gate_full);
+                }
+                ++n_pairs;
+            } else if (z0 < p.zpad && row0 + tr < M.rows) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (z0 + i < p.Z) ts_store(p, M, mi, row0 + tr, z0 + i, v[i]);
+            }
+        };
+
+        uint32_t tile = tile0, g = g0, seg = 0, seg_begin = g0, rs = 0, raw_phase = 0;
+        bool pending = false, pend_whole = false;
+        uint32_t pend_tile = 0, pend_slot = 0, pend_seg = 0;
+        // the raw words of a unit are fetched while the one before it is dequantised (rows are 9 / 17 chunks of 16 bytes apart, so a
+        // quarter warp's loads fall into different banks)
+        uint32_t L[4 * ts_load_chunks<QT>()];
+        auto fetch = [&]() {
+            ok = mbar_wait(&raw_full[rs], raw_phase, p.err);
+            if (!ok) return;
+            const uint4* src = reinterpret_cast<const uint4*>(rawring + rs * kRawStage + tr * kRawRowBytes) + (QT == T_Q4_0 ? 2u : 4u) * tt;
+#pragma unroll
+            for (int c = 0; c < ts_load_chunks<QT>(); ++c) {
+                const uint4 v = src[c];
+                L[4 * c] = v.x; L[4 * c + 1] = v.y; L[4 * c + 2] = v.z; L[4 * c + 3] = v.w;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&raw_empty[rs]);
+            if (++rs == plan.n_raw) { rs = 0; raw_phase ^= 1u; }
+        };
+        fetch();
+        for (uint32_t i = 0; i < n_units && ok; ++i) {
+            uint32_t cols[32];
+            switch (tt) {                      // (the same for the whole warp)
+                case 0: ts_dequant<QT, 0>(L, cols); break;
+                case 1: ts_dequant<QT, 1>(L, cols); break;
+                case 2: ts_dequant<QT, 2>(L, cols); break;
+                default: ts_dequant<QT, 3>(L, cols); break;
+            }
+            if (i + 1 < n_units) fetch();
+            if (!ok) break;
+            const uint32_t ab = i & 1u;
+            if (i >= 2) {
+                ok = mbar_wait(&a_empty[2 * ab + half], ((i >> 1) - 1) & 1u, p.err);
+                if (!ok) break;
+                tc_fence_after_sync();
+            }
+            const uint32_t taddr = tmem_base + lanes_at + kTsABase + (4u * ab + tt) * kTsTileCols;
+            asm volatile(
+                "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+                "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+                ::"r"(taddr), "r"(cols[0]), "r"(cols[1]), "r"(cols[2]), "r"(cols[3]), "r"(cols[4]), "r"(cols[5]), "r"(cols[6]), "r"(cols[7]),
+                  "r"(cols[8]), "r"(cols[9]), "r"(cols[10]), "r"(cols[11]), "r"(cols[12]), "r"(cols[13]), "r"(cols[14]), "r"(cols[15]),
+                  "r"(cols[16]), "r"(cols[17]), "r"(cols[18]), "r"(cols[19]), "r"(cols[20]), "r"(cols[21]), "r"(cols[22]), "r"(cols[23]),
+                  "r"(cols[24]), "r"(cols[25]), "r"(cols[26]), "r"(cols[27]), "r"(cols[28]), "r"(cols[29]), "r"(cols[30]), "r"(cols[31])
+                : "memory");
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&a_full[2 * ab + half]);
+            if (pending) {
+                drain(pend_seg, pend_tile, pend_whole, pend_slot);
+                pending = false;
+            }
+            if (++g == G || i + 1 == n_units) {
+                pending = true;
+                pend_whole = seg_begin == 0 && g == G;
+                pend_tile = tile;
+                pend_slot = (seg == 0) ? 0u : 1u;
+                pend_seg = seg;
+                ++seg;
+                ++tile;
+                g = seg_begin = 0;
+            }
+        }
+        // (the warps of a CTA may disagree about `ok` only after a lost wait, whose error word ends every later wait; barriers below
+        // are reached by all of them)
+        if (ok && pending) drain(pend_seg, pend_tile, pend_whole, pend_slot);
+
+        // ---- tiles that other CTAs work on as well ----
+        const uint32_t u_end = u0 + n_units, last_tile = (u_end - 1) / G;
+        const bool cut_first = g0 != 0 || u_end < (tile0 + 1) * G, cut_last = last_tile != tile0 && u_end < (last_tile + 1) * G;
+        if (cut_first || cut_last) {
+            asm volatile("bar.sync 2, 512;" ::: "memory");
+            if (threadIdx.x < 2) {
+                const uint32_t t = threadIdx.x == 0 ? tile0 : last_tile;
+                uint32_t mine = 0;
+                if (threadIdx.x == 0 ? cut_first : cut_last) {
+                    const uint32_t parts = ((t + 1) * G - 1) / plan.per - t * G / plan.per + 1;
+                    __threadfence();
+                    if (atomicAdd(&p.counters[t], 1u) + 1 == parts) {
+                        mine = 1;
+                        __threadfence();
+                        p.counters[t] = 0;                          // ready for the next launch
+                    }
+                }
+                s_last[threadIdx.x] = mine;
+            }
+            asm volatile("bar.sync 2, 512;" ::: "memory");
+            // (two tiles are finished side by side)
+            const bool both = *reinterpret_cast<volatile uint32_t*>(&s_last[0]) != 0 && *reinterpret_cast<volatile uint32_t*>(&s_last[1]) != 0;
+            const uint32_t k = both ? uint32_t(warp) / (kTsProducers / 2) : (*reinterpret_cast<volatile uint32_t*>(&s_last[0]) != 0 ? 0u : 1u);
+            const uint32_t n_warps = both ? kTsProducers / 2 : kTsProducers;
+            if (*reinterpret_cast<volatile uint32_t*>(&s_last[k]) != 0 && ok) {
+                const uint32_t t = k == 0 ? tile0 : last_tile;
+                const uint32_t c_first = t * G / plan.per, c_last = ((t + 1) * G - 1) / plan.per;
+                uint32_t row0;
+                const int mi = matrix_of(t, row0);
+                const GemvMatrix& M = p.m[mi];
+                // a warp has whole tokens, a lane four rows of them; the parts of four tokens and three CTAs are on their way together
+                constexpr uint32_t kTok = 4, kParts = 3;
+                for (uint32_t zb = uint32_t(warp) % n_warps; zb < p.Z; zb += kTok * n_warps) {
+                    float4 sum[kTok] = {};
+                    for (uint32_t cb = c_first; cb <= c_last; cb += kParts) {
+                        float4 x[kParts][kTok];
+#pragma unroll
+                        for (uint32_t j = 0; j < kParts; ++j) {
+                            const uint32_t c = min(cb + j, c_last), slot = c * plan.per >= t * G ? 0u : 1u;        // its first segment, or its last
+                            const float* q = p.scratch + size_t(2 * c + slot) * p.zpad * kTcRows + 4 * lane;
+#pragma unroll
+                            for (uint32_t i = 0; i < kTok; ++i)
+                                x[j][i] = __ldcg(reinterpret_cast<const float4*>(q + size_t(min(zb + i * n_warps, p.Z - 1)) * kTcRows));
+                        }
+#pragma unroll
+                        for (uint32_t j = 0; j < kParts; ++j)
+#pragma unroll
+                            for (uint32_t i = 0; i < kTok; ++i)
+                                if (cb + j <= c_last) {
+                                    sum[i].x += x[j][i].x;
+                                    sum[i].y += x[j][i].y;
+                                    sum[i].z += x[j][i].z;
+                                    sum[i].w += x[j][i].w;
+                                }
+                    }
+#pragma unroll
+                    for (uint32_t i = 0; i < kTok; ++i) {
+                        const uint32_t z = zb + i * n_warps, row = row0 + 4 * uint32_t(lane);
+                        if (z >= p.Z) break;
+                        float4 v = sum[i];
+                        if (pair) {                                // lanes 16 .. 31 hold the gate
+                            const float4 gate = make_float4(__shfl_down_sync(0xffffffffu, v.x, 16), __shfl_down_sync(0xffffffffu, v.y, 16),
+                                                            __shfl_down_sync(0xffffffffu, v.z, 16), __shfl_down_sync(0xffffffffu, v.w, 16));
+                            v = make_float4(ts_silu(v.x, gate.x), ts_silu(v.y, gate.y), ts_silu(v.z, gate.z), ts_silu(v.w, gate.w));
+                            if (lane >= 16) continue;
+                        }
+                        if (row < M.rows) ts_store4(p, M, mi, row, z, v);          // (rows come in multiples of 32)
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == kTsProducers + 1) {
+        tc_fence_after_sync();
+        tc_free(tmem_base, 512);
+    }
+}
+
+int gemm_tc_stream_configure(lv_ctx* ctx) {
+    LV_REQUIRE(size_t(ctx->max_smem_optin) >= size_t(kTsSmemBytes), "device has too little shared memory for the batched product");
+    LV_CUDA((cudaFuncSetAttribute(gemm_tc_stream_kernel<T_Q4_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTsSmemBytes))));
+    LV_CUDA((cudaFuncSetAttribute(gemm_tc_stream_kernel<T_Q8_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTsSmemBytes))));
+    return LV_OK;
+}
+
+template <int QT>
+static int launch_typed(lv_ctx* ctx, const GemmTcParams& p, const GemmTcMaps& maps, uint32_t tiles) {
+    TsPlan plan{};
+    plan.groups = p.K / (4 * kTcChunkK);
+    plan.units = tiles * plan.groups;
+    const uint32_t sms = uint32_t(ctx->sm_count);
+    // equal runs; at least two units each, since a part costs about as much as two units
+    plan.per = max((plan.units + sms - 1) / sms, min(2u, plan.groups));
+    // whole tiles only, where the arrival counters or the scratch (two parts per CTA) would not do
+    static const char* no_split = getenv("LV_GEMM_TC_NO_SPLIT");
+    if (tiles > kTcMaxTiles || size_t(sms) * 2 * p.zpad * kTcRows * sizeof(float) > kTcScratchBytes || (no_split != nullptr && no_split[0] == '1'))
+        plan.per = (tiles + sms - 1) / sms * plan.groups;
+    // shared memory: up to 128 KB of activations (96 KB beside the larger q8_0 stages) in an even number of stages, the rest raw stages
+    const uint32_t b_stage = ts_b_tiles<QT>() * 4u * p.zpad * kTcChunkK;
+    plan.n_b = min(uint32_t(kTsMaxB), (QT == T_Q4_0 ? 131072u : 98304u) / b_stage) & ~1u;
+    plan.n_raw = min(uint32_t(kTsMaxRaw), (kTsSmemBytes - 1024 - kTsGateBytes - kTsBarBytes - plan.n_b * b_stage) / uint32_t(tc_raw_stage<QT>()));
+    LV_CUDA((launch_pdl(ctx, gemm_tc_stream_kernel<QT>, dim3((plan.units + plan.per - 1) / plan.per), dim3(kTsThreads), kTsSmemBytes, p, plan, maps)));
+    return LV_OK;
+}
+
+int launch_gemm_tc_stream(lv_ctx* ctx, const GemmTcParams& p, const GemmTcMaps& maps, int wtype, uint32_t tiles) {
+    return wtype == T_Q4_0 ? launch_typed<T_Q4_0>(ctx, p, maps, tiles) : launch_typed<T_Q8_0>(ctx, p, maps, tiles);
+}
+
+}  // namespace lv

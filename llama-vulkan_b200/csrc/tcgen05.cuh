@@ -46,6 +46,13 @@ __device__ __forceinline__ uint64_t tc_smem_desc(uint32_t smem_addr) {
            (uint64_t(2) << 61);
 }
 
+// True in one lane of a converged warp, the same one every time.
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t yes;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(yes));
+    return yes != 0;
+}
+
 // Sixteen accumulator columns of this warp's quarter of the lanes; waits for the data.
 __device__ __forceinline__ void tc_load16(uint32_t (&u)[16], uint32_t taddr) {
     asm volatile(
