@@ -3,10 +3,19 @@
 //   out[t][r] = act(factor * sum_k W[r][k] x[t][k])        W and x bfloat16, sums f32
 //
 // A CTA covers 128 rows of W (the M of the MMA) and NT tokens (its N).  Both operands are K-major and come by TMA in boxes of
-// 64 columns with the 128-byte swizzle, 4 to 8 stages deep; one lane issues the loads, one lane the MMAs, four warps read the
+// 64 columns with the 128-byte swizzle; one lane issues the loads, one lane the MMAs, four warps read the
 // accumulator from tensor memory (lane = row, column = token, so a warp stores 32 consecutive features of a token).  The
-// first weight tiles are requested before the previous kernel has finished.  Matrices with few tiles are split along K over
-// several CTAs: each leaves its partial sums in scratch and the last to arrive adds them in split order (deterministic).
+// first weight tiles are requested before the previous kernel has finished.
+//
+// What bounds it: the operands' way from L2.  An SM takes in about 46 bytes per clock (measured), so 64 columns of a tile cost
+// (128 + NT) * 128 / 46 clocks against 2 NT of the tensor pipe: 534 / 128 at NT = 64, 712 / 256 at 128, 1070 / 512 at 256.  So wide tiles
+// come first, and a matrix whose wide tiles are too few is split along K over a cluster of up to eight CTAs: each leaves its
+// partial sums in its own shared memory, where the stages were, and they are added in split order (deterministic) through
+// distributed shared memory, every CTA finishing its share of the tokens.  A launch of more tiles than SMs without a split runs two CTAs
+// per SM, so that the set-up and the stores of one run beside the products of the other.
+// 512 tokens (before: tiles of 64 or 128 tokens, one CTA per SM, partial sums through global memory): 16512 x 4096 107.8 -> 57.1 us (1.21 PFLOP/s),
+// 4096 x 16512 79.6 -> 55.1, 8448 x 2048 30.1 -> 19.7, 2048 x 8448 41.6 -> 21.0; 2048 tokens: 16512 x 4096 389 -> 224, 4096 x 16512 317 -> 189 (1.46).
+// Sums of split products are nearer to 64 bits than before (2048 x 8448, 512 tokens: 9.4e-6 -> 2.2e-6 relative), the others the same.
 //
 // Experts: lv_expert_route sorts the (token, choice) pairs of a step by expert and lists tiles of NT rows; the input rows lie
 // in that order (lv_norm_conv scatters them there), a tile multiplies them with its expert's rows of the stacked matrix.
@@ -21,6 +30,7 @@
 
 #include <algorithm>
 
+#include "attention_gqa.cuh"
 #include "common.cuh"
 #include "ctx.h"
 #include "tcgen05.cuh"
@@ -31,18 +41,15 @@ namespace lv {
 constexpr int kBgThreads = 192;              // TMA warp, MMA warp, four epilogue warps
 constexpr int kBgRows = 128, kBgK = 64;
 constexpr uint32_t kBgTile = kBgRows * kBgK * 2;
-constexpr size_t kBgSmemBudget = 200 * 1024;
+constexpr size_t kBgSmemBudget = 200 * 1024, kBgSmemHalf = 108 * 1024;      // one / two CTAs per SM
 constexpr uint32_t kBgMaxStages = 8;
-constexpr uint32_t kBgMaxTiles = 4096;       // arrival counters of split launches
-constexpr size_t kBgScratchBytes = size_t(32) << 20;
+constexpr uint32_t kBgMaxSplits = 8;         // portable cluster size
 
 struct GemmBf16Params {
     uint32_t rows, tokens, K, splits, stages;
     void* out;
     uint32_t out_ld, out_bf16;
     float factor;
-    float* scratch;
-    uint32_t* counters;
     int act;
     const lv_expert_tile* tiles;
     const uint32_t* pos;        // windows: the position word, null otherwise
@@ -60,14 +67,24 @@ __host__ __device__ constexpr uint32_t bg_tmem_cols(int NT, bool pair) {
     return need <= 32 ? 32 : need <= 64 ? 64 : need <= 128 ? 128 : need <= 256 ? 256 : 512;
 }
 
+// four floats in the shared memory of another CTA of the cluster
+__device__ __forceinline__ float4 bg_cluster_load4(const float* local, uint32_t rank) {
+    uint32_t at;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+    return v;
+}
+
+// grid (row tiles, token tiles, splits), clusters of (1, 1, splits)
 template <int NT, bool PAIR, bool GROUPED>
-__global__ void __launch_bounds__(kBgThreads, 1) gemm_bf16_kernel(const GemmBf16Params p, const __grid_constant__ GemmBf16Maps maps) {
+__global__ void __launch_bounds__(kBgThreads, 2) gemm_bf16_kernel(const GemmBf16Params p, const __grid_constant__ GemmBf16Maps maps) {
     pdl_launch_dependents();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
     constexpr uint32_t kStage = bg_stage_bytes(NT, PAIR), kCols = bg_tmem_cols(NT, PAIR), kXAt = (PAIR ? 2 : 1) * kBgTile;
     __shared__ uint64_t full[kBgMaxStages], empty[kBgMaxStages], acc_full;
-    __shared__ uint32_t s_tmem, s_last;
+    __shared__ uint32_t s_tmem;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
     uint32_t row0 = blockIdx.x * kBgRows, tok0 = blockIdx.y * NT, n_tok;
@@ -156,8 +173,7 @@ __global__ void __launch_bounds__(kBgThreads, 1) gemm_bf16_kernel(const GemmBf16
         ok = mbar_wait_warp(&acc_full, 0, p.err);
         tc_fence_after_sync();
         constexpr int kAcc = PAIR ? 2 : 1;
-        const uint32_t tile = blockIdx.y * gridDim.x + blockIdx.x;
-        float* partial = p.splits > 1 ? p.scratch + size_t(tile) * p.splits * (kAcc * NT * kBgRows) : nullptr;
+        float* partial = reinterpret_cast<float*>(smem);         // [accumulator][token][128 rows]: all stages have been used up
         auto finish = [&](const float (&v)[16], const float (&g)[16], uint32_t z0) {
             if (row >= p.rows) return;
 #pragma unroll
@@ -181,38 +197,11 @@ __global__ void __launch_bounds__(kBgThreads, 1) gemm_bf16_kernel(const GemmBf16
                 if (p.splits == 1) {
                     finish(v, g, z0);
                 } else {
-                    float* dst = partial + size_t(blockIdx.z) * (kAcc * NT * kBgRows);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
-                        dst[(z0 + i) * kBgRows + tr] = v[i];
-                        if constexpr (PAIR) dst[(NT + z0 + i) * kBgRows + tr] = g[i];
+                        partial[(z0 + i) * kBgRows + tr] = v[i];
+                        if constexpr (PAIR) partial[(NT + z0 + i) * kBgRows + tr] = g[i];
                     }
-                }
-            }
-        }
-        if (p.splits > 1) {
-            __threadfence();
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (threadIdx.x == 64) {
-                const uint32_t last = atomicAdd(&p.counters[tile], 1u) + 1 == p.splits ? 1u : 0u;
-                if (last) p.counters[tile] = 0;
-                s_last = last;
-            }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (*reinterpret_cast<volatile uint32_t*>(&s_last) != 0 && ok) {
-                __threadfence();
-                for (uint32_t z0 = 0; z0 < NT && z0 < n_tok; z0 += 16) {
-                    float v[16] = {}, g[16] = {};
-#pragma unroll 2
-                    for (uint32_t s = 0; s < p.splits; ++s) {
-                        const float* src = partial + size_t(s) * (kAcc * NT * kBgRows);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            v[i] += __ldcg(src + (z0 + i) * kBgRows + tr);
-                            if constexpr (PAIR) g[i] += __ldcg(src + (NT + z0 + i) * kBgRows + tr);
-                        }
-                    }
-                    finish(v, g, z0);
                 }
             }
         }
@@ -222,6 +211,57 @@ __global__ void __launch_bounds__(kBgThreads, 1) gemm_bf16_kernel(const GemmBf16
     if (warp == 1) {
         tc_fence_after_sync();
         tc_free(tmem, kCols);
+    }
+    if (p.splits > 1) {
+        __syncwarp();
+        cluster_sync();                                   // the partial sums of all CTAs are in place
+        // a warp has whole tokens, a lane four rows of them; kTok tokens are on their way together
+        constexpr int kTok = PAIR ? 2 : 4, kWarps = kBgThreads / 32;
+        const float* mine = reinterpret_cast<const float*>(smem) + 4 * lane;
+        const uint32_t row = row0 + 4 * uint32_t(lane), z_end = n_tok * (blockIdx.z + 1) / p.splits;
+        const bool vec = row + 4 <= p.rows && p.out_ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
+        pdl_wait();                                       // (of the warps only the loading one has waited for the previous kernel)
+        for (uint32_t z0 = n_tok * blockIdx.z / p.splits + warp; z0 < z_end; z0 += kTok * kWarps) {
+            float4 v[kTok] = {}, g[kTok] = {};
+#pragma unroll 2
+            for (uint32_t c = 0; c < p.splits; ++c) {
+#pragma unroll
+                for (int i = 0; i < kTok; ++i) {
+                    const uint32_t z = min(z0 + uint32_t(i) * kWarps, n_tok - 1);
+                    const float4 a = bg_cluster_load4(mine + z * kBgRows, c);
+                    v[i] = make_float4(v[i].x + a.x, v[i].y + a.y, v[i].z + a.z, v[i].w + a.w);
+                    if constexpr (PAIR) {
+                        const float4 b = bg_cluster_load4(mine + (NT + z) * kBgRows, c);
+                        g[i] = make_float4(g[i].x + b.x, g[i].y + b.y, g[i].z + b.z, g[i].w + b.w);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < kTok; ++i) {
+                const uint32_t z = z0 + uint32_t(i) * kWarps;
+                if (z >= z_end) break;
+                const float x[4] = {v[i].x, v[i].y, v[i].z, v[i].w}, y[4] = {g[i].x, g[i].y, g[i].z, g[i].w};
+                float o[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) o[j] = PAIR ? silu_f32(x[j]) * y[j] : product_act(x[j] * p.factor, p.act);
+                const size_t at = size_t(tok0 + z) * p.out_ld + row;
+                if (p.out_bf16) {
+                    auto* to = static_cast<__nv_bfloat16*>(p.out) + at;
+                    if (vec) {
+                        const __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
+                        *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                    } else {
+                        for (int j = 0; j < 4; ++j) if (row + j < p.rows) to[j] = __float2bfloat16_rn(o[j]);
+                    }
+                } else {
+                    float* to = static_cast<float*>(p.out) + at;
+                    if (vec) *reinterpret_cast<float4*>(to) = make_float4(o[0], o[1], o[2], o[3]);
+                    else for (int j = 0; j < 4; ++j) if (row + j < p.rows) to[j] = o[j];
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync();                                   // no CTA leaves while another reads its shared memory
     }
 }
 
@@ -279,37 +319,79 @@ __global__ void __launch_bounds__(1024) expert_route_kernel(const lv_route_job* 
     for (uint32_t i = threadIdx.x; i < pairs; i += blockDim.x) job.index[i] = atomicAdd(&s_cursor[expert(i)], 1u);
 }
 
+// How many clusters of each size the device holds at a time, one CTA per SM: the SMs of a cluster are neighbours, so of 148 SMs clusters of
+// eight fill fewer than clusters of two.  (Two waves of clusters made a product of 2048 x 2048 with 60 tokens 18 us instead of 9.)
 int gemm_bf16_configure(lv_ctx* ctx) {
-    LV_CUDA(cudaMalloc(&ctx->bg_scratch, kBgScratchBytes));
-    LV_CUDA(cudaMalloc(&ctx->bg_counters, kBgMaxTiles * sizeof(uint32_t)));
-    LV_CUDA(cudaMemset(ctx->bg_counters, 0, kBgMaxTiles * sizeof(uint32_t)));
+    auto* kernel = gemm_bf16_kernel<128, false, false>;
+    LV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBgSmemBudget + 1024)));
+    for (uint32_t s = 2; s <= kBgMaxSplits; ++s) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(1, 1, s);
+        cfg.blockDim = dim3(kBgThreads);
+        cfg.dynamicSmemBytes = kBgSmemBudget;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = s;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        LV_CUDA(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
+        ctx->bg_clusters[s] = uint32_t(n);
+    }
     return LV_OK;
 }
 
-void gemm_bf16_release(lv_ctx* ctx) {
-    cudaFree(ctx->bg_scratch);
-    cudaFree(ctx->bg_counters);
-    ctx->bg_scratch = ctx->bg_counters = nullptr;
+// Clocks of 64 columns of a tile on one SM: the tensor pipe, or the way of the operands.
+static float bg_chunk_clocks(uint32_t nt, bool pair) { return std::max(2.f * nt * (pair ? 2 : 1), ((pair ? 2 : 1) * kBgTile + nt * 128.f) / 64.f); }
+
+// Splits along K: as many as fill the SMs once, each with at least four chunks; a split costs the meeting of its cluster, about 4000 clocks and
+// 16 more per token of the tile.
+static uint32_t bg_splits(const lv_ctx* ctx, uint32_t ctas, uint32_t chunks, uint32_t nt, bool pair, float* clocks) {
+    const uint32_t sms = uint32_t(ctx->sm_count);
+    const float c = bg_chunk_clocks(nt, pair);
+    // without a split: two CTAs share an SM, so a last wave that is not full costs its part only
+    float best = ctas > sms ? (float(ctas) / sms + 0.25f) * chunks * c + 4000.f : chunks * c + 4000.f;
+    uint32_t splits = 1;
+    for (uint32_t s = 2; s <= kBgMaxSplits && chunks / s >= 4; ++s) {
+        if (ctas > ctx->bg_clusters[s]) continue;
+        const float t = (chunks + s - 1) / s * c + 8000.f + 16.f * nt;
+        if (t < best) { best = t; splits = s; }
+    }
+    *clocks = best;
+    return splits;
 }
 
 template <int NT, bool PAIR, bool GROUPED>
 static int gemm_bf16_launch(lv_ctx* ctx, GemmBf16Params p, const GemmBf16Maps& maps, uint32_t token_tiles) {
     constexpr uint32_t kStage = bg_stage_bytes(NT, PAIR);
-    p.stages = std::min<uint32_t>(kBgMaxStages, kBgSmemBudget / kStage);
     const uint32_t row_tiles = (p.rows + kBgRows - 1) / kBgRows, chunks = (p.K + kBgK - 1) / kBgK, ctas = row_tiles * token_tiles;
-    // K splits: as many as fill the SMs once, each with at least four chunks
-    p.splits = 1;
-    while (ctas * (p.splits + 1) <= uint32_t(ctx->sm_count) && chunks / (p.splits + 1) >= 4 && p.splits < 16) ++p.splits;
-    if (ctas > kBgMaxTiles || size_t(ctas) * p.splits * (PAIR ? 2 : 1) * NT * kBgRows * 4 > kBgScratchBytes) p.splits = 1;
-    p.scratch = static_cast<float*>(ctx->bg_scratch);
-    p.counters = static_cast<uint32_t*>(ctx->bg_counters);
+    float clocks;
+    p.splits = bg_splits(ctx, ctas, chunks, NT, PAIR, &clocks);
+    p.stages = std::min<uint32_t>(kBgMaxStages, uint32_t((p.splits == 1 && ctas > uint32_t(ctx->sm_count) ? kBgSmemHalf : kBgSmemBudget) / kStage));
     p.err = ctx->d_err;
-    const size_t smem = size_t(p.stages) * kStage + 1024;
+    const size_t smem = std::max(size_t(p.stages) * kStage, p.splits > 1 ? size_t(PAIR ? 2 : 1) * NT * kBgRows * sizeof(float) : 0) + 1024;
     auto* kernel = gemm_bf16_kernel<NT, PAIR, GROUPED>;
     LV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     LV_REQUIRE(token_tiles <= 65535, "gemm_bf16: too many token tiles");
-    LV_CUDA(launch_pdl(ctx, kernel, dim3(row_tiles, token_tiles, p.splits), dim3(kBgThreads), smem, p, maps));
+    const dim3 grid(row_tiles, token_tiles, p.splits);
+    if (p.splits == 1) LV_CUDA(launch_pdl(ctx, kernel, grid, dim3(kBgThreads), smem, p, maps));
+    else LV_CUDA(launch_pdl_cluster(ctx, kernel, grid, dim3(kBgThreads), dim3(1, 1, p.splits), smem, p, maps));
     return LV_OK;
+}
+
+// Tokens of a tile for a product of `tokens` rows: the width that takes least by the model above.
+static uint32_t bg_token_tile(lv_ctx* ctx, uint32_t rows, uint32_t cols, uint32_t tokens) {
+    uint32_t nt = 0;
+    float best = 0.f;
+    for (uint32_t n : {16u, 32u, 64u, 128u, 256u}) {
+        if (n > 32 && n / 2 >= tokens) break;                    // (half of it would do)
+        if (n == 16 && tokens > 16) continue;
+        float t;
+        bg_splits(ctx, (rows + kBgRows - 1) / kBgRows * ((tokens + n - 1) / n), (cols + kBgK - 1) / kBgK, n, false, &t);
+        if (nt == 0 || t < best) { best = t; nt = n; }
+    }
+    return nt;
 }
 
 template <bool PAIR, bool GROUPED>
@@ -318,7 +400,10 @@ static int gemm_bf16_pick(lv_ctx* ctx, const GemmBf16Params& p, const GemmBf16Ma
         case 16: return gemm_bf16_launch<16, PAIR, GROUPED>(ctx, p, maps, token_tiles);
         case 32: return gemm_bf16_launch<32, PAIR, GROUPED>(ctx, p, maps, token_tiles);
         case 64: return gemm_bf16_launch<64, PAIR, GROUPED>(ctx, p, maps, token_tiles);
-        default: return gemm_bf16_launch<128, PAIR, GROUPED>(ctx, p, maps, token_tiles);
+        case 128: return gemm_bf16_launch<128, PAIR, GROUPED>(ctx, p, maps, token_tiles);
+        default:
+            if constexpr (!GROUPED) return gemm_bf16_launch<256, PAIR, GROUPED>(ctx, p, maps, token_tiles);
+            return fail(LV_ERR_BAD_ARGUMENTS, "gemm_bf16: tile of an expert");
     }
 }
 
@@ -336,9 +421,7 @@ extern "C" int lv_gemm_bf16(lv_ctx* ctx, void* out, int out_type, uint32_t out_l
     LV_REQUIRE(act == LV_ACT_NONE || act == LV_ACT_RELU2, "gemm_bf16: unknown activation");
     GemmBf16Params p{};
     p.rows = rows; p.tokens = batch; p.K = cols; p.out = out; p.out_ld = out_ld; p.out_bf16 = out_type == LV_TYPE_BF16; p.factor = factor; p.act = act;
-    uint32_t nt = batch <= 16 ? 16 : batch <= 32 ? 32 : batch <= 64 ? 64 : 128;
-    // narrower token tiles before K splits: partial sums cost more than reading a weight tile twice
-    while (nt > 32 && (rows + kBgRows - 1) / kBgRows * ((batch + nt - 1) / nt) * 2 <= uint32_t(ctx->sm_count) && batch > nt / 2) nt /= 2;
+    const uint32_t nt = bg_token_tile(ctx, rows, cols, batch);
     GemmBf16Maps maps{};
     if (int rc = make_bf16_map(&maps.w, w, rows, cols, ld, kBgRows)) return rc;
     if (int rc = make_bf16_map(&maps.x, x, batch, cols, x_ld, nt)) return rc;
@@ -354,8 +437,7 @@ extern "C" int lv_gemm_bf16_window(lv_ctx* ctx, void* out, int out_type, uint32_
     GemmBf16Params p{};
     p.rows = rows; p.tokens = max_rows; p.K = cols; p.out = out; p.out_ld = out_ld; p.out_bf16 = out_type == LV_TYPE_BF16; p.factor = 1.0f;
     p.pos = pos; p.window = window; p.batch = batch;
-    uint32_t nt = max_rows <= 16 ? 16 : max_rows <= 32 ? 32 : max_rows <= 64 ? 64 : 128;
-    while (nt > 32 && (rows + kBgRows - 1) / kBgRows * ((max_rows + nt - 1) / nt) * 2 <= uint32_t(ctx->sm_count)) nt /= 2;
+    const uint32_t nt = bg_token_tile(ctx, rows, cols, max_rows);
     GemmBf16Maps maps{};
     if (int rc = make_bf16_map(&maps.w, w, rows, cols, ld, kBgRows)) return rc;
     if (int rc = make_bf16_map(&maps.x, x, x_rows, cols, x_ld, nt)) return rc;

@@ -41,6 +41,14 @@ def test_gemm_bf16(gpu, rows, cols, batch, out_bf16):
     assert rel(got, want) < (3e-3 if out_bf16 else 2e-5)
 
 
+@pytest.mark.parametrize("rows,cols,batch", [(257, 1100, 255), (300, 2600, 512), (5, 4104, 257), (1030, 520, 700), (2600, 136, 2000), (40, 2048, 65), (129, 776, 16)])
+@pytest.mark.parametrize("out_bf16", [False, True])
+def test_gemm_bf16_tiles_and_splits(gpu, rows, cols, batch, out_bf16):
+    """Token tiles of 16 to 256, ragged in rows and tokens; splits along K over clusters of two to eight CTAs with remainders of K; more
+    tiles than SMs (two CTAs per SM); rows that four consecutive values of a lane reach past."""
+    test_gemm_bf16(gpu, rows, cols, batch, out_bf16)
+
+
 def expert_args(d, w0, w1, rows, cols, table, ids, pos, vocab):
     n, top = w0.shape[0], table.shape[1]
     a = pkg.ExpertArgs()
