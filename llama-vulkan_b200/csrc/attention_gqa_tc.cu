@@ -88,7 +88,6 @@ __device__ __forceinline__ float gt_exp2(float x) {
 // NH: halves a row is split into; PAIRS: 64 PAIRS >= head size (chunks of a key for LATENT)
 template <int NH, int PAIRS, bool LATENT>
 __global__ void __launch_bounds__(32 * kGtFirstSoftmax + 128 * NH) gqa_tc_kernel(const GqaTcParams p, const __grid_constant__ GqaTcMaps maps) {
-    pdl_launch_dependents();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
     const lv_gqa_args& a = p.a;
@@ -110,7 +109,10 @@ __global__ void __launch_bounds__(32 * kGtFirstSoftmax + 128 * NH) gqa_tc_kernel
         for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4 * NH); mbar_init(&pv_done[i], 1); }
         fence_mbar_init();
     }
-    if (warp == 1) tc_alloc(&s_tmem, p.tmem_cols);
+    if (warp == 1) {
+        tc_alloc(&s_tmem, p.tmem_cols);
+        pdl_launch_dependents();        // (not before: a CTA of the next launch could take the tensor memory that this one needs, and wait for it)
+    }
     pdl_wait();
     const uint32_t P = *a.pos;
     const bool inside = P + p.n_tokens <= a.ctx_rows;            // (lv_qk_norm_append reports positions beyond the cache)

@@ -79,7 +79,6 @@ __device__ __forceinline__ float4 bg_cluster_load4(const float* local, uint32_t 
 // grid (row tiles, token tiles, splits), clusters of (1, 1, splits)
 template <int NT, bool PAIR, bool GROUPED>
 __global__ void __launch_bounds__(kBgThreads, 2) gemm_bf16_kernel(const GemmBf16Params p, const __grid_constant__ GemmBf16Maps maps) {
-    pdl_launch_dependents();
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
     constexpr uint32_t kStage = bg_stage_bytes(NT, PAIR), kCols = bg_tmem_cols(NT, PAIR), kXAt = (PAIR ? 2 : 1) * kBgTile;
@@ -119,6 +118,9 @@ __global__ void __launch_bounds__(kBgThreads, 2) gemm_bf16_kernel(const GemmBf16
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&s_tmem);
+    // not before every CTA of this launch has its tensor memory: a CTA of the next one beside it could take what is missing, and wait for
+    // this launch with it
+    pdl_launch_dependents();
     bool ok = true;
 
     if (warp == 0) {
