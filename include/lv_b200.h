@@ -217,6 +217,14 @@ int lv_dequant_rows_group(lv_ctx* ctx, float* out, const void* table, int wtype,
 int lv_gemm_tc_qkv_kvappend_group(lv_ctx* ctx, float* q_out, const void* wq, const void* wk, const void* wv, int wtype,
                                   const void* xh, const lv_group_member* members, uint32_t rows_each, uint32_t dim,
                                   uint32_t n, uint32_t ctx_rows);
+/* What the next step of a group needs from the host: member z's pending token goes to its token log at `position`, and where `move` is
+ * set its position words (pos[0 .. 3]) are set to `position`.  feed: n items in pinned host memory (lv_host_alloc), unchanged until the
+ * launch has run. */
+typedef struct {
+    uint32_t position, token, move;
+} lv_group_feed_item;
+int lv_group_feed(lv_ctx* ctx, const lv_group_member* members, const lv_group_feed_item* feed, uint32_t n, uint32_t log_capacity);
+
 /* lv_attention_fused with query row z attending over members[z]'s caches up to *members[z].pos. */
 int lv_attention_fused_group(lv_ctx* ctx, float* out, const float* q, const lv_group_member* members, const float* rope_table,
                              void* scratch, uint32_t heads, uint32_t rot, uint32_t backlog, uint32_t n);

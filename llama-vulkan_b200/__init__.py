@@ -132,6 +132,7 @@ KERNEL_API = {
     "lv_act_split_f16_padded": (_int, [_p, _p, _p, _p, _u32, _u32, _u32]),
     "lv_dequant_rows_group": (_int, [_p, _p, _p, _int, _p, _u32, _u32, _u32]),
     "lv_gemm_tc_qkv_kvappend_group": (_int, [_p, _p, _p, _p, _p, _int, _p, _p, _u32, _u32, _u32, _u32]),
+    "lv_group_feed": (_int, [_p, _p, _p, _u32, _u32]),
     "lv_attention_fused_group": (_int, [_p, _p, _p, _p, _p, _p, _u32, _u32, _u32, _u32]),
     "lv_argmax_advance_group": (_int, [_p, _p, _u32, _p, _u32, _u32, _p, _p]),
     "lv_gemm_tc_set_exact": (_int, [_p, _int]),

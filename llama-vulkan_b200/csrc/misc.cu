@@ -238,6 +238,20 @@ __global__ void __launch_bounds__(1024) argmax_advance_group_kernel(const float*
     }
 }
 
+// One thread per member.  `feed` is pinned host memory, read in place: 12 bytes a member are not worth a copy of their own.
+__global__ void __launch_bounds__(64) group_feed_kernel(const lv_group_member* __restrict__ group, const lv_group_feed_item* __restrict__ feed,
+                                                        uint32_t n, uint32_t log_capacity, uint32_t* err) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t z = threadIdx.x;
+    if (z >= n) return;
+    const lv_group_feed_item f = feed[z];
+    if (f.position < log_capacity) group[z].token_log[f.position] = f.token;
+    else atomicOr(err, ERR_BAD_INDEX);
+    if (f.move != 0)
+        for (int i = 0; i < 4; ++i) group[z].pos[i] = f.position;
+}
+
 __global__ void decode_advance_kernel(uint32_t* config, const uint32_t* argmax, uint32_t* token_log, uint32_t batch,
                                       uint32_t log_capacity, uint32_t* tp_step, uint32_t* err) {
     pdl_launch_dependents();
@@ -279,6 +293,13 @@ extern "C" int lv_argmax_advance_group(lv_ctx* ctx, const float* logits, uint32_
     LV_REQUIRE(logits && vocab && members && n, "bad argmax_advance arguments");
     LV_CUDA(launch_pdl(ctx, argmax_advance_group_kernel, dim3(n), dim3(1024), 0, logits, vocab, members, log_capacity, out_tokens,
                        static_cast<volatile uint32_t*>(host_tokens), ctx->d_err));
+    return LV_OK;
+}
+
+extern "C" int lv_group_feed(lv_ctx* ctx, const lv_group_member* members, const lv_group_feed_item* feed, uint32_t n, uint32_t log_capacity) {
+    LV_ENTER(ctx);
+    LV_REQUIRE(members && feed && n >= 1 && n <= 64 && log_capacity, "bad group feed arguments");
+    LV_CUDA(launch_pdl(ctx, group_feed_kernel, dim3(1), dim3(64), 0, members, feed, n, log_capacity, ctx->d_err));
     return LV_OK;
 }
 

@@ -50,6 +50,8 @@ llava_session_group::llava_session_group(llava_context* _ctx, vector<llava_sessi
     void* p = nullptr;
     if (lv_host_alloc(ctx->lv(), size_t(k) * 4, &p) != LV_OK) return;
     pinned_tokens = static_cast<u32*>(p);
+    if (lv_host_alloc(ctx->lv(), size_t(k) * sizeof(lv_group_feed_item), &p) != LV_OK) return;
+    pinned_feed = static_cast<lv_group_feed_item*>(p);
     valid = true;
 }
 
@@ -57,6 +59,7 @@ llava_session_group::~llava_session_group() {
     discard_ahead();
     drop_graph();
     if (pinned_tokens) lv_host_free(ctx->lv(), pinned_tokens);
+    if (pinned_feed) lv_host_free(ctx->lv(), pinned_feed);
     for (llava_buffer* b : {x, q, vout, ff, split, logits, scratch, tables, tokens_dev, sampler_backup}) delete b;
     delete memory;
 }
@@ -100,17 +103,23 @@ bool llava_session_group::prepare_members(u32* backlog) {
         if (!tables->write_raw(0, table.data(), table_bytes)) return false;
         uploaded_table.assign(reinterpret_cast<const u8*>(table.data()), reinterpret_cast<const u8*>(table.data()) + table_bytes);
     }
+    // the pending tokens and the positions of members that were moved, in one launch (a copy per member and word took about 6 us each).
+    // Every step before this one has been waited for, so the words are free.
     vector<bool> sampled_now;
-    for (llava_session* s : members) {
-        if (!s->sync_device_position(s->current_tokens_in_gpu)) return false;
+    for (u32 i = 0; i < k; ++i) {
+        llava_session* s = members[i];
+        const u32 at = s->current_tokens_in_gpu;
         if (s->sampling_on_device() && !s->upload_sampler_state()) return false;
-        if (!s->upload_pending_tokens(s->current_tokens_in_gpu, 1)) return false;
+        if (!s->token_log_complete && !s->upload_pending_tokens(at, 1)) return false;         // a new log: the evaluated tokens as well
+        pinned_feed[i] = {at, s->token_buffer[at], s->device_pos != at ? 1u : 0u};
         if (!s->deterministic && s->host_sampler) {
             cerr << "[!] group step: a member samples on the host; only greedy members and the device sampler are supported" << endl;
             return false;
         }
         sampled_now.push_back(s->sampling_on_device());
     }
+    if (lv_group_feed(ctx->lv(), static_cast<const lv_group_member*>(tables->device_ptr()), pinned_feed, k, max_backlog_size + 1) != LV_OK) return false;
+    for (llava_session* s : members) s->device_pos = s->current_tokens_in_gpu;
     if (sampled_now != sampled) {            // the sampler launches are part of the recorded step
         drop_graph();
         sampled = sampled_now;

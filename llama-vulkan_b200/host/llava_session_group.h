@@ -67,6 +67,7 @@ private:
                  *tables = nullptr, *tokens_dev = nullptr, *sampler_backup = nullptr;
     std::vector<bool> sampled;               // per member: the recorded step ends with its sampler launch
     std::vector<u8> uploaded_table;          // the member tables as the device holds them
+    lv_group_feed_item* pinned_feed = nullptr;      // what a step takes from the host
     u32* pinned_tokens = nullptr;
     lv_graph* graph = nullptr;
     u32 graph_backlog = 0;

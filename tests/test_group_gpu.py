@@ -182,3 +182,30 @@ def test_group_members_that_sample_draw_with_their_own_sampler(pkg, world):
     g.close()
     for s in alone + grouped:
         s.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 33, 64])
+def test_group_feed_sets_tokens_and_moved_positions(gpu, pkg, n):
+    """lv_group_feed: tokens at their places of the members' logs, position words of moved members only; a place beyond the log is
+    reported and not written."""
+    cap, lib, h = 9, gpu.lib, gpu.handle
+    words = gpu.upload(np.full(n * (4 + cap + 1), 7, np.uint32))                     # per member: pos[4], log[cap], a guard
+    base = words.value if hasattr(words, "value") else int(words)
+    members = np.zeros((n, 4), np.uint64)
+    members[:, 2] = base + np.arange(n, dtype=np.uint64) * (4 * (5 + cap))
+    members[:, 3] = members[:, 2] + 16
+    table = gpu.upload(members)
+    host = C.c_void_p()
+    pkg.check(lib.lv_host_alloc(h, 12 * n, C.byref(host)))
+    feed = np.ctypeslib.as_array(C.cast(host, C.POINTER(C.c_uint32)), (n, 3))
+    feed[:] = [(z % cap, 100 + z, z % 3 == 0) for z in range(n)]
+    pkg.check(lib.lv_group_feed(h, table, host, n, cap))
+    gpu.sync()
+    want = np.full((n, 5 + cap), 7, np.uint32)
+    for z, (at, token, move) in enumerate(feed.tolist()):
+        want[z, 4 + at] = token
+        if move:
+            want[z, :4] = at
+    assert np.array_equal(gpu.download(words, np.uint32, want.size).reshape(want.shape), want)
+    assert lib.lv_group_feed(h, table, host, 65, cap) == pkg.LV_ERR_BAD_ARGUMENTS
+    pkg.check(lib.lv_host_free(h, host))
