@@ -276,6 +276,11 @@ int lv_gemm_tc(lv_ctx* ctx, float* out, const void* W, int wtype, const void* xh
 /* matmul_silu_ff for a batch (shaders/matmul_silu_ff.comp:49-97). */
 int lv_gemm_tc_silu(lv_ctx* ctx, float* out, const void* w3, const void* w1, int wtype, const void* xh, uint32_t ff,
                     uint32_t dim, uint32_t batch);
+/* lv_gemm_tc_silu whose finished rows become the split activations of a product with ff columns: xh_out, 16-byte aligned,
+ * lv_act_split_bytes(ff, batch), not xh.  Rows of the padding are left as they are.  out: f32 [batch][ff], used where the form of the weight
+ * tiles (lv_gemm_tc_set_exact) needs a launch of its own for it. */
+int lv_gemm_tc_silu_split(lv_ctx* ctx, void* xh_out, float* out, const void* w3, const void* w1, int wtype, const void* xh, uint32_t ff,
+                          uint32_t dim, uint32_t batch);
 
 /* wk, wq, wv products of a batch with the K and V rows written as f16 into the
  * caches at rows *pos + z (llava_layer.cpp:53-58); xh holds the normalised input. */
@@ -307,6 +312,11 @@ size_t lv_attention_scratch_bytes(uint32_t heads, uint32_t rot, uint32_t max_ctx
 int lv_attention_fused(lv_ctx* ctx, float* out, const float* q, const void* k_cache, const void* v_cache,
                        const uint32_t* pos, const float* rope_table, void* scratch, uint32_t heads, uint32_t rot,
                        uint32_t max_ctx, uint32_t batch);
+
+/* lv_attention_fused whose outputs become the split activations (lv_act_split_f16) of a product with heads * rot columns: xh_out, 16-byte
+ * aligned, lv_act_split_bytes(heads * rot, batch), batch <= 64.  Rows of the padding are left as they are. */
+int lv_attention_fused_split(lv_ctx* ctx, void* xh_out, const float* q, const void* k_cache, const void* v_cache, const uint32_t* pos,
+                             const float* rope_table, void* scratch, uint32_t heads, uint32_t rot, uint32_t max_ctx, uint32_t batch);
 
 /* Same computation as lv_attention_fused for callers that cannot allocate
  * device memory at the point where they need attention -- code that runs

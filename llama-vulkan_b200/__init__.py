@@ -126,6 +126,8 @@ KERNEL_API = {
     "lv_attention_scratch_bytes": (_sz, [_u32, _u32, _u32, _u32]),
     "lv_attention_fused": (_int, [_p, _p, _p, _p, _p, _p, _p, _p, _u32, _u32, _u32, _u32]),
     "lv_attention_static_scratch_limit": (_sz, []),
+    "lv_attention_fused_split": (_int, [_p, _p, _p, _p, _p, _p, _p, _p, _u32, _u32, _u32, _u32]),
+    "lv_gemm_tc_silu_split": (_int, [_p, _p, _p, _p, _p, _int, _p, _u32, _u32, _u32]),
     "lv_attention_fused_static": (_int, [_p, _p, _p, _p, _p, _p, _p, _u32, _u32, _u32, _u32]),
     "lv_act_split_bytes": (_sz, [_u32, _u32]),
     "lv_act_split_f16": (_int, [_p, _p, _p, _p, _u32, _u32]),

@@ -127,6 +127,7 @@ __host__ __device__ inline size_t attn_partial_floats(uint32_t heads, uint32_t n
     return size_t(batch) * heads * nchunks * (kRot + 2);
 }
 
+// xh: the outputs go there as split activations of zpad rows (lv_act_split_f16) instead of to out.
 // grid (heads, nchunks, batch).  CTA (h, c, z) covers cache rows [c*256, c*256+256)
 // up to P; contexts of up to 256 rows need one CTA per head and no combine, longer
 // ones end with the last CTA of a (z, h) combining the chunks.
@@ -161,7 +162,8 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
                                                                        const uint32_t* __restrict__ pos, const float* __restrict__ table,
                                                                        float* __restrict__ partial, uint32_t* __restrict__ counters,
                                                                        uint32_t heads, uint32_t nchunks, uint32_t max_ctx, float scale,
-                                                                       uint32_t* err, const lv_group_member* __restrict__ group) {
+                                                                       uint32_t* err, const lv_group_member* __restrict__ group,
+                                                                       __half* __restrict__ xh, uint32_t zpad) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float s_e[kAttnChunk];
@@ -350,7 +352,8 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
             l += s_l[r];
         }
         if (active == 1) {
-            out[size_t(z) * dim + h * kRot + threadIdx.x] = o / l;
+            if (xh != nullptr) split_store(xh, zpad, z, h * kRot + threadIdx.x, o / l);
+            else out[size_t(z) * dim + h * kRot + threadIdx.x] = o / l;
         } else {
             my[threadIdx.x] = o;
             if (threadIdx.x == 0) { my[kRot] = m; my[kRot + 1] = l; }
@@ -395,7 +398,8 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
 #pragma unroll
             for (int u = 0; u < 8; ++u) num = fmaf(oj[u], __shfl_sync(0xffffffffu, wj, (j0 + u) & 31), num);
         }
-        out[size_t(z) * dim + h * kRot + threadIdx.x] = num / den;
+        if (xh != nullptr) split_store(xh, zpad, z, h * kRot + threadIdx.x, num / den);
+        else out[size_t(z) * dim + h * kRot + threadIdx.x] = num / den;
     }
 }
 
@@ -419,7 +423,9 @@ static bool use_prompt_attention(uint32_t batch, uint32_t max_ctx) { return batc
 // ones (context beyond ~1280 rows, batches) stage key rows and the compact table, two CTAs per SM.
 static int launch_attention_fused(lv_ctx* ctx, dim3 grid, float* out, const float* q, const void* k_cache, const void* v_cache,
                                   const uint32_t* pos, const float* rope_table, float* partial, uint32_t* counters, uint32_t heads,
-                                  uint32_t nchunks, uint32_t max_ctx, uint32_t rot, const lv_group_member* group = nullptr) {
+                                  uint32_t nchunks, uint32_t max_ctx, uint32_t rot, const lv_group_member* group = nullptr, void* split = nullptr) {
+    auto* xh = static_cast<__half*>(split);
+    const uint32_t zpad = (grid.z + 15u) & ~15u;
     const float scale = 1.0f / sqrtf(static_cast<float>(rot));
     static const char* no_stage = getenv("LV_ATTENTION_NO_STAGING");
     // the compact table variant always copies the table rows of distances 0..31
@@ -428,19 +434,19 @@ static int launch_attention_fused(lv_ctx* ctx, dim3 grid, float* out, const floa
     if (!staged) {
         if (big) {
             LV_CUDA(launch_pdl(ctx, attention_fused_kernel<2, 0>, grid, dim3(kFusedThreads), 0, out, q, static_cast<const __half*>(k_cache),
-                               static_cast<const __half*>(v_cache), pos, rope_table, partial, counters, heads, nchunks, max_ctx, scale, ctx->d_err, group));
+                               static_cast<const __half*>(v_cache), pos, rope_table, partial, counters, heads, nchunks, max_ctx, scale, ctx->d_err, group, xh, zpad));
         } else {
             LV_CUDA(launch_pdl(ctx, attention_fused_kernel<1, 0>, grid, dim3(kFusedThreads), 0, out, q, static_cast<const __half*>(k_cache),
-                               static_cast<const __half*>(v_cache), pos, rope_table, partial, counters, heads, nchunks, max_ctx, scale, ctx->d_err, group));
+                               static_cast<const __half*>(v_cache), pos, rope_table, partial, counters, heads, nchunks, max_ctx, scale, ctx->d_err, group, xh, zpad));
         }
     } else if (big) {
         LV_CUDA(launch_pdl(ctx, attention_fused_kernel<2, 1>, grid, dim3(kFusedThreads), kCompactSmemBytes, out, q,
                            static_cast<const __half*>(k_cache), static_cast<const __half*>(v_cache), pos, rope_table, partial, counters,
-                           heads, nchunks, max_ctx, scale, ctx->d_err, group));
+                           heads, nchunks, max_ctx, scale, ctx->d_err, group, xh, zpad));
     } else {
         LV_CUDA(launch_pdl(ctx, attention_fused_kernel<1, 2>, grid, dim3(kFusedThreads), kStagedSmemBytes, out, q,
                            static_cast<const __half*>(k_cache), static_cast<const __half*>(v_cache), pos, rope_table, partial, counters,
-                           heads, nchunks, max_ctx, scale, ctx->d_err, group));
+                           heads, nchunks, max_ctx, scale, ctx->d_err, group, xh, zpad));
     }
     return LV_OK;
 }
@@ -547,6 +553,20 @@ extern "C" int lv_attention_fused(lv_ctx* ctx, float* out, const float* q, const
     dim3 grid(heads, nchunks, batch);
     if (int rc = launch_attention_fused(ctx, grid, out, q, k_cache, v_cache, pos, rope_table, partial, counters, heads, nchunks, max_ctx, rot)) return rc;
     return LV_OK;
+}
+
+extern "C" int lv_attention_fused_split(lv_ctx* ctx, void* xh_out, const float* q, const void* k_cache, const void* v_cache, const uint32_t* pos,
+                                        const float* rope_table, void* scratch, uint32_t heads, uint32_t rot, uint32_t max_ctx, uint32_t batch) {
+    LV_ENTER(ctx);
+    LV_REQUIRE(xh_out && q && k_cache && v_cache && pos && rope_table && scratch && (reinterpret_cast<uintptr_t>(xh_out) & 15u) == 0, "null or misaligned argument");
+    if (int rc = check_attn_shape(max_ctx, heads, rot, batch)) return rc;
+    LV_REQUIRE(batch <= 64, "split activations have at most 64 rows");
+    if (use_prompt_attention(batch, max_ctx)) return launch_attention_prompt(ctx, nullptr, q, k_cache, v_cache, pos, rope_table, heads, max_ctx, batch, xh_out);
+    const uint32_t nchunks = (max_ctx + kAttnChunk - 1) / kAttnChunk;
+    uint32_t* counters = static_cast<uint32_t*>(scratch);
+    float* partial = static_cast<float*>(scratch) + attn_counter_words(heads, batch);
+    return launch_attention_fused(ctx, dim3(heads, nchunks, batch), nullptr, q, k_cache, v_cache, pos, rope_table, partial, counters, heads, nchunks, max_ctx, rot,
+                                  nullptr, xh_out);
 }
 
 extern "C" int lv_attention_fused_group(lv_ctx* ctx, float* out, const float* q, const lv_group_member* members, const float* rope_table,

@@ -73,12 +73,14 @@ __device__ __forceinline__ float4 ap_cluster_load4(const float* local, uint32_t 
 // rows, four threads) that read 16 bytes of their rows hit different banks.
 __device__ __forceinline__ uint32_t ap_first_dim(uint32_t ks, uint32_t t) { return 64 * (ks >> 2) + 16 * t + 8 * ((ks >> 1) & 1) + 4 * (ks & 1); }
 
+// xh: the outputs go there as split activations of zpad rows (lv_act_split_f16) instead of to out
 // grid (heads, C, ceil(batch / 64)), clusters of (1, C, 1): CTA `rank` takes the 128-key chunks rank, rank + C, ...; ONE_PASS: C chunks at most
 template <bool ONE_PASS>
 __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* __restrict__ out, const float* __restrict__ q,
                                                                          const __half* __restrict__ kc, const __half* __restrict__ vc,
                                                                          const uint32_t* __restrict__ pos, const float* __restrict__ table,
-                                                                         uint32_t heads, uint32_t batch, uint32_t max_ctx, float scale, uint32_t* err) {
+                                                                         uint32_t heads, uint32_t batch, uint32_t max_ctx, float scale, uint32_t* err,
+                                                                         __half* __restrict__ xh, uint32_t zpad) {
     pdl_launch_dependents();
     extern __shared__ __align__(128) uint8_t smem[];
     uint8_t* s_q = smem;                                            // [plane][m tile][k step][lane][16 bytes]
@@ -334,7 +336,11 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
                 const float f = 1.f / s_l[r];
                 float* to = out + size_t(z0 + r) * dim + h * kApHead + 16 * warp + 2 * t;
 #pragma unroll
-                for (int j = 0; j < 2; ++j) *reinterpret_cast<float2*>(to + 8 * j) = make_float2(o[i][j][2 * u] * f, o[i][j][2 * u + 1] * f);
+                for (int j = 0; j < 2; ++j) {
+                    const float v[2] = {o[i][j][2 * u] * f, o[i][j][2 * u + 1] * f};
+                    if (xh != nullptr) split_store_n<2>(xh, zpad, z0 + r, h * kApHead + 16 * warp + 2 * t + 8 * j, v);
+                    else *reinterpret_cast<float2*>(to + 8 * j) = make_float2(v[0], v[1]);
+                }
             }
         return;
     }
@@ -371,7 +377,9 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
             sum.z = fmaf(part[c].z, f, sum.z);
             sum.w = fmaf(part[c].w, f, sum.w);
         }
-        *reinterpret_cast<float4*>(out + size_t(z0 + r) * dim + h * kApHead + 4 * lane) = make_float4(sum.x / den, sum.y / den, sum.z / den, sum.w / den);
+        const float v[4] = {sum.x / den, sum.y / den, sum.z / den, sum.w / den};
+        if (xh != nullptr) split_store_n<4>(xh, zpad, z0 + r, h * kApHead + 4 * lane, v);
+        else *reinterpret_cast<float4*>(out + size_t(z0 + r) * dim + h * kApHead + 4 * lane) = make_float4(v[0], v[1], v[2], v[3]);
     }
     cluster_sync();                                      // no CTA leaves while another reads its shared memory
 }
@@ -384,12 +392,12 @@ int attention_prompt_configure(lv_ctx* ctx) {
 }
 
 int launch_attention_prompt(lv_ctx* ctx, float* out, const float* q, const void* k_cache, const void* v_cache, const uint32_t* pos,
-                            const float* rope_table, uint32_t heads, uint32_t max_ctx, uint32_t batch) {
+                            const float* rope_table, uint32_t heads, uint32_t max_ctx, uint32_t batch, void* xh) {
     const uint32_t chunks = (max_ctx + kApKeys - 1) / kApKeys, C = std::min(kApMaxCluster, chunks);
     auto* kernel = chunks <= C ? attention_prompt_kernel<true> : attention_prompt_kernel<false>;
     LV_CUDA(launch_pdl_cluster(ctx, kernel, dim3(heads, C, (batch + kApQ - 1) / kApQ), dim3(kApThreads), dim3(1, C), kApSmemBytes, out, q,
                                static_cast<const __half*>(k_cache), static_cast<const __half*>(v_cache), pos, rope_table, heads, batch, max_ctx,
-                               1.0f / sqrtf(float(kApHead)), ctx->d_err));
+                               1.0f / sqrtf(float(kApHead)), ctx->d_err, static_cast<__half*>(xh), (batch + 15u) & ~15u));
     return LV_OK;
 }
 

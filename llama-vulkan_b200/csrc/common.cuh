@@ -235,6 +235,38 @@ __device__ __forceinline__ float silu_f32(float z) { return z / (1.f + expf(-z))
 // (for values that are rounded to bfloat16)
 __device__ __forceinline__ float silu_fast(float z) { return __fdividef(z, 1.f + __expf(-z)); }
 
+// Split activations (lv_act_split_f16): where the hi half of value (token z, column c) lies, in halves; its lo half is 64 zpad further on.  One
+// tile of 2 zpad rows x 64 columns after the other, each row's eight 16-byte units at unit ^ (row & 7).
+__device__ __forceinline__ size_t split_index(uint32_t zpad, uint32_t z, uint32_t c) {
+    return size_t(c >> 6) * 2 * zpad * 64 + size_t(z) * 64 + ((((c & 63u) >> 3) ^ (z & 7u)) << 3) + (c & 7u);
+}
+__device__ __forceinline__ void split_store(__half* xh, uint32_t zpad, uint32_t z, uint32_t c, float v) {
+    const size_t at = split_index(zpad, z, c);
+    const __half h = __float2half_rn(v);
+    xh[at] = h;
+    xh[at + size_t(zpad) * 64] = __float2half_rn(v - __half2float(h));
+}
+// N consecutive values from column c on, c a multiple of N (2 or 4)
+template <int N>
+__device__ __forceinline__ void split_store_n(__half* xh, uint32_t zpad, uint32_t z, uint32_t c, const float (&v)[N]) {
+    const size_t at = split_index(zpad, z, c);
+    uint32_t hi[N / 2], lo[N / 2];
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+        const __half h0 = __float2half_rn(v[2 * i]), h1 = __float2half_rn(v[2 * i + 1]);
+        const __half2 h = __halves2half2(h0, h1), l = __halves2half2(__float2half_rn(v[2 * i] - __half2float(h0)), __float2half_rn(v[2 * i + 1] - __half2float(h1)));
+        hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+        lo[i] = *reinterpret_cast<const uint32_t*>(&l);
+    }
+    if constexpr (N == 4) {
+        *reinterpret_cast<uint2*>(xh + at) = make_uint2(hi[0], hi[1]);
+        *reinterpret_cast<uint2*>(xh + at + size_t(zpad) * 64) = make_uint2(lo[0], lo[1]);
+    } else {
+        *reinterpret_cast<uint32_t*>(xh + at) = hi[0];
+        *reinterpret_cast<uint32_t*>(xh + at + size_t(zpad) * 64) = lo[0];
+    }
+}
+
 // Activation of a finished product (LV_ACT_* of lv_b200.h; 1: the square of relu).
 __device__ __forceinline__ float product_act(float v, int act) {
     if (act == 1) {

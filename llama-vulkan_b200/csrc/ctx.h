@@ -43,7 +43,7 @@ int gemv_configure(lv_ctx* ctx);
 int attention_configure(lv_ctx* ctx);
 int attention_prompt_configure(lv_ctx* ctx);
 int launch_attention_prompt(lv_ctx* ctx, float* out, const float* q, const void* k_cache, const void* v_cache, const uint32_t* pos,
-                            const float* rope_table, uint32_t heads, uint32_t max_ctx, uint32_t batch);      // attention_prompt.cu
+                            const float* rope_table, uint32_t heads, uint32_t max_ctx, uint32_t batch, void* xh = nullptr);      // attention_prompt.cu
 int gemm_tc_configure(lv_ctx* ctx);
 void gemm_tc_release(lv_ctx* ctx);
 int gemm_bf16_configure(lv_ctx* ctx);

@@ -681,6 +681,12 @@ int gemm_tc_configure(lv_ctx* ctx) {
     return gemm_tc_stream_configure(ctx);
 }
 
+// Which kernel takes a product: gemm_tc_stream.cu, unless exact tiles or tiles in shared memory were asked for.
+static bool tiles_in_tensor_memory(const lv_ctx* ctx, int wtype) {
+    static const char* smem_tiles = getenv("LV_GEMM_TC_SMEM_TILES");
+    return !ctx->tc_exact && !(wtype == T_Q4_0 && smem_tiles != nullptr && smem_tiles[0] == '1');
+}
+
 template <int QT>
 static int launch_gemm_tc_typed(lv_ctx* ctx, GemmTcParams& p, const __half* xh) {
     LV_REQUIRE(p.K != 0 && p.K % 256 == 0, "cols must be a non-zero multiple of 256");
@@ -706,9 +712,7 @@ static int launch_gemm_tc_typed(lv_ctx* ctx, GemmTcParams& p, const __half* xh) 
     p.scratch = static_cast<float*>(ctx->tc_scratch);
     p.counters = static_cast<uint32_t*>(ctx->tc_counters);
     const bool fast = !ctx->tc_exact;
-    static const char* smem_tiles = getenv("LV_GEMM_TC_SMEM_TILES");
-    const bool in_smem = QT == T_Q4_0 && smem_tiles != nullptr && smem_tiles[0] == '1';
-    if (fast && !in_smem) return launch_gemm_tc_stream(ctx, p, maps, QT, tiles);
+    if (tiles_in_tensor_memory(ctx, QT)) return launch_gemm_tc_stream(ctx, p, maps, QT, tiles);
     const uint32_t groups_all = p.K / (4 * kTcChunkK);
     uint32_t splits = 1;
     auto fits = [&](uint32_t s) {
@@ -798,6 +802,24 @@ extern "C" int lv_gemm_tc_silu(lv_ctx* ctx, float* out, const void* w3, const vo
     p.n_mat = 1;
     p.K = dim;
     p.Z = batch;
+    p.err = ctx->d_err;
+    return launch_gemm_tc(ctx, p, static_cast<const __half*>(xh), wtype);
+}
+
+extern "C" int lv_gemm_tc_silu_split(lv_ctx* ctx, void* xh_out, float* out, const void* w3, const void* w1, int wtype, const void* xh, uint32_t ff,
+                                     uint32_t dim, uint32_t batch) {
+    LV_ENTER(ctx);
+    LV_REQUIRE(xh_out && out && w3 && w1 && xh_out != xh && (reinterpret_cast<uintptr_t>(xh_out) & 15u) == 0 && ff % 64 == 0, "bad gemm_tc_silu_split arguments");
+    if (!tiles_in_tensor_memory(ctx, wtype)) {
+        if (int rc = lv_gemm_tc_silu(ctx, out, w3, w1, wtype, xh, ff, dim, batch)) return rc;
+        return lv_act_split_f16(ctx, xh_out, out, nullptr, ff, batch);
+    }
+    GemmTcParams p{};
+    p.m[0] = {static_cast<const uint8_t*>(w3), static_cast<const uint8_t*>(w1), out, ff, EPI_STORE};
+    p.n_mat = 1;
+    p.K = dim;
+    p.Z = batch;
+    p.split_out = static_cast<__half*>(xh_out);
     p.err = ctx->d_err;
     return launch_gemm_tc(ctx, p, static_cast<const __half*>(xh), wtype);
 }

@@ -37,6 +37,7 @@ struct GemmTcParams {
     float* scratch;          // splits > 1: partial accumulators [tile][split][zpad][128]
     uint32_t* counters;      // splits > 1: arrivals per tile (zero between launches)
     uint32_t* err;
+    __half* split_out;       // SiLU pairs, gemm_tc_stream.cu: finished rows go there as the split activations of the next product, not to m[0].out
     const lv_group_member* group;   // non-null: token z is member z of a group step; cache rows go to its own caches at its own position
 };
 

@@ -69,7 +69,9 @@ __device__ __forceinline__ __half* ts_cache_row(const GemmTcParams& p, const Gem
 
 // Stores one value / four consecutive rows of a token.  (mi: matrix of the launch)
 __device__ __forceinline__ void ts_store(const GemmTcParams& p, const GemvMatrix& M, int mi, uint32_t row, uint32_t z, float v) {
-    if (M.epilogue == EPI_STORE_F16_AT_POS) {
+    if (p.split_out != nullptr) {
+        split_store(p.split_out, p.zpad, z, row, v);
+    } else if (M.epilogue == EPI_STORE_F16_AT_POS) {
         if (__half* to = ts_cache_row(p, M, mi, z)) to[row] = __float2half_rn(v);
     } else {
         float* o = static_cast<float*>(M.out) + size_t(z) * M.rows + row;
@@ -77,6 +79,11 @@ __device__ __forceinline__ void ts_store(const GemmTcParams& p, const GemvMatrix
     }
 }
 __device__ __forceinline__ void ts_store4(const GemmTcParams& p, const GemvMatrix& M, int mi, uint32_t row, uint32_t z, float4 v) {
+    if (p.split_out != nullptr) {
+        const float x[4] = {v.x, v.y, v.z, v.w};
+        split_store_n<4>(p.split_out, p.zpad, z, row, x);
+        return;
+    }
     if (M.epilogue == EPI_STORE_F16_AT_POS) {
         __half* to = ts_cache_row(p, M, mi, z);
         if (to == nullptr) return;

@@ -101,8 +101,10 @@ bool llama_architecture::make_scratch(llava_session* s) {
     const size_t scratch = lv_attention_scratch_bytes(h.n_heads / ranks, h.rot, max_backlog_size, B);
     if (scratch == 0) return false;
     s->attn_scratch = new llava_buffer(ctx, F, u32((scratch + 3) / 4), 1, m);
-    if (B >= llava_command_buffer::kTensorCoreMinBatch)
+    if (B >= llava_command_buffer::kTensorCoreMinBatch) {
         s->act_split = new llava_buffer(ctx, F, u32(lv_act_split_bytes(max(max(dim, ff_len), vout_len), B) / 4), 1, m);
+        if (ranks == 1) s->ff_split = new llava_buffer(ctx, F, u32(lv_act_split_bytes(ff, B) / 4), 1, m);
+    }
     return true;
 }
 

@@ -233,6 +233,23 @@ void llava_command_buffer::gemm_silu_ff(llava_buffer* outbuf, llava_buffer* w3, 
                          w3->shape.second, batch_size));
 }
 
+// the same with outputs in the form that the next product reads
+void llava_command_buffer::attention_fused_split(llava_buffer* split, llava_buffer* query, llava_buffer* k_cache, llava_buffer* v_cache) {
+    const ggml_header& h = session->model->get_header();
+    if (!expect(query->shape.first == h.dim && k_cache->shape.second == h.dim && size_t(split->shape.first) * 4 >= lv_act_split_bytes(h.dim, batch_size),
+                "attention shapes")) return;
+    note(lv_attention_fused_split(lv(), split->device_ptr(), f32(query), k_cache->device_ptr(), v_cache->device_ptr(),
+                                  static_cast<u32*>(session->config_buffer->device_ptr()), session->ctx->rope_table,
+                                  session->attn_scratch->device_ptr(), h.n_heads, h.rot, backlog_size, batch_size));
+}
+
+void llava_command_buffer::gemm_silu_split(llava_buffer* split_out, llava_buffer* outbuf, llava_buffer* w3, llava_buffer* w1, llava_buffer* split) {
+    if (!expect(w3->shape == w1->shape && w3->type == w1->type && outbuf->shape.first >= w3->shape.first &&
+                size_t(split_out->shape.first) * 4 >= lv_act_split_bytes(w3->shape.first, batch_size), "gemm_silu_split shapes")) return;
+    note(lv_gemm_tc_silu_split(lv(), split_out->device_ptr(), f32(outbuf), w3->device_ptr(), w1->device_ptr(), w3->kernel_type(), split->device_ptr(),
+                               w3->shape.first, w3->shape.second, batch_size));
+}
+
 void llava_command_buffer::tp_arm_push(u32 exchange) {
     note(lv_tp_arm_push(lv(), int(exchange), 2 * u32(session->ctx->get_layers().size())));
 }

@@ -63,6 +63,8 @@ public:
     void gemm_qkv_kvappend(llava_buffer* q_out, llava_buffer* k_cache, llava_buffer* v_cache, llava_buffer* wq, llava_buffer* wk,
                            llava_buffer* wv, llava_buffer* split);
     void gemm_add_inplace(llava_buffer* outbuf, llava_buffer* matrix, llava_buffer* split);
+    void attention_fused_split(llava_buffer* split, llava_buffer* query, llava_buffer* k_cache, llava_buffer* v_cache);
+    void gemm_silu_split(llava_buffer* split_out, llava_buffer* outbuf, llava_buffer* w3_matrix, llava_buffer* w1_matrix, llava_buffer* split);
     void gemm_silu_ff(llava_buffer* outbuf, llava_buffer* w3_matrix, llava_buffer* w1_matrix, llava_buffer* split);
 
     int status() const { return first_error; }

@@ -82,13 +82,13 @@ llava_buffer* llava_layer::execute(llava_command_buffer* cmd_buf, llava_layer_se
         // it is not tracing (llava_layer.cpp:45-51)
         llava_buffer* x = session->current_thought;
         if (cmd_buf->use_tensor_cores(attention_wq)) {
-            // six or more tokens: every matrix is read once for the whole batch (tcgen05), nine launches
+            // six or more tokens: every matrix is read once for the whole batch (tcgen05), seven launches
             llava_buffer* split = session->act_split;
             cmd_buf->act_split(split, x, attention_norm);
             cmd_buf->gemm_qkv_kvappend(session->current_Q, layer_data->k_cache, layer_data->v_cache, attention_wq, attention_wk,
                                        attention_wv, split);
-            cmd_buf->attention_fused(session->current_Vout, session->current_Q, layer_data->k_cache, layer_data->v_cache);
             if (context->tp_size() > 1) {
+                cmd_buf->attention_fused(session->current_Vout, session->current_Q, layer_data->k_cache, layer_data->v_cache);
                 // this rank's heads and FFN rows; the column shards of wo and w2 have rows padded with zero blocks, so
                 // their (dense) inputs are padded while they are split; the partial products of all tokens are summed
                 // over the ranks by one exchange per sub-block
@@ -102,12 +102,11 @@ llava_buffer* llava_layer::execute(llava_command_buffer* cmd_buf, llava_layer_se
                 cmd_buf->allreduce_add(x, session->tp_partial);
                 return x;
             }
-            cmd_buf->act_split(split, session->current_Vout, nullptr);
+            cmd_buf->attention_fused_split(split, session->current_Q, layer_data->k_cache, layer_data->v_cache);
             cmd_buf->gemm_add_inplace(x, attention_wo, split);
             cmd_buf->act_split(split, x, ffn_norm);
-            cmd_buf->gemm_silu_ff(session->main_ff_result, feed_forward_w3, feed_forward_w1, split);
-            cmd_buf->act_split(split, session->main_ff_result, nullptr);
-            cmd_buf->gemm_add_inplace(x, feed_forward_w2, split);
+            cmd_buf->gemm_silu_split(session->ff_split, session->main_ff_result, feed_forward_w3, feed_forward_w1, split);
+            cmd_buf->gemm_add_inplace(x, feed_forward_w2, session->ff_split);
             return x;
         }
         if (context->tp_size() > 1 && context->fused_exchange() && layer_id > 0) {

@@ -150,7 +150,7 @@ bool llava_session::recreate_buffers() {
 void llava_session::reset_main_buffers() {
     for (llava_buffer** b : {&current_thought, &current_thought_sublayer, &current_thought_middle_normd, &current_Q, &current_K,
                              &current_V, &current_Vout, &main_attn_result, &config_buffer, &output_probs, &main_ff_result,
-                             &token_log, &argmax_result, &attn_scratch, &tp_partial, &act_split, &sampler_state}) {
+                             &token_log, &argmax_result, &attn_scratch, &tp_partial, &act_split, &ff_split, &sampler_state}) {
         delete *b;
         *b = nullptr;
     }

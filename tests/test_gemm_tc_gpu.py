@@ -286,3 +286,64 @@ def test_gemm_tc_silu_pair_on_the_shards_of_eight_ranks(gpu, pkg, ff, dim, batch
     for z in list(range(0, batch, 13)) + [batch - 1]:
         close(got[z], ob.gemv_silu(w3, w1, qn.Q4_0, ob.norm(x[z], nw), ff, dim, workers_for(dim)), **loose(form, qn.Q4_0))
     assert (got[batch] == 7.0).all()                                     # the ragged tile wrote nothing past the matrix
+
+
+@pytest.mark.parametrize("wtype", [qn.Q4_0, qn.Q8_0], ids=["q4_0", "q8_0"])
+@pytest.mark.parametrize("rows,cols,batch", [(32, 256, 64), (160, 256, 17), (4096, 256, 48), (19008, 512, 33), (4096, 2816, 64), (992, 5120, 1), (131200, 256, 6)])
+def test_gemm_tc_runs_of_units(gpu, pkg, rows, cols, batch, wtype, form):
+    """Every SM takes an equal run of (row tile, 256 columns): tiles of one unit, runs inside a tile, over several whole tiles and over the
+    edges of tiles, more tiles than arrival counters (whole tiles only).  Against float64 with the weights rounded to fp16, which is what
+    this form multiplies: left are 22-bit activations (2^-23 each) and f32 sums, below 1e-5 of the result."""
+    if form == "exact":
+        pytest.skip("another kernel")
+    rng = np.random.default_rng(rows + batch)
+    W = np.tile(matrix(rng, 32, cols, wtype=wtype).reshape(32, -1), (rows // 32, 1))
+    W = W[rng.permutation(rows)]
+    x = rng.standard_normal((batch, cols)).astype(np.float32)
+    out = gpu.zeros(batch * rows * 4)
+    dW = gpu.upload(W)
+    want = rounded_weights_product(W.reshape(-1), x, rows, cols, wtype)
+    for add in (0, 1):
+        pkg.check(gpu.lib.lv_gemm_tc(gpu.handle, out, dW, wtype, split(gpu, pkg, x), rows, cols, batch, add))
+        gpu.sync()
+        close(gpu.download(out, np.float32, batch * rows).reshape(batch, rows), (1 + add) * want, rel_l2=1e-5, max_abs_frac=1e-5)
+    gpu.free(dW)
+    gpu.free(out)
+
+
+@pytest.mark.parametrize("wtype", [qn.Q4_0, qn.Q8_0], ids=["q4_0", "q8_0"])
+@pytest.mark.parametrize("ff,dim,batch", [(64, 256, 1), (192, 512, 16), (11008, 4096, 37), (2048, 1024, 64)])
+def test_gemm_tc_silu_split_is_the_split_of_its_rows(gpu, pkg, ff, dim, batch, wtype, form):
+    rng = np.random.default_rng(ff + batch)
+    w3, w1 = gpu.upload(matrix(rng, ff, dim, wtype=wtype)), gpu.upload(matrix(rng, ff, dim, wtype=wtype))
+    xh = split(gpu, pkg, rng.standard_normal((batch, dim)).astype(np.float32))
+    out, nbytes, zpad = gpu.zeros(batch * ff * 4), gpu.lib.lv_act_split_bytes(ff, batch), (batch + 15) // 16 * 16
+    fused, apart = gpu.zeros(nbytes), gpu.zeros(nbytes)
+    pkg.check(gpu.lib.lv_gemm_tc_silu_split(gpu.handle, fused, out, w3, w1, wtype, xh, ff, dim, batch))
+    pkg.check(gpu.lib.lv_gemm_tc_silu(gpu.handle, out, w3, w1, wtype, xh, ff, dim, batch))
+    pkg.check(gpu.lib.lv_act_split_f16(gpu.handle, apart, out, None, ff, batch))
+    gpu.sync()
+    got, want = ([p[:batch] for p in planes_of(gpu.download(d, np.float16, nbytes // 2), zpad, ff)] for d in (fused, apart))
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    assert gpu.lib.lv_gemm_tc_silu_split(gpu.handle, xh, out, w3, w1, wtype, xh, ff, dim, batch) == pkg.LV_ERR_BAD_ARGUMENTS
+
+
+@pytest.mark.parametrize("batch,pos,max_ctx", [(3, 20, 128), (3, 300, 512), (7, 700, 1024), (12, 5, 128), (37, 364, 512), (64, 64, 128), (64, 1900, 2048)])
+def test_attention_split_is_the_split_of_its_outputs(gpu, pkg, batch, pos, max_ctx, form):
+    if form == "exact":
+        pytest.skip("no products here")
+    heads, dim, lib, h = 8, 1024, gpu.lib, gpu.handle
+    rng = np.random.default_rng(pos)
+    k, v = (gpu.upload((0.7 * rng.standard_normal((max_ctx, dim))).astype(np.float16)) for _ in range(2))
+    q, at = gpu.upload(rng.standard_normal((batch, dim)).astype(np.float32)), gpu.upload(np.full(4, pos, np.uint32))
+    table = gpu.alloc(2048 * 128 * 4)
+    pkg.check(lib.lv_rope_table_build(h, table, 2048, 128))
+    scratch = gpu.zeros(lib.lv_attention_scratch_bytes(heads, 128, max_ctx, batch))
+    out, nbytes, zpad = gpu.zeros(batch * dim * 4), lib.lv_act_split_bytes(dim, batch), (batch + 15) // 16 * 16
+    fused, apart = gpu.zeros(nbytes), gpu.zeros(nbytes)
+    pkg.check(lib.lv_attention_fused_split(h, fused, q, k, v, at, table, scratch, heads, 128, max_ctx, batch))
+    pkg.check(lib.lv_attention_fused(h, out, q, k, v, at, table, scratch, heads, 128, max_ctx, batch))
+    pkg.check(lib.lv_act_split_f16(h, apart, out, None, dim, batch))
+    gpu.sync()
+    got, want = ([p[:batch] for p in planes_of(gpu.download(d, np.float16, nbytes // 2), zpad, dim)] for d in (fused, apart))
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])

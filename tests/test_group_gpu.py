@@ -6,6 +6,8 @@ prompt evaluated in batches: with exact weight tiles the decode tolerance (1e-2 
 with the default fast tiles rel-L2 <= 3e-3 and the same token unless the oracle's two best logits are closer than the
 logits differ.  The per-member references are the oracle's trajectories.
 """
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -186,8 +188,7 @@ def test_group_members_that_sample_draw_with_their_own_sampler(pkg, world):
 
 @pytest.mark.parametrize("n", [1, 2, 33, 64])
 def test_group_feed_sets_tokens_and_moved_positions(gpu, pkg, n):
-    """lv_group_feed: tokens at their places of the members' logs, position words of moved members only; a place beyond the log is
-    reported and not written."""
+    """lv_group_feed: tokens at their places of the members' logs, position words of moved members only."""
     cap, lib, h = 9, gpu.lib, gpu.handle
     words = gpu.upload(np.full(n * (4 + cap + 1), 7, np.uint32))                     # per member: pos[4], log[cap], a guard
     base = words.value if hasattr(words, "value") else int(words)
