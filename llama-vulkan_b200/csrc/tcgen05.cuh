@@ -72,4 +72,47 @@ __device__ __forceinline__ void tc_free(uint32_t base, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
 }
 
+// ---- two CTAs of a cluster on one tile (cta_group::2) --------------------------------------------------------------
+// Ranks 2n and 2n + 1 of a cluster are a pair.  A product of M = 256 rows and N columns takes 128 rows of A and N / 2 rows of B from each
+// CTA's shared memory (the same offsets in both) and leaves 128 rows x N columns in each CTA's tensor memory; one thread of the first
+// CTA issues it.
+
+// A tiled load into this CTA's shared memory that counts its bytes on a barrier of either CTA of the pair (a shared::cluster address).
+__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const void* tensor_map, int x, int y, uint32_t cluster_bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(smem_u32(smem_dst)), "l"(tensor_map), "r"(x), "r"(y), "r"(cluster_bar)
+        : "memory");
+}
+
+// Arrives at the barrier of the same offset in the CTAs of `mask` when this thread's products are done.
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar, uint32_t mask) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"(static_cast<unsigned short>(mask)) : "memory");
+}
+
+// The products of tc_mma_f16, or those of a pair.
+template <bool TWO>
+__device__ __forceinline__ void tc_mma_16bit(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    if constexpr (TWO) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+            : "memory");
+    } else {
+        tc_mma_f16(tmem_d, a_desc, b_desc, idesc, accumulate);
+    }
+}
+
+// Allocation and release for a pair: one warp of each CTA.
+__device__ __forceinline__ void tc_alloc_pair(uint32_t* slot, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tc_free_pair(uint32_t base, uint32_t cols) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
+}
+
 }  // namespace lv
