@@ -479,7 +479,9 @@ int lv_mingru_scan(lv_ctx* ctx, void* out, int out_type, uint32_t out_ld, const 
 /* Feed-forward experts chosen by token id: table u32 [vocab][top] gives every id its experts.  w0 (and w1) are the experts'
  * matrices stacked, [experts * rows][ld].
  *   gate_up: out[t * top + s] = silu(gate_e x[t]) * (up_e x[t]), e = table[id_t][s] (w0 gate, w1 up; rows = ff, cols = width)
- *   down:    out[t] = (1 / top) sum_s down_e x[t * top + s]                        (w0 down; rows = width, cols = ff) */
+ *   down:    out[t] = (1 / top) sum_s down_e x[t * top + s]                        (w0 down; rows = width, cols = ff)
+ * One token: *pos, its entry of the log and the table are read before earlier launches of the stream have finished, and again after them;
+ * whatever *pos holds meanwhile has to be a place of the log. */
 typedef struct lv_expert_args {
     const void* w0;
     const void* w1;

@@ -49,10 +49,15 @@ __device__ __forceinline__ void gb_fma(float& acc, uint4 w, const float (&x)[8])
     }
 }
 
+struct GbSettled {
+    __device__ __forceinline__ bool operator()() const { return false; }
+};
+
 // Partial dot products of NR rows with x over this lane's share of K.  WAIT: the rows are known before the previous kernel
-// has finished and their first elements are requested before waiting for it.
-template <int NR, bool WAIT>
-__device__ __forceinline__ void gb_dot(float (&acc)[NR], const __nv_bfloat16* const (&row)[NR], const float* x, uint32_t K) {
+// has finished and their first elements are requested before waiting for it.  settle: called after the wait; true: it has changed the rows
+// (which were only a guess) and their first elements are requested again.
+template <int NR, bool WAIT, typename Settle = GbSettled>
+__device__ __forceinline__ void gb_dot(float (&acc)[NR], const __nv_bfloat16* const (&row)[NR], const float* x, uint32_t K, Settle settle = Settle()) {
     const uint32_t lane8 = (threadIdx.x & 31u) * 8u;
     uint4 w[kGbUnroll][NR];
     auto fetch = [&](uint32_t k0) {
@@ -65,6 +70,7 @@ __device__ __forceinline__ void gb_dot(float (&acc)[NR], const __nv_bfloat16* co
     };
     fetch(0);
     if constexpr (WAIT) pdl_wait();
+    if (settle()) fetch(0);
     for (uint32_t k0 = 0; k0 < K; k0 += 256u * kGbUnroll) {
 #pragma unroll
         for (int u = 0; u < kGbUnroll; ++u) {
@@ -155,35 +161,89 @@ __device__ __forceinline__ uint32_t gb_expert(const ExpertGemvParams& p, uint32_
     return 0;
 }
 
+// The same before the previous kernel has finished: a guess.  The position and the token are those of the step unless an earlier launch
+// that is still running writes them; whoever uses the guess asks again after the wait.  One token only (a position is always inside the log,
+// the tokens behind it may not be).
+__device__ __forceinline__ uint32_t gb_expert_guess(const ExpertGemvParams& p, uint32_t slot) {
+    const uint32_t at = *reinterpret_cast<const volatile uint32_t*>(p.pos), id = *reinterpret_cast<const volatile uint32_t*>(p.token_log + at);
+    const uint32_t e = id < p.vocab ? p.table[size_t(id) * p.top + slot] : 0;
+    return e < p.experts ? e : 0;
+}
+
+// A token's experts are known when the step begins, so one token's weights are on their way while the norm before it runs (a single CTA):
+// half of a row of 2048 columns.
 __global__ void __launch_bounds__(kGbThreads) gemv_bf16_expert_gate_up_kernel(const ExpertGemvParams p) {
     pdl_launch_dependents();
     const uint32_t t = blockIdx.y, slot = blockIdx.z;
     const uint32_t i = blockIdx.x * kGbWarps + (threadIdx.x >> 5);
-    pdl_wait();
-    const uint32_t e = gb_expert(p, t, slot);
-    if (i >= p.rows) return;
-    const size_t at = (size_t(e) * p.rows + i) * p.ld;
-    const __nv_bfloat16* row[2] = {p.gate + at, p.up + at};
+    const __nv_bfloat16* row[2];
+    auto rows_of = [&](uint32_t e) {
+        const size_t at = (size_t(e) * p.rows + min(i, p.rows - 1)) * p.ld;
+        row[0] = p.gate + at;
+        row[1] = p.up + at;
+    };
     float acc[2] = {0.f, 0.f};
-    gb_dot<2, false>(acc, row, p.x + size_t(t) * p.x_ld, p.K);
+    if (gridDim.y == 1) {
+        const uint32_t guess = gb_expert_guess(p, slot);
+        rows_of(guess);
+        gb_dot<2, true>(acc, row, p.x, p.K, [&]() {
+            const uint32_t e = gb_expert(p, 0, slot);
+            if (e == guess) return false;
+            rows_of(e);
+            return true;
+        });
+    } else {
+        pdl_wait();
+        rows_of(gb_expert(p, t, slot));
+        gb_dot<2, false>(acc, row, p.x + size_t(t) * p.x_ld, p.K);
+    }
     const float g = warp_sum(acc[0]), u = warp_sum(acc[1]);
-    if ((threadIdx.x & 31u) == 0) p.out[(size_t(t) * p.top + slot) * p.out_ld + i] = silu_f32(g) * u;
+    if (i < p.rows && (threadIdx.x & 31u) == 0) p.out[(size_t(t) * p.top + slot) * p.out_ld + i] = silu_f32(g) * u;
 }
 
+// SHARE warps share two rows, each taking every SHARE-th expert of the token, and their sums are added in that order.  One warp for all
+// experts had their rows in flight one after the other: four experts of 2048 x 1408 took 17 us where HBM needs 3.5.
+template <int SHARE>
 __global__ void __launch_bounds__(kGbThreads) gemv_bf16_expert_down_kernel(const ExpertGemvParams p) {
     pdl_launch_dependents();
-    const uint32_t t = blockIdx.y;
-    const uint32_t r = 2u * (blockIdx.x * kGbWarps + (threadIdx.x >> 5));
-    pdl_wait();
-    if (r >= p.rows) return;
+    __shared__ float s_part[kGbWarps][2];
+    const uint32_t t = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, mine = warp % SHARE;
+    const uint32_t r = 2u * (blockIdx.x * (kGbWarps / SHARE) + warp / SHARE);
+    const __nv_bfloat16* row[2];
+    auto rows_of = [&](uint32_t e) {
+        const size_t first = size_t(e) * p.rows;
+        row[0] = p.gate + (first + min(r, p.rows - 1)) * p.ld;
+        row[1] = p.gate + (first + min(r + 1, p.rows - 1)) * p.ld;
+    };
+    const float* x = p.x + size_t(t) * p.top * p.x_ld;
     float acc[2] = {0.f, 0.f};
-    for (uint32_t s = 0; s < p.top; ++s) {
-        const size_t first = size_t(gb_expert(p, t, s)) * p.rows;
-        const __nv_bfloat16* row[2] = {p.gate + (first + r) * p.ld, p.gate + (first + min(r + 1, p.rows - 1)) * p.ld};
-        gb_dot<2, false>(acc, row, p.x + (size_t(t) * p.top + s) * p.x_ld, p.K);
+    uint32_t s = mine;                                       // (SHARE <= top)
+    if (gridDim.y == 1) {
+        const uint32_t guess = gb_expert_guess(p, s);
+        rows_of(guess);
+        gb_dot<2, true>(acc, row, x + size_t(s) * p.x_ld, p.K, [&]() {
+            const uint32_t e = gb_expert(p, 0, s);
+            if (e == guess) return false;
+            rows_of(e);
+            return true;
+        });
+        s += SHARE;
+    } else {
+        pdl_wait();
     }
-    const float a0 = warp_sum(acc[0]), a1 = warp_sum(acc[1]);
-    const uint32_t lane = threadIdx.x & 31u;
+    for (; s < p.top; s += SHARE) {
+        rows_of(gb_expert(p, t, s));
+        gb_dot<2, false>(acc, row, x + size_t(s) * p.x_ld, p.K);
+    }
+    float a0 = warp_sum(acc[0]), a1 = warp_sum(acc[1]);
+    if constexpr (SHARE > 1) {
+        if (lane == 0) { s_part[warp][0] = a0; s_part[warp][1] = a1; }
+        __syncthreads();
+        if (mine != 0) return;
+        a0 = a1 = 0.f;
+#pragma unroll
+        for (int k = 0; k < SHARE; ++k) { a0 += s_part[warp + k][0]; a1 += s_part[warp + k][1]; }
+    }
     if (lane < 2 && r + lane < p.rows) p.out[size_t(t) * p.out_ld + r + lane] = (lane ? a1 : a0) / float(p.top);
 }
 
@@ -253,6 +313,9 @@ extern "C" int lv_gemv_bf16_expert_down(lv_ctx* ctx, float* out, uint32_t out_ld
     if (const int rc = expert_params(a, &p)) return rc;
     LV_REQUIRE(out && x && gb_aligned(x) && batch && batch <= 65535 && out_ld >= p.rows && x_ld >= p.K && x_ld % 4 == 0, "bad expert_down arguments");
     p.x = x; p.x_ld = x_ld; p.out = out; p.out_ld = out_ld; p.err = ctx->d_err;
-    LV_CUDA(launch_pdl(ctx, gemv_bf16_expert_down_kernel, dim3((p.rows + 2 * kGbWarps - 1) / (2 * kGbWarps), batch), dim3(kGbThreads), 0, p));
+    // warps per pair of rows: as many as there are experts, a power of two up to four
+    const uint32_t share = p.top >= 4 ? 4 : p.top >= 2 ? 2 : 1, per_cta = 2 * kGbWarps / share;
+    auto* kernel = share == 4 ? gemv_bf16_expert_down_kernel<4> : share == 2 ? gemv_bf16_expert_down_kernel<2> : gemv_bf16_expert_down_kernel<1>;
+    LV_CUDA(launch_pdl(ctx, kernel, dim3((p.rows + per_cta - 1) / per_cta, batch), dim3(kGbThreads), 0, p));
     return LV_OK;
 }

@@ -65,6 +65,32 @@ def draw_table(rng, vocab, n, top):
     return np.stack([rng.permutation(n)[:top] for _ in range(vocab)]).astype(np.int32)
 
 
+@pytest.mark.parametrize("width,ff,n,top", [(64, 40, 3, 1), (2056, 1100, 5, 2), (72, 1032, 7, 3), (1030, 2200, 6, 4), (7, 24, 9, 5), (130, 64, 11, 9)])
+@pytest.mark.parametrize("late", [False, True])
+def test_experts_of_one_token(gpu, width, ff, n, top, late):
+    """One token: its experts are looked up before the launches ahead have finished and again after them; the down product's experts are
+    shared by one, two or four warps.  late: a launch just ahead moves the position, so an early look finds another token's experts."""
+    rng = np.random.default_rng(width + top)
+    vocab, pos = 50, 3
+    gate, up, down = weights(rng, n, ff, width), weights(rng, n, ff, width), weights(rng, n, width, ff)
+    table, ids = draw_table(rng, vocab, n, top), rng.integers(0, vocab, 1)
+    x = weights(rng, 1, width, scale=1.0)
+    want = sp.table_moe(x.astype(np.float64), ids, table, [(gate[e].astype(np.float64), up[e].astype(np.float64), down[e].astype(np.float64)) for e in range(n)])
+    with Dev(gpu) as d:
+        gu = expert_args(d, gate, up, ff, width, table, ids, pos, vocab)
+        dn = expert_args(d, down, None, width, ff, table, ids, pos, vocab)
+        xp = np.zeros((1, pad8(width)), np.float32)
+        xp[:, :width] = x
+        xp, act, out = d.f32(xp), d.zeros(top * pad8(ff) * 4), d.zeros(width * 4)
+        if late:
+            for a in (gu, dn):
+                a.pos = d.u32([pos - 1] * 4).value
+                d.call("lv_decode_advance", a.pos, None, None, 1, 0)
+        d.call("lv_gemv_bf16_expert_gate_up", act, pad8(ff), C.byref(gu), xp, pad8(width), 1)
+        d.call("lv_gemv_bf16_expert_down", out, width, C.byref(dn), act, pad8(ff), 1)
+        assert rel(d.get(out, (1, width)), want) < 2e-6
+
+
 @pytest.mark.parametrize("width,ff,n,top,batch", [(64, 40, 5, 2, 1), (48, 96, 3, 1, 2), (136, 72, 9, 3, 23), (64, 200, 4, 4, 70), (96, 32, 70, 2, 300),
                                                   (64, 64, 3, 2, 290)])
 def test_experts_chosen_by_token(gpu, width, ff, n, top, batch):
