@@ -347,3 +347,21 @@ def test_attention_split_is_the_split_of_its_outputs(gpu, pkg, batch, pos, max_c
     gpu.sync()
     got, want = ([p[:batch] for p in planes_of(gpu.download(d, np.float16, nbytes // 2), zpad, dim)] for d in (fused, apart))
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("batch,cols", [(1, 64), (3, 4096), (17, 4160), (64, 5120), (16, 8192), (5, 8256)])
+def test_act_split_of_normalised_rows(gpu, pkg, batch, cols, form):
+    """Rows that a thread block holds in registers (up to 8192 values, ragged in its threads) and longer ones.  22 bits of a value are left."""
+    if form == "exact":
+        pytest.skip("no products here")
+    rng = np.random.default_rng(cols)
+    x = (rng.standard_normal((batch, cols)) + 0.5).astype(np.float32)
+    w = (1 + 0.1 * rng.standard_normal(cols)).astype(np.float32)
+    zpad = (batch + 15) // 16 * 16
+    xh = split(gpu, pkg, x, w)
+    gpu.sync()
+    hi, lo = planes_of(gpu.download(xh, np.float16, 2 * zpad * cols), zpad, cols)
+    assert not hi[batch:].any() and not lo[batch:].any()
+    x64 = x.astype(np.float64)
+    want = x64 * w / np.sqrt(((x64 - x64.mean(1, keepdims=True)) ** 2).mean(1, keepdims=True))
+    close(hi[:batch] + lo[:batch], want, rel_l2=1e-6, max_abs_frac=1e-6)
