@@ -34,7 +34,7 @@ struct GemmTcParams {
     uint32_t ctx_rows;
     const __half* xh;        // split activations, one contiguous pre-swizzled B tile per 64 columns of K (act_split_kernel)
     uint32_t splits;         // CTAs that share one tile of rows, each taking a contiguous range of K
-    float* scratch;          // splits > 1: partial accumulators [tile][split][zpad][128]
+    float* scratch;          // splits > 1: partial accumulators [tile][split][zpad][128]; gemm_tc_stream.cu: [CTA][first, last tile][zpad][128]
     uint32_t* counters;      // splits > 1: arrivals per tile (zero between launches)
     uint32_t* err;
     __half* split_out;       // SiLU pairs, gemm_tc_stream.cu: finished rows go there as the split activations of the next product, not to m[0].out

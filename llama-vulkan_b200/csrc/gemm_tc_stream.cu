@@ -21,8 +21,13 @@
 //   16     raw ring: 2-D tensor-map loads of q4_0 / q8_0 rows.
 //   17, 18 one lane each issues tcgen05.mma: tiles 0 and 1 of a group into accumulator bank 0, tiles 2 and 3 into bank 1 (two fp32
 //          chains of half the length); N = 2 zpad columns: the activations' hi and lo planes.
-//   19     activation ring: one bulk copy per two tiles of K (q8_0, whose raw stages are larger: one).  The number of stages is even, so that a stage always belongs to one
-//          issuing lane (a parity wait cannot tell a phase from the one two uses later).
+//   19     activation ring: one bulk copy per two tiles of K (q8_0, whose raw stages are larger: one).  The number of stages is even, so that
+//          a stage always belongs to one issuing lane (a parity wait cannot tell a phase from the one two uses later).
+//
+// us per launch, one CTA per tile and share of K -> this, 16 / 64 tokens of q4_0: 11008 x 4096 pair 42.9 -> 33.4 / 47.7 -> 40.9, 4096 x 11008 22.0 ->
+// 17.1 / 24.2 -> 24.0, 4096 x 4096 10.2 -> 10.6 / 12.0 -> 12.5 back to back; behind a smaller kernel the set-up is hidden (a prompt of 1024 tokens,
+// 7B q4_0: 91.5 -> 83.4 ms).  A unit takes about 1700 clocks: 700 of dequantisation, 450 of waiting for and fetching raw words, 90 of tcgen05.st, the
+// rest loop, barriers and drains; the tensor pipe needs 1024 of them at 64 tokens.
 //
 // Every wait is bounded (common.cuh); a lost wait sets the context's error word, the CTA drains and frees its tensor memory.
 #include <cstdlib>
