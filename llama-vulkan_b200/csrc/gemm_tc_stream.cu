@@ -24,8 +24,8 @@
 //   19     activation ring: one bulk copy per two tiles of K (q8_0, whose raw stages are larger: one).  The number of stages is even, so that
 //          a stage always belongs to one issuing lane (a parity wait cannot tell a phase from the one two uses later).
 //
-// us per launch, one CTA per tile and share of K -> this, 16 / 64 tokens of q4_0: 11008 x 4096 pair 42.9 -> 33.4 / 47.7 -> 40.9, 4096 x 11008 22.0 ->
-// 17.1 / 24.2 -> 24.0, 4096 x 4096 10.2 -> 10.6 / 12.0 -> 12.5 back to back; behind a smaller kernel the set-up is hidden (a prompt of 1024 tokens,
+// us per launch, one CTA per tile and share of K -> this, 16 / 64 tokens of q4_0: 11008 x 4096 pair 42.9 -> 35.7 / 47.7 -> 43.6, 4096 x 11008 22.0 ->
+// 17.5 / 24.2 -> 24.1, 4096 x 4096 10.2 -> 10.7 / 12.0 -> 12.5 back to back; behind a smaller kernel the set-up is hidden (a prompt of 1024 tokens,
 // 7B q4_0: 91.5 -> 83.4 ms).  A unit takes about 1700 clocks: 700 of dequantisation, 450 of waiting for and fetching raw words, 90 of tcgen05.st, the
 // rest loop, barriers and drains; the tensor pipe needs 1024 of them at 64 tokens.
 //
