@@ -60,6 +60,13 @@ __device__ __forceinline__ void ap_split(float x, float y, uint32_t& hi, uint32_
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
+// the two halves of w, 0 in place of one that is not finite
+__device__ __forceinline__ uint32_t ap_finite(uint32_t w) {
+    if ((w & 0x7c00u) == 0x7c00u) w &= 0xffff0000u;
+    if ((w & 0x7c000000u) == 0x7c000000u) w &= 0x0000ffffu;
+    return w;
+}
+
 // four floats in the shared memory of another CTA of the cluster
 __device__ __forceinline__ float4 ap_cluster_load4(const float* local, uint32_t rank) {
     uint32_t at;
@@ -300,12 +307,33 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
         }
         // ---- values: warp w owns dims 16 w ..; a step is the 16 keys of one warp ---------------------------------------
         const uint32_t steps = min(uint32_t(kApWarps), (last - p0) / 16 + 1);
+        auto load_values = [&](uint32_t (&b)[4], uint32_t ks) {
+            const uint32_t vrow = smem_u32(s_v + (16 * ks + (lane & 15)) * kApStride + (16 * warp + (lane >> 4) * 8) * 2);
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"(vrow) : "memory");
+        };
+        // A row must not depend on keys behind it, and a probability of 0 does not take a value out of a product that is not finite (an entry
+        // of the cache that left the range of f16).  So a warp looks for such values in chunks with keys that some row does not see, leaves
+        // them out of the products and adds them below to the rows that see them.
+        bool odd = false;
+        if (p0 + kApKeys - 1 > P) {
+            __half2 nan = __float2half2_rn(0.f);
+            for (uint32_t ks = 0; ks < steps; ++ks) {
+                uint32_t b[4];
+                load_values(b, ks);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) nan = __hfma2(*reinterpret_cast<const __half2*>(&b[i]), __float2half2_rn(0.f), nan);
+            }
+            odd = __any_sync(0xffffffffu, __hisnan(__low2half(nan)) || __hisnan(__high2half(nan)));
+        }
 #pragma unroll
         for (uint32_t ks = 0; ks < uint32_t(kApWarps); ++ks) {
             if (ks >= steps) break;
             uint32_t b[4];
-            const uint32_t vrow = smem_u32(s_v + (16 * ks + (lane & 15)) * kApStride + (16 * warp + (lane >> 4) * 8) * 2);
-            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"(vrow) : "memory");
+            load_values(b, ks);
+            if (odd) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) b[i] = ap_finite(b[i]);
+            }
 #pragma unroll
             for (int i = 0; i < 4; i += 2) {
                 if (uint32_t(i) >= n_mt) break;
@@ -316,6 +344,28 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
                 for (int j = 0; j < 2; ++j) { ap_mma(o[i][j], al0, b[2 * j], b[2 * j + 1]); ap_mma(o[i + 1][j], al1, b[2 * j], b[2 * j + 1]); }
 #pragma unroll
                 for (int j = 0; j < 2; ++j) { ap_mma(o[i][j], ah0, b[2 * j], b[2 * j + 1]); ap_mma(o[i + 1][j], ah1, b[2 * j], b[2 * j + 1]); }
+            }
+        }
+        if (odd) {
+            for (uint32_t k = 0; k < 16 * steps; ++k) {
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const uint32_t v = *reinterpret_cast<const uint32_t*>(s_v + k * kApStride + 2 * (16 * warp + 8 * j + 2 * t));
+                    const uint32_t f = v ^ ap_finite(v);            // what was left out
+                    if (f == 0) continue;
+                    const float2 x = __half22float2(*reinterpret_cast<const __half2*>(&f));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            if (uint32_t(i) >= n_mt || p0 + k > P + 16 * i + g + 8 * u) continue;
+                            // the probability of row 16 i + g + 8 u and key k in the fragments
+                            const uint8_t* at = s_k + ((i * 8 + (k >> 4)) * 32 + 4 * g + ((k & 7) >> 1)) * 16 + (2 * ((k >> 3) & 1) + u) * 4 + 2 * (k & 1);
+                            const float e = __half2float(*reinterpret_cast<const __half*>(at)) + __half2float(*reinterpret_cast<const __half*>(at + kApPlane));
+                            if ((f & 0xffffu) != 0) o[i][j][2 * u] = fmaf(e, x.x, o[i][j][2 * u]);
+                            if ((f >> 16) != 0) o[i][j][2 * u + 1] = fmaf(e, x.y, o[i][j][2 * u + 1]);
+                        }
+                }
             }
         }
         __syncthreads();                                            // values and probabilities are used up

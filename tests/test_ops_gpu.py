@@ -403,6 +403,35 @@ def test_prompt_attention(gpu, pkg, rope_table, batch, pos, max_ctx):
         gpu.free(d)
 
 
+@pytest.mark.parametrize("batch,pos,max_ctx", [(64, 0, 128), (50, 100, 256), (64, 448, 512), (70, 90, 256)])
+def test_prompt_attention_rows_do_not_depend_on_later_values(gpu, pkg, rope_table, batch, pos, max_ctx):
+    """Values of the cache that are not finite (the append rounds to f16) reach the rows that see them, and no row before: against the same
+    caches with 0 in their place every other output has the same bits."""
+    rng = np.random.default_rng(600 + batch)
+    k, v = _caches(rng, pos + batch, max_ctx)
+    odd = [(pos + 3, 5, np.inf), (pos + 20, 5 + ROT, -np.inf), (pos + 21, 2 * ROT + 77, np.nan), (pos + batch - 1, 9, np.inf), (pos + batch - 1, 7 * ROT + 64, np.nan)]
+    q = rng.standard_normal((batch, DIM)).astype(np.float32)
+    dk, dq, at = gpu.upload(k), gpu.upload(q), u32_dev(gpu, pos)
+    scratch, d_out = gpu.zeros(gpu.lib.lv_attention_scratch_bytes(HEADS, ROT, max_ctx, batch)), gpu.alloc(batch * DIM * 4)
+    got = []
+    for put in (False, True):
+        w = v.copy().view(np.float16)
+        for row, col, x in odd:
+            w[row, col] = x if put else 0
+        dv = gpu.upload(w)
+        pkg.check(gpu.lib.lv_attention_fused(gpu.handle, d_out, dq, dk, dv, at, rope_table, scratch, HEADS, ROT, max_ctx, batch))
+        gpu.sync()
+        got.append(gpu.download(d_out, np.float32, batch * DIM).reshape(batch, DIM))
+        gpu.free(dv)
+    sees = np.zeros((batch, DIM), bool)
+    for row, col, _ in odd:
+        sees[row - pos:, col] = True
+    assert not np.isfinite(got[1][sees]).any()
+    assert np.array_equal(got[0][~sees].view(np.uint32), got[1][~sees].view(np.uint32))
+    for d in (dk, dq, at, scratch, d_out):
+        gpu.free(d)
+
+
 def test_prompt_attention_leaves_out_rows_outside_the_cache(gpu, pkg, rope_table):
     rng = np.random.default_rng(34)
     batch, pos, max_ctx = 20, 245, 256                      # rows 0 .. 10 lie inside
