@@ -368,6 +368,7 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
                 }
             }
         }
+        if (!ONE_PASS) fence_proxy_async();                         // the next keys come by bulk copies into bytes that were written by stores
         __syncthreads();                                            // values and probabilities are used up
         if (ONE_PASS) break;
         if (chunk + C < n_chunks) {

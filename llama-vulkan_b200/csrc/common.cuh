@@ -98,6 +98,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t* err) {
     uint32_t ok = 1;
     if ((threadIdx.x & 31u) == 0) ok = mbar_wait(bar, parity, err) ? 1u : 0u;
+    __syncwarp();                                        // what the lane has seen to be there is there for all (a shuffle orders no memory)
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 

@@ -432,6 +432,29 @@ def test_prompt_attention_rows_do_not_depend_on_later_values(gpu, pkg, rope_tabl
         gpu.free(d)
 
 
+def test_prompt_attention_of_several_passes_repeats_itself(gpu, pkg, rope_table):
+    """More than 1024 positions: a CTA brings new keys to where it kept probabilities.  The same bits from every launch, and the first
+    rows of a step the same bits as in a shorter one."""
+    rng = np.random.default_rng(35)
+    batch, pos, max_ctx = 64, 1900, 2048
+    k, v = _caches(rng, pos + batch, max_ctx)
+    q = rng.standard_normal((batch, DIM)).astype(np.float32)
+    dk, dv, dq, at = gpu.upload(k), gpu.upload(v), gpu.upload(q), u32_dev(gpu, pos)
+    scratch, n = gpu.zeros(gpu.lib.lv_attention_scratch_bytes(HEADS, ROT, max_ctx, batch)), batch * DIM
+    outs = [gpu.alloc(n * 4) for _ in range(20)]
+    for d in outs:
+        pkg.check(gpu.lib.lv_attention_fused(gpu.handle, d, dq, dk, dv, at, rope_table, scratch, HEADS, ROT, max_ctx, batch))
+    part = gpu.alloc(n * 4)
+    pkg.check(gpu.lib.lv_attention_fused(gpu.handle, part, dq, dk, dv, at, rope_table, scratch, HEADS, ROT, max_ctx, batch // 2))
+    gpu.sync()
+    first = gpu.download(outs[0], np.uint32, n)
+    for d in outs[1:]:
+        assert np.array_equal(first, gpu.download(d, np.uint32, n))
+    assert np.array_equal(first[:n // 2], gpu.download(part, np.uint32, n // 2))
+    for d in outs + [dk, dv, dq, at, scratch, part]:
+        gpu.free(d)
+
+
 def test_prompt_attention_leaves_out_rows_outside_the_cache(gpu, pkg, rope_table):
     rng = np.random.default_rng(34)
     batch, pos, max_ctx = 20, 245, 256                      # rows 0 .. 10 lie inside
