@@ -497,6 +497,8 @@ int lv_gemv_bf16_expert_down(lv_ctx* ctx, float* out, uint32_t out_ld, const lv_
  * x [batch][x_ld] with x_ld a multiple of 8; out f32 or bfloat16 [batch][out_ld]. */
 int lv_gemm_bf16(lv_ctx* ctx, void* out, int out_type, uint32_t out_ld, const void* w, uint32_t rows, uint32_t ld, uint32_t cols,
                  const void* x, uint32_t x_ld, uint32_t batch, float factor, int act);
+/* How this context cuts such a product: plan[0] tokens of a tile, plan[1] CTAs that share a tile's products, plan[2] shares of K. */
+int lv_gemm_bf16_plan(lv_ctx* ctx, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t* plan);
 /* The same for the rows of a cache [x_rows][x_ld] that `batch` tokens at *pos see through a window of `window` positions (0: all):
  * out row i = W times cache row first + i, first = max(0, *pos + 1 - window), for all rows below *pos + batch.  max_rows: upper
  * bound of the number of rows, sizes the grid. */

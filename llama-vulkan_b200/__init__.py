@@ -156,6 +156,7 @@ KERNEL_API = {
     "lv_gemv_bf16_expert_gate_up": (_int, [_p, _p, _u32, C.POINTER(ExpertArgs), _p, _u32, _u32]),
     "lv_gemv_bf16_expert_down": (_int, [_p, _p, _u32, C.POINTER(ExpertArgs), _p, _u32, _u32]),
     "lv_gemm_bf16": (_int, [_p, _p, _int, _u32, _p, _u32, _u32, _u32, _p, _u32, _u32, _f32, _int]),
+    "lv_gemm_bf16_plan": (_int, [_p, _u32, _u32, _u32, C.POINTER(_u32)]),
     "lv_gemm_bf16_window": (_int, [_p, _p, _int, _u32, _p, _u32, _u32, _u32, _p, _u32, _u32, _p, _u32, _u32, _u32]),
     "lv_expert_tile_rows": (_u32, [_u32, _u32, _u32]),
     "lv_expert_max_tiles": (_u32, [_u32, _u32, _u32]),

@@ -235,18 +235,18 @@ __global__ void __launch_bounds__(kBgThreads, 2) gemm_bf16_kernel(const GemmBf16
         tc_fence_before_sync();
     }
     __syncthreads();
+    // Of a pair, either CTA's release may ask for both: not before both have read their accumulators.  Nor does a CTA leave while the other
+    // one's products or signals may reach it; of a split, the partial sums of all CTAs are in place.
+    if (TWO || p.splits > 1) {
+        __syncwarp();
+        cluster_sync();
+    }
     if (warp == 1) {
         tc_fence_after_sync();
         if constexpr (TWO) tc_free_pair(tmem, kCols);
         else tc_free(tmem, kCols);
     }
-    if (TWO && p.splits == 1) {                               // no CTA leaves while the other one's products or signals may reach it
-        __syncwarp();
-        cluster_sync();
-    }
     if (p.splits > 1) {
-        __syncwarp();
-        cluster_sync();                                   // the partial sums of all CTAs are in place
         // a warp has whole tokens, a lane four rows of them; kTok tokens are on their way together
         constexpr int kTok = PAIR ? 2 : 4, kWarps = kBgThreadsSplit / 32;
         const float* mine = reinterpret_cast<const float*>(smem) + 4 * lane;
@@ -473,6 +473,16 @@ extern "C" int lv_gemm_bf16(lv_ctx* ctx, void* out, int out_type, uint32_t out_l
     if (int rc = make_bf16_map(&maps.x, x, batch, cols, x_ld, plan.two ? nt / 2 : nt)) return rc;
     maps.w2 = maps.w;
     return gemm_bf16_pick<false, false>(ctx, p, maps, plan, (batch + nt - 1) / nt);
+}
+
+extern "C" int lv_gemm_bf16_plan(lv_ctx* ctx, uint32_t rows, uint32_t cols, uint32_t tokens, uint32_t* plan) {
+    LV_ENTER(ctx);
+    LV_REQUIRE(rows && cols && tokens && plan, "bad gemm_bf16_plan arguments");
+    const BgPlan p = bg_plan(ctx, rows, cols, tokens);
+    plan[0] = p.nt;
+    plan[1] = p.two ? 2 : 1;
+    plan[2] = p.splits;
+    return LV_OK;
 }
 
 extern "C" int lv_gemm_bf16_window(lv_ctx* ctx, void* out, int out_type, uint32_t out_ld, const void* w, uint32_t rows, uint32_t ld, uint32_t cols,

@@ -49,6 +49,26 @@ def test_gemm_bf16_tiles_and_splits(gpu, rows, cols, batch, out_bf16):
     test_gemm_bf16(gpu, rows, cols, batch, out_bf16)
 
 
+@pytest.mark.parametrize("rows,cols,batch,nt,splits", [(1100, 1032, 400, 128, 3), (1500, 3000, 500, 256, 4), (1100, 1032, 1400, 128, 1), (2600, 2056, 1999, 256, 1), (2048, 2048, 512, 256, 3)])
+def test_gemm_bf16_pairs(gpu, rows, cols, batch, nt, splits):
+    """Pairs of CTAs on one tile, with and without shares of K, ragged and whole, with more chunks of K than stages.  Launches one behind the
+    other, so that tensor memory changes hands: the same bits from all."""
+    plan = (C.c_uint32 * 3)()
+    pkg.check(gpu.lib.lv_gemm_bf16_plan(gpu.handle, rows, cols, batch, plan))
+    assert list(plan) == [nt, 2, splits]
+    rng = np.random.default_rng(rows + batch)
+    w, x = weights(rng, rows, cols), weights(rng, batch, cols, scale=1.0)
+    with Dev(gpu) as d:
+        dw, dx, outs = d.bf16(w), d.bf16(x), [d.zeros(batch * rows * 4) for _ in range(6)]
+        for out in outs:
+            pkg.check(gpu.lib.lv_gemm_bf16(gpu.handle, out, pkg.TYPE_F32, rows, dw, rows, pad8(cols), cols, dx, pad8(cols), batch, 0.5, 0))
+        gpu.sync()
+        got = [d.get(out, (batch, rows)) for out in outs]
+    assert rel(got[0], 0.5 * x.astype(np.float64) @ w.T.astype(np.float64)) < 2e-5
+    for other in got[1:]:
+        assert np.array_equal(got[0].view(np.uint32), other.view(np.uint32))
+
+
 def expert_args(d, w0, w1, rows, cols, table, ids, pos, vocab):
     n, top = w0.shape[0], table.shape[1]
     a = pkg.ExpertArgs()

@@ -69,9 +69,8 @@ def test_squared_relu_behind_a_product(gpu, rows, cols, batch):
 
 
 @pytest.mark.parametrize("window,pos,batch", [(0, 0, 5), (0, 130, 2), (1, 40, 3), (20, 7, 9), (20, 19, 2), (20, 20, 2), (64, 100, 70), (130, 300, 200), (600, 300, 12)])
-def test_products_of_the_rows_in_a_window(gpu, window, pos, batch):
+def test_products_of_the_rows_in_a_window(gpu, window, pos, batch, rows=144, cols=72, total=512):
     rng = np.random.default_rng(window + pos)
-    rows, cols, total = 144, 72, 512
     w, x = weights(rng, rows, cols), weights(rng, total, cols, scale=1.0)
     first = max(0, pos + 1 - window) if window else 0
     n = pos + batch - first
@@ -82,6 +81,14 @@ def test_products_of_the_rows_in_a_window(gpu, window, pos, batch):
         got = d.get(out, (bound, rows))
     assert rel(got[:n], x[first:pos + batch].astype(np.float64) @ w.T.astype(np.float64)) < 2e-5
     assert (got[n:] == -7.0).all()
+
+
+@pytest.mark.parametrize("window,pos,batch,splits", [(300, 77, 100, 3), (300, 400, 100, 3), (1000, 900, 200, 1), (1000, 10, 200, 1)])
+def test_products_of_a_window_by_pairs_of_ctas(gpu, window, pos, batch, splits):
+    plan = (C.c_uint32 * 3)()
+    pkg.check(gpu.lib.lv_gemm_bf16_plan(gpu.handle, 1100, 1032, window + batch - 1, plan))
+    assert plan[1] == 2 and plan[2] == splits
+    test_products_of_the_rows_in_a_window(gpu, window, pos, batch, 1100, 1032, 1536)
 
 
 # ---- rotation --------------------------------------------------------------------------------
