@@ -351,29 +351,6 @@ __global__ void __launch_bounds__(1024) expert_route_kernel(const lv_route_job* 
     for (uint32_t i = threadIdx.x; i < pairs; i += blockDim.x) job.index[i] = atomicAdd(&s_cursor[expert(i)], 1u);
 }
 
-// How many clusters of each size the device holds at a time, one CTA per SM: the SMs of a cluster are neighbours, so of 148 SMs clusters of
-// eight fill fewer than clusters of two.  (Two waves of clusters made a product of 2048 x 2048 with 60 tokens 18 us instead of 9.)
-int gemm_bf16_configure(lv_ctx* ctx) {
-    auto* kernel = gemm_bf16_kernel<128, false, false, false>;
-    LV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBgSmemBudget + 1024)));
-    for (uint32_t s = 2; s <= kBgMaxSplits; ++s) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(1, 1, s);
-        cfg.blockDim = dim3(kBgThreads);
-        cfg.dynamicSmemBytes = kBgSmemBudget;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = s;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int n = 0;
-        LV_CUDA(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
-        ctx->bg_clusters[s] = uint32_t(n);
-    }
-    return LV_OK;
-}
-
 // How a product is cut: tokens of a tile, pairs of CTAs, splits along K.
 struct BgPlan {
     uint32_t nt = 0, splits = 1;
@@ -398,16 +375,61 @@ static void bg_cut(const lv_ctx* ctx, BgPlan* plan, uint32_t rows, uint32_t cols
     }
 }
 
+// Shared memory of a launch, from a budget for its stages; the parts of a split take the stages' place.
+template <int NT, bool PAIR, bool TWO>
+constexpr uint32_t bg_stages(size_t budget) { return std::min<uint32_t>(kBgMaxStages, uint32_t(budget / bg_stage_bytes(NT, PAIR, TWO))); }
+template <int NT, bool PAIR, bool TWO>
+constexpr size_t bg_smem(uint32_t stages, bool split) {
+    return std::max(size_t(stages) * bg_stage_bytes(NT, PAIR, TWO), split ? size_t(PAIR ? 2 : 1) * NT * kBgRows * sizeof(float) : 0) + 1024;
+}
+
+// The largest size is set once: the attribute belongs to the kernel, and contexts launch from threads of their own.
+template <int NT, bool PAIR, bool GROUPED, bool TWO>
+static int bg_configure(lv_ctx* ctx) {
+    constexpr size_t smem = bg_smem<NT, PAIR, TWO>(bg_stages<NT, PAIR, TWO>(kBgSmemBudget), true);
+    LV_REQUIRE(size_t(ctx->max_smem_optin) >= smem, "device has too little shared memory for the bfloat16 product");
+    LV_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<NT, PAIR, GROUPED, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    return LV_OK;
+}
+
+// How many clusters of each size the device holds at a time, one CTA per SM: the SMs of a cluster are neighbours, so of 148 SMs clusters of
+// eight fill fewer than clusters of two.  (Two waves of clusters made a product of 2048 x 2048 with 60 tokens 18 us instead of 9.)
+int gemm_bf16_configure(lv_ctx* ctx) {
+    auto* kernel = gemm_bf16_kernel<128, false, false, false>;
+    int (*const configure[])(lv_ctx*) = {
+        bg_configure<16, false, false, false>, bg_configure<32, false, false, false>, bg_configure<64, false, false, false>, bg_configure<128, false, false, false>,
+        bg_configure<128, false, false, true>, bg_configure<256, false, false, false>, bg_configure<256, false, false, true>,
+        bg_configure<16, false, true, false>, bg_configure<32, false, true, false>, bg_configure<64, false, true, false>, bg_configure<128, false, true, false>,
+        bg_configure<16, true, true, false>, bg_configure<32, true, true, false>, bg_configure<64, true, true, false>, bg_configure<128, true, true, false>};
+    for (auto* f : configure)
+        if (int rc = f(ctx)) return rc;
+    for (uint32_t s = 2; s <= kBgMaxSplits; ++s) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(1, 1, s);
+        cfg.blockDim = dim3(kBgThreads);
+        cfg.dynamicSmemBytes = bg_smem<128, false, false>(bg_stages<128, false, false>(kBgSmemBudget), true);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = s;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        LV_CUDA(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
+        ctx->bg_clusters[s] = uint32_t(n);
+    }
+    return LV_OK;
+}
+
 template <int NT, bool PAIR, bool GROUPED, bool TWO>
 static int gemm_bf16_launch(lv_ctx* ctx, GemmBf16Params p, const GemmBf16Maps& maps, const BgPlan& plan, uint32_t token_tiles) {
-    constexpr uint32_t kStage = bg_stage_bytes(NT, PAIR, TWO), kCluster = TWO ? 2 : 1;
+    constexpr uint32_t kCluster = TWO ? 2 : 1;
     const uint32_t row_tiles = ((p.rows + kBgRows - 1) / kBgRows + kCluster - 1) / kCluster * kCluster, ctas = row_tiles * token_tiles;
     p.splits = plan.splits;
-    p.stages = std::min<uint32_t>(kBgMaxStages, uint32_t((p.splits == 1 && ctas > uint32_t(ctx->sm_count) ? kBgSmemHalf : kBgSmemBudget) / kStage));
+    p.stages = bg_stages<NT, PAIR, TWO>(p.splits == 1 && ctas > uint32_t(ctx->sm_count) ? kBgSmemHalf : kBgSmemBudget);
     p.err = ctx->d_err;
-    const size_t smem = std::max(size_t(p.stages) * kStage, p.splits > 1 ? size_t(PAIR ? 2 : 1) * NT * kBgRows * sizeof(float) : 0) + 1024;
+    const size_t smem = bg_smem<NT, PAIR, TWO>(p.stages, p.splits > 1);
     auto* kernel = gemm_bf16_kernel<NT, PAIR, GROUPED, TWO>;
-    LV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     LV_REQUIRE(token_tiles <= 65535, "gemm_bf16: too many token tiles");
     const dim3 grid(row_tiles, token_tiles, p.splits);
     if (kCluster * p.splits == 1) LV_CUDA(launch_pdl(ctx, kernel, grid, dim3(kBgThreads), smem, p, maps));

@@ -1,6 +1,7 @@
 """Each mechanism of the bfloat16-weight decoders alone, through the C ABI, against the plain implementation in
 tests/sonuzen_plain.py (float64)."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -67,6 +68,29 @@ def test_gemm_bf16_pairs(gpu, rows, cols, batch, nt, splits):
     assert rel(got[0], 0.5 * x.astype(np.float64) @ w.T.astype(np.float64)) < 2e-5
     for other in got[1:]:
         assert np.array_equal(got[0].view(np.uint32), other.view(np.uint32))
+
+
+def test_gemm_bf16_from_contexts_on_two_threads(gpu):
+    """Launches of one kernel with the large and with the small share of an SM's shared memory, from two contexts at once: none is refused."""
+    def launches(rows, cols, failed):
+        with pkg.Context(0) as ctx:
+            w, x, out = ctx.zeros(rows * cols * 2), ctx.zeros(20 * cols * 2), ctx.zeros(20 * rows * 4)
+            for i in range(20000):
+                rc = ctx.lib.lv_gemm_bf16(ctx.handle, out, pkg.TYPE_F32, rows, w, rows, cols, cols, x, cols, 20, 1.0, 0)
+                if rc != pkg.LV_OK:
+                    failed.append((rows, i, rc))
+                    break
+                if i % 500 == 0:
+                    ctx.sync()
+            ctx.sync()
+
+    failed = []
+    threads = [threading.Thread(target=launches, args=(rows, cols, failed)) for rows, cols in ((20000, 64), (1000, 2048))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
 
 
 def expert_args(d, w0, w1, rows, cols, table, ids, pos, vocab):
