@@ -157,7 +157,7 @@ __device__ __forceinline__ uint32_t gb_expert(const ExpertGemvParams& p, uint32_
     const uint32_t id = p.token_log[*p.pos + t];
     const uint32_t e = id < p.vocab ? p.table[size_t(id) * p.top + slot] : p.experts;
     if (e < p.experts) return e;
-    if (threadIdx.x == 0) atomicOr(p.err, ERR_BAD_INDEX);
+    if ((threadIdx.x & 31u) == 0) atomicOr(p.err, ERR_BAD_INDEX);      // (each warp looks up its own choices)
     return 0;
 }
 

@@ -135,6 +135,27 @@ def test_experts_of_one_token(gpu, width, ff, n, top, late):
         assert rel(d.get(out, (1, width)), want) < 2e-6
 
 
+@pytest.mark.parametrize("top,slot", [(1, 0), (2, 1), (3, 1), (4, 1), (4, 3), (5, 2), (9, 7)])
+@pytest.mark.parametrize("batch", [1, 3])
+def test_down_product_reports_a_bad_expert_of_any_choice(gpu, top, slot, batch):
+    rng = np.random.default_rng(top)
+    width, ff, n, vocab = 72, 40, 10, 30
+    table, ids = draw_table(rng, vocab, n, top), np.arange(batch)
+    for bad in (False, True):
+        if bad:
+            table[ids[-1], slot] = n
+        with Dev(gpu) as d:
+            dn = expert_args(d, weights(rng, n, width, ff), None, width, ff, table, ids, 2, vocab)
+            act, out = d.f32(rng.standard_normal((batch * top, pad8(ff)))), d.zeros(batch * width * 4)
+            pkg.check(gpu.lib.lv_gemv_bf16_expert_down(gpu.handle, out, width, C.byref(dn), act, pad8(ff), batch))
+            if bad:
+                with pytest.raises(pkg.LvError) as e:
+                    gpu.sync()
+                assert e.value.code == pkg.LV_ERR_DEVICE_WAIT
+            else:
+                gpu.sync()
+
+
 @pytest.mark.parametrize("width,ff,n,top,batch", [(64, 40, 5, 2, 1), (48, 96, 3, 1, 2), (136, 72, 9, 3, 23), (64, 200, 4, 4, 70), (96, 32, 70, 2, 300),
                                                   (64, 64, 3, 2, 290)])
 def test_experts_chosen_by_token(gpu, width, ff, n, top, batch):
