@@ -480,8 +480,9 @@ int lv_mingru_scan(lv_ctx* ctx, void* out, int out_type, uint32_t out_ld, const 
  * matrices stacked, [experts * rows][ld].
  *   gate_up: out[t * top + s] = silu(gate_e x[t]) * (up_e x[t]), e = table[id_t][s] (w0 gate, w1 up; rows = ff, cols = width)
  *   down:    out[t] = (1 / top) sum_s down_e x[t * top + s]                        (w0 down; rows = width, cols = ff)
- * One token: *pos, its entry of the log and the table are read before earlier launches of the stream have finished, and again after them;
- * whatever *pos holds meanwhile has to be a place of the log. */
+ * log_places: places of token_log, and no earlier launch of the stream writes the table or the matrices.  One token's experts are then looked
+ * up and requested while earlier launches run, whatever *pos and the log hold meanwhile, and looked up again after them.  0: not known,
+ * everything is read after earlier launches. */
 typedef struct lv_expert_args {
     const void* w0;
     const void* w1;
@@ -489,6 +490,7 @@ typedef struct lv_expert_args {
     const uint32_t* table;
     const uint32_t* token_log;
     const uint32_t* pos;
+    uint32_t log_places;
 } lv_expert_args;
 int lv_gemv_bf16_expert_gate_up(lv_ctx* ctx, float* out, uint32_t out_ld, const lv_expert_args* a, const float* x, uint32_t x_ld, uint32_t batch);
 int lv_gemv_bf16_expert_down(lv_ctx* ctx, float* out, uint32_t out_ld, const lv_expert_args* a, const float* x, uint32_t x_ld, uint32_t batch);

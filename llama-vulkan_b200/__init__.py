@@ -46,7 +46,7 @@ class NormConvArgs(C.Structure):
 class ExpertArgs(C.Structure):
     """lv_expert_args"""
     _fields_ = [("w0", _p), ("w1", _p), ("ld", _u32), ("rows", _u32), ("cols", _u32), ("experts", _u32), ("top", _u32), ("vocab", _u32),
-                ("table", _p), ("token_log", _p), ("pos", _p)]
+                ("table", _p), ("token_log", _p), ("pos", _p), ("log_places", _u32)]
 
 
 class GqaArgs(C.Structure):

@@ -146,6 +146,7 @@ struct ExpertGemvParams {
     const uint32_t* table;          // [vocab][top]
     const uint32_t* token_log;
     const uint32_t* pos;
+    uint32_t log_places;            // one token: places of token_log, 0 where its experts may not be looked up early
     const float* x;
     uint32_t x_ld;
     float* out;
@@ -162,10 +163,10 @@ __device__ __forceinline__ uint32_t gb_expert(const ExpertGemvParams& p, uint32_
 }
 
 // The same before the previous kernel has finished: a guess.  The position and the token are those of the step unless an earlier launch
-// that is still running writes them; whoever uses the guess asks again after the wait.  One token only (a position is always inside the log,
-// the tokens behind it may not be).
+// that is still running writes them; whoever uses the guess asks again after the wait.
 __device__ __forceinline__ uint32_t gb_expert_guess(const ExpertGemvParams& p, uint32_t slot) {
-    const uint32_t at = *reinterpret_cast<const volatile uint32_t*>(p.pos), id = *reinterpret_cast<const volatile uint32_t*>(p.token_log + at);
+    const uint32_t at = *reinterpret_cast<const volatile uint32_t*>(p.pos);
+    const uint32_t id = at < p.log_places ? *reinterpret_cast<const volatile uint32_t*>(p.token_log + at) : p.vocab;
     const uint32_t e = id < p.vocab ? p.table[size_t(id) * p.top + slot] : 0;
     return e < p.experts ? e : 0;
 }
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(kGbThreads) gemv_bf16_expert_gate_up_kernel(co
         row[1] = p.up + at;
     };
     float acc[2] = {0.f, 0.f};
-    if (gridDim.y == 1) {
+    if (p.log_places != 0) {
         const uint32_t guess = gb_expert_guess(p, slot);
         rows_of(guess);
         gb_dot<2, true>(acc, row, p.x, p.K, [&]() {
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(kGbThreads) gemv_bf16_expert_down_kernel(const
     const float* x = p.x + size_t(t) * p.top * p.x_ld;
     float acc[2] = {0.f, 0.f};
     uint32_t s = mine;                                       // (SHARE <= top)
-    if (gridDim.y == 1) {
+    if (p.log_places != 0) {
         const uint32_t guess = gb_expert_guess(p, s);
         rows_of(guess);
         gb_dot<2, true>(acc, row, x + size_t(s) * p.x_ld, p.K, [&]() {
@@ -287,20 +288,21 @@ extern "C" int lv_gemv_bf16_mingru(lv_ctx* ctx, float* out, const void* wz, cons
     return LV_OK;
 }
 
-static int expert_params(const lv_expert_args* a, ExpertGemvParams* p) {
+static int expert_params(const lv_expert_args* a, ExpertGemvParams* p, uint32_t batch) {
     LV_REQUIRE(a && a->table && a->token_log && a->pos && a->experts && a->top && a->vocab && a->rows && a->cols, "bad expert arguments");
     LV_REQUIRE(a->ld % 8 == 0 && a->ld >= a->cols && a->w0 && gb_aligned(a->w0) && (!a->w1 || gb_aligned(a->w1)), "experts: bad matrices");
     p->gate = static_cast<const __nv_bfloat16*>(a->w0);
     p->up = static_cast<const __nv_bfloat16*>(a->w1);
     p->ld = a->ld; p->K = a->cols; p->rows = a->rows; p->experts = a->experts; p->top = a->top; p->vocab = a->vocab;
     p->table = a->table; p->token_log = a->token_log; p->pos = a->pos;
+    p->log_places = batch == 1 ? a->log_places : 0;
     return LV_OK;
 }
 
 extern "C" int lv_gemv_bf16_expert_gate_up(lv_ctx* ctx, float* out, uint32_t out_ld, const lv_expert_args* a, const float* x, uint32_t x_ld, uint32_t batch) {
     LV_ENTER(ctx);
     ExpertGemvParams p{};
-    if (const int rc = expert_params(a, &p)) return rc;
+    if (const int rc = expert_params(a, &p, batch)) return rc;
     LV_REQUIRE(out && x && gb_aligned(x) && batch && batch <= 65535 && a->top <= 65535 && p.up && out_ld >= p.rows && x_ld >= p.K && (batch == 1 || x_ld % 4 == 0), "bad expert_gate_up arguments");
     p.x = x; p.x_ld = x_ld; p.out = out; p.out_ld = out_ld; p.err = ctx->d_err;
     LV_CUDA(launch_pdl(ctx, gemv_bf16_expert_gate_up_kernel, dim3((p.rows + kGbWarps - 1) / kGbWarps, batch, p.top), dim3(kGbThreads), 0, p));
@@ -310,7 +312,7 @@ extern "C" int lv_gemv_bf16_expert_gate_up(lv_ctx* ctx, float* out, uint32_t out
 extern "C" int lv_gemv_bf16_expert_down(lv_ctx* ctx, float* out, uint32_t out_ld, const lv_expert_args* a, const float* x, uint32_t x_ld, uint32_t batch) {
     LV_ENTER(ctx);
     ExpertGemvParams p{};
-    if (const int rc = expert_params(a, &p)) return rc;
+    if (const int rc = expert_params(a, &p, batch)) return rc;
     LV_REQUIRE(out && x && gb_aligned(x) && batch && batch <= 65535 && out_ld >= p.rows && x_ld >= p.K && x_ld % 4 == 0, "bad expert_down arguments");
     p.x = x; p.x_ld = x_ld; p.out = out; p.out_ld = out_ld; p.err = ctx->d_err;
     // warps per pair of rows: as many as there are experts, a power of two up to four

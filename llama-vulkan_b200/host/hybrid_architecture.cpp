@@ -565,6 +565,7 @@ struct hybrid_recorder {
         gate_up.table = static_cast<const u32*>(l.table->device_ptr());
         gate_up.token_log = log;
         gate_up.pos = pos;
+        gate_up.log_places = s->log_capacity();
         down = gate_up;
         down.w0 = l.down->device_ptr();
         down.w1 = nullptr;

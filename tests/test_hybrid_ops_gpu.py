@@ -102,6 +102,7 @@ def expert_args(d, w0, w1, rows, cols, table, ids, pos, vocab):
     a.table = d.u32(table).value
     a.token_log = d.u32(np.concatenate([np.full(pos, vocab - 1), ids])).value
     a.pos = d.u32([pos] * 4).value
+    a.log_places = pos + len(ids)
     return a
 
 
@@ -110,12 +111,13 @@ def draw_table(rng, vocab, n, top):
 
 
 @pytest.mark.parametrize("width,ff,n,top", [(64, 40, 3, 1), (2056, 1100, 5, 2), (72, 1032, 7, 3), (1030, 2200, 6, 4), (7, 24, 9, 5), (130, 64, 11, 9)])
-@pytest.mark.parametrize("late", [False, True])
+@pytest.mark.parametrize("late", [False, True, "from outside", "unknown log"])
 def test_experts_of_one_token(gpu, width, ff, n, top, late):
     """One token: its experts are looked up before the launches ahead have finished and again after them; the down product's experts are
-    shared by one, two or four warps.  late: a launch just ahead moves the position, so an early look finds another token's experts."""
+    shared by one, two or four warps.  late: a launch just ahead moves the position, so an early look finds another token's experts, or
+    none, where the position lay outside the log, or is not taken, where the size of the log is not given."""
     rng = np.random.default_rng(width + top)
-    vocab, pos = 50, 3
+    vocab, pos = 50, 3 if late in (False, True) else 0
     gate, up, down = weights(rng, n, ff, width), weights(rng, n, ff, width), weights(rng, n, width, ff)
     table, ids = draw_table(rng, vocab, n, top), rng.integers(0, vocab, 1)
     x = weights(rng, 1, width, scale=1.0)
@@ -128,7 +130,9 @@ def test_experts_of_one_token(gpu, width, ff, n, top, late):
         xp, act, out = d.f32(xp), d.zeros(top * pad8(ff) * 4), d.zeros(width * 4)
         if late:
             for a in (gu, dn):
-                a.pos = d.u32([pos - 1] * 4).value
+                a.pos = d.u32([(pos - 1) % 2**32] * 4).value
+                if late == "unknown log":
+                    a.log_places = 0
                 d.call("lv_decode_advance", a.pos, None, None, 1, 0)
         d.call("lv_gemv_bf16_expert_gate_up", act, pad8(ff), C.byref(gu), xp, pad8(width), 1)
         d.call("lv_gemv_bf16_expert_down", out, width, C.byref(dn), act, pad8(ff), 1)
