@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
 // tensor-parallel column shard).
 //
 // Bound by latency (1 MB at 64 x 4096): a normalised row of up to kSplitUnits * 4096 values stays in registers between its sums and its
-// conversion, and the norm's weights are requested before the previous kernel ends, so that one trip to L2 is left of four.
+// conversion, and the norm's weights are requested together with it, so that one trip to L2 is left of four.
 // A prompt of 1024 tokens, 7B q4_0 (two such launches per layer and step): 79.9 -> 75.7 ms.
 constexpr int kSplitThreads = 512, kSplitUnits = 2;
 
@@ -640,12 +640,7 @@ __global__ void __launch_bounds__(kSplitThreads) act_split_kernel(__half* __rest
     const uint32_t units = K / 8;
     if (norm_w != nullptr && units <= uint32_t(kSplitUnits * kSplitThreads)) {
         float v[kSplitUnits][8], w[kSplitUnits][8];
-#pragma unroll
-        for (int u = 0; u < kSplitUnits; ++u) {
-            const uint32_t unit = threadIdx.x + u * kSplitThreads;
-            if (unit < units) load8(w[u], norm_w + 8 * unit);
-        }
-        pdl_wait();
+        pdl_wait();                                                          // (the weights may come from the launch before, like x)
         float part = 0.f;
 #pragma unroll
         for (int u = 0; u < kSplitUnits; ++u) {
@@ -653,6 +648,7 @@ __global__ void __launch_bounds__(kSplitThreads) act_split_kernel(__half* __rest
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[u][i] = 0.f;
             if (z < Z && unit < units) load8(v[u], xr + 8 * unit);
+            if (unit < units) load8(w[u], norm_w + 8 * unit);
         }
 #pragma unroll
         for (int u = 0; u < kSplitUnits; ++u)

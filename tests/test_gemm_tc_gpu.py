@@ -365,3 +365,23 @@ def test_act_split_of_normalised_rows(gpu, pkg, batch, cols, form):
     x64 = x.astype(np.float64)
     want = x64 * w / np.sqrt(((x64 - x64.mean(1, keepdims=True)) ** 2).mean(1, keepdims=True))
     close(hi[:batch] + lo[:batch], want, rel_l2=1e-6, max_abs_frac=1e-6)
+
+
+def test_act_split_takes_the_weights_of_the_launch_before(gpu, pkg, form):
+    """The norm's weights are the end of a long row that one thread block normalises in the launch just before."""
+    if form == "exact":
+        pytest.skip("no products here")
+    n, cols, batch = 1 << 22, 4096, 3
+    rng = np.random.default_rng(7)
+    x, long_row = rng.standard_normal((batch, cols)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    w = (long_row[-cols:] / long_row.astype(np.float64).std())
+    x64 = x.astype(np.float64)
+    want = x64 * w / np.sqrt(((x64 - x64.mean(1, keepdims=True)) ** 2).mean(1, keepdims=True))
+    out, row, ones, dx, xh = gpu.zeros(n * 4), gpu.upload(long_row), gpu.upload(np.ones(n, np.float32)), gpu.upload(x), gpu.alloc(gpu.lib.lv_act_split_bytes(cols, batch))
+    pkg.check(gpu.lib.lv_norm_f32(gpu.handle, out, row, ones, n, 1))
+    pkg.check(gpu.lib.lv_act_split_f16(gpu.handle, xh, dx, pkg.offset(out, (n - cols) * 4), cols, batch))
+    gpu.sync()
+    hi, lo = planes_of(gpu.download(xh, np.float16, 2 * 16 * cols), 16, cols)
+    close(hi[:batch] + lo[:batch], want, rel_l2=1e-5, max_abs_frac=1e-5)
+    for d in (out, row, ones, dx, xh):
+        gpu.free(d)
