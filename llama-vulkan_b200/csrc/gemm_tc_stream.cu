@@ -279,12 +279,12 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
         for (uint32_t i = 0; i < n_units && ok; ++i) {
             const uint32_t ab = i & 1u;
             // the accumulators of the previous segment have been read
-            if (first && seg > 0) ok = mbar_wait_warp(acc_empty, (seg - 1) & 1u, p.err);
-            ok = ok && mbar_wait_warp(&a_full[2 * ab + h], (i >> 1) & 1u, p.err);
+            if (first && seg > 0) ok = mbar_wait_elect(acc_empty, (seg - 1) & 1u, p.err);
+            ok = ok && mbar_wait_elect(&a_full[2 * ab + h], (i >> 1) & 1u, p.err);
             const uint32_t a_tmem = tmem_base + kTsABase + (4u * ab + 2u * h) * kTsTileCols;
 #pragma unroll
             for (uint32_t st = 0; st < 2 / kBT; ++st) {
-                ok = ok && mbar_wait_warp(&b_full[bs], b_phase, p.err);
+                ok = ok && mbar_wait_elect(&b_full[bs], b_phase, p.err);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint64_t b_desc = b_desc0 + ((bs * b_stage) >> 4);

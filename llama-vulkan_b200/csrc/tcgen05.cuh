@@ -53,6 +53,14 @@ __device__ __forceinline__ bool tc_elect() {
     return yes != 0;
 }
 
+// Waits like mbar_wait_warp, for a warp whose elected lane alone goes on to use what the barrier guards: that lane looks at the barrier itself, so the
+// others need no ordering behind it.
+__device__ __forceinline__ bool mbar_wait_elect(uint64_t* bar, uint32_t parity, uint32_t* err) {
+    bool ok = false;
+    if (tc_elect()) ok = mbar_wait(bar, parity, err);
+    return __any_sync(0xffffffffu, ok);
+}
+
 // Sixteen accumulator columns of this warp's quarter of the lanes; waits for the data.
 __device__ __forceinline__ void tc_load16(uint32_t (&u)[16], uint32_t taddr) {
     asm volatile(
