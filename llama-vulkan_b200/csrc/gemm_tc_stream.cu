@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
         uint32_t n_pairs = 0;
         // reads the accumulators of segment `seg` (16 tokens per warp) and stores or parks them
         auto drain = [&](uint32_t seg, uint32_t tile, bool whole, uint32_t slot) {
-            ok = mbar_wait_warp(acc_full, seg & 1u, p.err);
+            ok = mbar_wait_warp_tc(acc_full, seg & 1u, p.err);
             if (!ok) return;
             tc_fence_after_sync();
             const uint32_t z0 = 16u * tt;

@@ -61,6 +61,14 @@ __device__ __forceinline__ bool mbar_wait_elect(uint64_t* bar, uint32_t parity, 
     return __any_sync(0xffffffffu, ok);
 }
 
+// mbar_wait_warp for a warp whose next step is tc_load16, an instruction of the whole warp that the fence in front of it orders: without the
+// ordering of ordinary loads by other lanes (0.1 us for each of the ends of a segment in gemm_tc_stream.cu).
+__device__ __forceinline__ bool mbar_wait_warp_tc(uint64_t* bar, uint32_t parity, uint32_t* err) {
+    uint32_t ok = 1;
+    if ((threadIdx.x & 31u) == 0) ok = mbar_wait(bar, parity, err) ? 1u : 0u;
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
 // Sixteen accumulator columns of this warp's quarter of the lanes; waits for the data.
 __device__ __forceinline__ void tc_load16(uint32_t (&u)[16], uint32_t taddr) {
     asm volatile(
