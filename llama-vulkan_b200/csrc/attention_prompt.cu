@@ -8,19 +8,24 @@
 //   S = Q K^T     A = queries, B = keys, both as f16 pairs hi + lo (22 bits): q_hi k_hi + q_lo k_hi + q_hi k_lo
 //   O = P V       A = probabilities as f16 pairs, B = values, f16 as they are in the cache
 //
-// with f32 sums, so scores and probabilities are as exact as the f32 arithmetic of attention_fused_kernel.  The operands are 64
-// rows high and a CTA has one pass over 128 keys: nothing to pipeline, and half a tcgen05 tile, so these are mma.sync.
+// with f32 sums.  The lo halves keep their bits because queries and keys are scaled by a power of two per row and the probabilities by 2^15,
+// and the sums of 16 values that a tensor-core instruction forms (it truncates) are added by ordinary f32 additions.  Relative error of the
+// outputs against 64 bits, scores of rms 1, 32 heads, attention_fused_kernel / here (one long chain of sums, keys as they are):
+//   positions      0 .. 63              192 .. 255           900 .. 963           1900 .. 1963
+//                  1.4e-7 / 2.0e-7      5.9e-7 / 5.8e-7      2.57e-6 / 2.48e-6    6.1e-6 / 5.9e-6      for keys of any size from 2^-14 to 2^12
+//                  (4.7e-7)             (8.5e-7)             (2.8e-6)                                  (and 4e-4 for keys of size 2^-14)
+// The operands are 64 rows high and a CTA has one pass over 128 keys: nothing to pipeline, and half a tcgen05 tile, so these are mma.sync.
 //
-// Rotation: the score of query z (position P + z) and key p turns by the distance P + z - p.  Keys are turned by P - p, with the
-// table row of that distance (the sign of sin is flipped for p > P), and queries by z, so no row of the table is needed per pair.
-// A warp owns 16 keys: a thread reads its part of two key rows from shared memory (raw rows, brought by bulk copies) in 16-byte loads
-// -- the order of the head's 128 values is free as long as Q uses the same one --, turns pairs in f32 and splits them in registers.
+// Rotation: the score of query z (position P + z) and key p turns by the distance P + z - p.  Both are turned from one position, queries forwards and
+// keys backwards, so no row of the table is needed per pair.
+// A warp owns 16 keys: a thread reads its part of two key rows from shared memory (raw rows, brought by bulk copies) -- the order of the head's
+// 128 values is free as long as Q uses the same one --, turns pairs in f32 and splits them in registers.
 //
 // The softmax of a CTA's keys needs the maximum over its eight warps (one exchange), the CTAs of the cluster meet once at the end
 // through distributed shared memory, each finishing its share of the rows.  No scratch, no counters.
 //
-// Bound by latency: 64 rows at 1000 positions take 24.5 us (237 before), of which the matrix products are 5; 2 are the query preparation,
-// 3 the softmax's exchanges, 4 the meeting of the cluster.  Two CTAs per SM hide some of it behind each other.
+// Bound by latency: 64 rows at 964 positions of 1024 take 25.3 us (233 before; 22.7 with one long chain of sums and a table row of any distance), of
+// which the matrix products are 5; 2 are the query preparation, 3 the softmax's exchanges, 4 the meeting of the cluster.  Two CTAs per SM hide some of it behind each other.
 #include <math.h>
 
 #include <algorithm>
@@ -42,7 +47,7 @@ constexpr uint32_t kApRedBytes = (2 * kApWarps + 5) * kApQ * 4;
 constexpr size_t kApSmemBytes = kApQBytes + 2 * kApRowBytes + kApRedBytes;      // two CTAs per SM
 static_assert(size_t(kApQ) * kApOStride * 4 <= kApRowBytes, "the outputs of a CTA take the place of its values");
 constexpr float kApLog2e = 1.4426950408889634f;
-constexpr float kApPScale = 12.f;                                       // log2: probabilities as f16 pairs keep 22 bits down to 2^-26
+constexpr float kApPScale = 15.f;                                       // log2: probabilities as f16 pairs keep 22 bits down to 2^-17, 11 down to 2^-29
 
 __device__ __forceinline__ void ap_mma(float (&c)[4], const uint4& a, uint32_t b0, uint32_t b1) {
     asm(
@@ -74,6 +79,16 @@ __device__ __forceinline__ float4 ap_cluster_load4(const float* local, uint32_t 
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(local)), "r"(rank));
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
     return v;
+}
+
+// (cos, sin) of two pairs at the distance d (sin turns its sign with it), from the table
+__device__ __forceinline__ float4 ap_table_row(const float* table, int d, uint32_t dim) {
+    float4 w = *reinterpret_cast<const float4*>(table + size_t(abs(d)) * kApHead + dim);
+    if (d < 0) { w.y = -w.y; w.w = -w.w; }
+    return w;
+}
+__device__ __forceinline__ float4 ap_add_angles(const float4& a, const float4& b) {
+    return make_float4(fmaf(a.x, b.x, -(a.y * b.y)), fmaf(a.y, b.x, a.x * b.y), fmaf(a.z, b.z, -(a.w * b.w)), fmaf(a.w, b.z, a.z * b.w));
 }
 
 // The order of the head's values in the fragments: step ks of thread t holds the four from ap_first_dim(ks, t) on; eight lanes (two key
@@ -133,40 +148,45 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
         else bulk_g2s(s_v + i * kApStride, vc + row, kApHead * sizeof(__half), &s_bar[1]);
     };
     static_assert(kApThreads == 2 * kApKeys, "one key and one value row per pair of threads");
-    float4 cs[2][2][4];                                             // table rows of this thread's two keys: [half][key][step]
-    float turn[2];
-    auto load_table = [&](uint32_t p0, int half) {
+    // Angles: position 32 c + d, |d| <= 16 where the table has the rows, is turned from 32 c0 by the table rows of 32 (c - c0) and of d, queries forwards
+    // and keys backwards.  (The table's angles are rounded products of distance and frequency: rows of few distances, mostly small or powers
+    // of two times 32, keep that error below that of a row of any distance.)
+    const uint32_t c0 = P >> 5, c_max = (max_ctx - 1) >> 5;
+    float4 far[4];                                                  // of this warp's 32 positions, four steps ahead
+    auto load_far = [&](uint32_t p0, uint32_t ks, int i) {
+        far[i] = ap_table_row(table, int(32 * c0) - int(32 * min((p0 + 16 * warp + 16) >> 5, c_max)), ap_first_dim(ks, t));
+    };
+    auto load_first_far = [&](uint32_t p0) {
+        if (p0 + 16 * warp > last) return;
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const uint32_t p = min(p0 + 16 * warp + 8 * j + g, last);
-            const float* row = table + size_t(p > P ? p - P : P - p) * kApHead;
-            turn[j] = p > P ? -0.5f : 0.5f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) cs[half][j][i] = *reinterpret_cast<const float4*>(row + ap_first_dim(4 * half + i, t));
-        }
+        for (int i = 0; i < 4; ++i) load_far(p0, i, i);
     };
     if (rank < n_chunks) {
         load_rows(rank * kApKeys);
         // ---- queries: turned by their row, scaled by a power of two so that the largest value of a row is in [1024, 2048) --------
         constexpr int kRows = 4;                                    // rows of a warp at a time, all loads before the first use
         for (uint32_t r0 = warp; r0 < 16 * n_mt; r0 += kRows * kApWarps) {
-            float4 x[kRows], w[kRows];
+            float4 x[kRows], near[kRows], far[kRows];
 #pragma unroll
             for (int i = 0; i < kRows; ++i) {
                 const uint32_t r = r0 + i * kApWarps;
-                x[i] = r < nq ? *reinterpret_cast<const float4*>(q + size_t(z0 + r) * dim + h * kApHead + 4 * lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-                w[i] = r < nq ? *reinterpret_cast<const float4*>(table + size_t(r) * kApHead + 4 * lane) : x[i];
+                x[i] = near[i] = far[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (r >= nq) continue;
+                const uint32_t c = min((P + r + 16) >> 5, c_max);
+                x[i] = *reinterpret_cast<const float4*>(q + size_t(z0 + r) * dim + h * kApHead + 4 * lane);
+                near[i] = ap_table_row(table, int(P + r) - int(32 * c), 4 * lane);
+                far[i] = ap_table_row(table, int(32 * (c - c0)), 4 * lane);
             }
 #pragma unroll
             for (int i = 0; i < kRows; ++i) {
                 const uint32_t r = r0 + i * kApWarps;
                 if (r >= 16 * n_mt) break;
-                const float4 v = make_float4(w[i].x * x[i].x - w[i].y * x[i].y, w[i].y * x[i].x + w[i].x * x[i].y,
-                                             w[i].z * x[i].z - w[i].w * x[i].w, w[i].w * x[i].z + w[i].z * x[i].w);
+                const float4 w = ap_add_angles(far[i], near[i]);
+                const float4 v = make_float4(w.x * x[i].x - w.y * x[i].y, w.y * x[i].x + w.x * x[i].y, w.z * x[i].z - w.w * x[i].w, w.w * x[i].z + w.z * x[i].w);
                 const float top = warp_max(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
                 const uint32_t e = max(__float_as_uint(top) >> 23, 11u);
                 const float up = __uint_as_float((264u - e) << 23), down = __uint_as_float((e - 10u) << 23);      // 2^(137 - e), 2^(e - 137)
-                if (lane == 0) s_qf[r] = 2.f * down * scale * kApLog2e;       // (keys enter halved, see below)
+                if (lane == 0) s_qf[r] = down * scale * kApLog2e;
                 uint32_t hi0, lo0, hi1, lo1;
                 ap_split(v.x * up, v.y * up, hi0, lo0);
                 ap_split(v.z * up, v.w * up, hi1, lo1);
@@ -179,8 +199,7 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
                 at[kApPlane / 4 + 2] = lo1;
             }
         }
-        load_table(rank * kApKeys, 0);
-        if (ONE_PASS) load_table(rank * kApKeys, 1);                // (with several passes the outputs take the registers)
+        load_first_far(rank * kApKeys);
     }
     __syncthreads();
 
@@ -203,36 +222,67 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
 #pragma unroll
                 for (int c = 0; c < 4; ++c) s[i][j][c] = 0.f;
         ok = mbar_wait_warp(&s_bar[0], phase, err) && ok;
+        float key_unit[2][2] = {{1.f, 1.f}, {1.f, 1.f}};            // of the keys 8 j + 2 t + c
         if (my0 <= last) {
+            // a key is scaled by a power of two so that its largest value is in [2048, 4096): turned it stays inside f16, and its lo half
+            // keeps its bits
+            const uint8_t* key[2];
+            float up[2];
+            int near[2];                                                            // from the keys to the table row of their 32 positions
+            const uint32_t c = min((my0 + 16) >> 5, c_max);
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                if (!ONE_PASS && half != 0) load_table(p0, 1);
+            for (int j = 0; j < 2; ++j) {
+                key[j] = s_k + (16 * warp + 8 * j + g) * kApStride;
+                __half2 top = __half2{};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(key[j] + 128 * (i >> 1) + 32 * t + 16 * (i & 1));
+                    const __half2* h2 = reinterpret_cast<const __half2*>(&w);
+                    top = __hmax2(top, __hmax2(__hmax2(__habs2(h2[0]), __habs2(h2[1])), __hmax2(__habs2(h2[2]), __habs2(h2[3]))));
+                }
+                float m = fmaxf(__low2float(top), __high2float(top));
+                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+                near[j] = int(32 * c) - int(min(my0 + 8 * j + g, last));
+                const uint32_t e = max(__float_as_uint(m) >> 23, 103u);            // (2^-24 is the smallest f16)
+                up[j] = __uint_as_float((265u - e) << 23);                          // 2^(138 - e)
+                const float down = __uint_as_float((e - 11u) << 23);                // 2^(e - 138)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) key_unit[j][c] = __shfl_sync(0xffffffffu, down, 4 * (2 * t + c));
+            }
+#pragma unroll 1
+            for (uint32_t half = 0; half < 2; ++half) {
 #pragma unroll
                 for (int k4 = 0; k4 < 4; ++k4) {
-                    const int ks = 4 * half + k4;
+                    const uint32_t ks = 4 * half + k4;
                     uint32_t bh[2][2], bl[2][2];
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
-                        const uint2 w = *reinterpret_cast<const uint2*>(s_k + (16 * warp + 8 * j + g) * kApStride + 2 * ap_first_dim(ks, t));
+                        const uint2 w = *reinterpret_cast<const uint2*>(key[j] + 2 * ap_first_dim(ks, t));
                         const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
-                        // mhsa.comp:50-54 with half the key, so that a turned value never leaves the range of f16
-                        const float4 f = cs[half][j][k4];
-                        const float c0 = 0.5f * f.x, s0 = turn[j] * f.y, c1 = 0.5f * f.z, s1 = turn[j] * f.w;
-                        ap_split(c0 * a.x + s0 * a.y, c0 * a.y - s0 * a.x, bh[j][0], bl[j][0]);
-                        ap_split(c1 * b.x + s1 * b.y, c1 * b.y - s1 * b.x, bh[j][1], bl[j][1]);
+                        const float4 f = ap_add_angles(far[k4], ap_table_row(table, near[j], ap_first_dim(ks, t)));      // mhsa.comp:50-54
+                        const float cos0 = up[j] * f.x, sin0 = up[j] * f.y, cos1 = up[j] * f.z, sin1 = up[j] * f.w;
+                        ap_split(cos0 * a.x + sin0 * a.y, cos0 * a.y - sin0 * a.x, bh[j][0], bl[j][0]);
+                        ap_split(cos1 * b.x + sin1 * b.y, cos1 * b.y - sin1 * b.x, bh[j][1], bl[j][1]);
                     }
+                    if (half == 0) load_far(p0, 4 + k4, k4);
 #pragma unroll
-                    for (int i = 0; i < 4; i += 2) {                // two tiles of rows: four sums in turn, so that none waits for its last product
+                    for (int i = 0; i < 4; ++i) {
                         if (uint32_t(i) >= n_mt) break;
                         const uint8_t* at = s_q + ((i * 8 + ks) * 32 + lane) * 16;
-                        const uint4 ah0 = *reinterpret_cast<const uint4*>(at), al0 = *reinterpret_cast<const uint4*>(at + kApPlane);
-                        const uint4 ah1 = *reinterpret_cast<const uint4*>(at + 4096), al1 = *reinterpret_cast<const uint4*>(at + kApPlane + 4096);
+                        const uint4 ah = *reinterpret_cast<const uint4*>(at), al = *reinterpret_cast<const uint4*>(at + kApPlane);
+                        // the tensor core's sums truncate: those of 16 values each are added here
+                        float d[2][4] = {};
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) { ap_mma(s[i][j], al0, bh[j][0], bh[j][1]); ap_mma(s[i + 1][j], al1, bh[j][0], bh[j][1]); }
+                        for (int j = 0; j < 2; ++j) ap_mma(d[j], al, bh[j][0], bh[j][1]);
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) { ap_mma(s[i][j], ah0, bl[j][0], bl[j][1]); ap_mma(s[i + 1][j], ah1, bl[j][0], bl[j][1]); }
+                        for (int j = 0; j < 2; ++j) ap_mma(d[j], ah, bl[j][0], bl[j][1]);
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) { ap_mma(s[i][j], ah0, bh[j][0], bh[j][1]); ap_mma(s[i + 1][j], ah1, bh[j][0], bh[j][1]); }
+                        for (int j = 0; j < 2; ++j) ap_mma(d[j], ah, bh[j][0], bh[j][1]);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j)
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) s[i][j][c] += d[j][c];
                     }
                 }
             }
@@ -251,7 +301,7 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
 #pragma unroll
                     for (int c = 0; c < 2; ++c) {
                         float& x = s[i][j][2 * u + c];
-                        x = my0 + 8 * j + 2 * t + c <= P + r ? x * f : -INFINITY;
+                        x = my0 + 8 * j + 2 * t + c <= P + r ? x * (f * key_unit[j][c]) : -INFINITY;
                         top = fmaxf(top, x);
                     }
                 top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
@@ -313,38 +363,58 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
         };
         // A row must not depend on keys behind it, and a probability of 0 does not take a value out of a product that is not finite (an entry
         // of the cache that left the range of f16).  So a warp looks for such values in chunks with keys that some row does not see, leaves
-        // them out of the products and adds them below to the rows that see them.
+        // them out of the products and adds them below to the rows that see them.  0 x value is NaN for them and stays so in a sum.
+        const bool look = p0 + kApKeys - 1 > P;
         bool odd = false;
-        if (p0 + kApKeys - 1 > P) {
-            __half2 nan = __float2half2_rn(0.f);
+        auto look_at = [](__half2& seen, const uint32_t (&b)[4]) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) seen = __hfma2(*reinterpret_cast<const __half2*>(&b[i]), __half2{}, seen);
+        };
+        auto is_odd = [](__half2 seen) { return __any_sync(0xffffffffu, __hisnan(__low2half(seen)) || __hisnan(__high2half(seen))) != 0; };
+        if (!ONE_PASS && look) {
+            __half2 seen = {};
             for (uint32_t ks = 0; ks < steps; ++ks) {
                 uint32_t b[4];
                 load_values(b, ks);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) nan = __hfma2(*reinterpret_cast<const __half2*>(&b[i]), __float2half2_rn(0.f), nan);
+                look_at(seen, b);
             }
-            odd = __any_sync(0xffffffffu, __hisnan(__low2half(nan)) || __hisnan(__high2half(nan)));
+            odd = is_odd(seen);
         }
+        while (true) {
+            __half2 seen = {};
+#pragma unroll 1
+            for (uint32_t ks = 0; ks < steps; ++ks) {
+                uint32_t b[4];
+                load_values(b, ks);
+                if (ONE_PASS) look_at(seen, b);
+                if (odd) {
 #pragma unroll
-        for (uint32_t ks = 0; ks < uint32_t(kApWarps); ++ks) {
-            if (ks >= steps) break;
-            uint32_t b[4];
-            load_values(b, ks);
-            if (odd) {
+                    for (int i = 0; i < 4; ++i) b[i] = ap_finite(b[i]);
+                }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) b[i] = ap_finite(b[i]);
+                for (int i = 0; i < 4; ++i) {
+                    if (uint32_t(i) >= n_mt) break;
+                    const uint8_t* at = s_k + ((i * 8 + ks) * 32 + lane) * 16;
+                    const uint4 ah = *reinterpret_cast<const uint4*>(at), al = *reinterpret_cast<const uint4*>(at + kApPlane);
+                    float d[2][4] = {};
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) ap_mma(d[j], al, b[2 * j], b[2 * j + 1]);
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) ap_mma(d[j], ah, b[2 * j], b[2 * j + 1]);
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) o[i][j][c] += d[j][c];
+                }
             }
+            if (!ONE_PASS || !look || odd || !is_odd(seen)) break;
+            odd = true;                                             // once more, without them
 #pragma unroll
-            for (int i = 0; i < 4; i += 2) {
-                if (uint32_t(i) >= n_mt) break;
-                const uint8_t* at = s_k + ((i * 8 + ks) * 32 + lane) * 16;
-                const uint4 ah0 = *reinterpret_cast<const uint4*>(at), al0 = *reinterpret_cast<const uint4*>(at + kApPlane);
-                const uint4 ah1 = *reinterpret_cast<const uint4*>(at + 4096), al1 = *reinterpret_cast<const uint4*>(at + kApPlane + 4096);
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 2; ++j) { ap_mma(o[i][j], al0, b[2 * j], b[2 * j + 1]); ap_mma(o[i + 1][j], al1, b[2 * j], b[2 * j + 1]); }
+                for (int j = 0; j < 2; ++j)
 #pragma unroll
-                for (int j = 0; j < 2; ++j) { ap_mma(o[i][j], ah0, b[2 * j], b[2 * j + 1]); ap_mma(o[i + 1][j], ah1, b[2 * j], b[2 * j + 1]); }
-            }
+                    for (int c = 0; c < 4; ++c) o[i][j][c] = 0.f;
         }
         if (odd) {
             for (uint32_t k = 0; k < 16 * steps; ++k) {
@@ -373,7 +443,7 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
         if (ONE_PASS) break;
         if (chunk + C < n_chunks) {
             load_rows((chunk + C) * kApKeys);
-            load_table((chunk + C) * kApKeys, 0);
+            load_first_far((chunk + C) * kApKeys);
         }
     }
 

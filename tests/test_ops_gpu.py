@@ -403,6 +403,40 @@ def test_prompt_attention(gpu, pkg, rope_table, batch, pos, max_ctx):
         gpu.free(d)
 
 
+def exact_attention(table, k, v, q, P):
+    """One row over positions 0 .. P in 64 bits, turned by the rows of the rotation table."""
+    kk = k[:P + 1].view(np.float16).astype(np.float64).reshape(P + 1, HEADS, ROT // 2, 2)
+    t = table[P - np.arange(P + 1)].astype(np.float64)[:, None]
+    turned = np.stack([t[..., 0] * kk[..., 0] + t[..., 1] * kk[..., 1], t[..., 0] * kk[..., 1] - t[..., 1] * kk[..., 0]], -1).reshape(P + 1, HEADS, ROT)
+    s = np.einsum("hd,phd->ph", q.astype(np.float64).reshape(HEADS, ROT), turned) / np.sqrt(ROT)
+    e = np.exp(s - s.max(0))
+    return np.einsum("ph,phd->hd", e / e.sum(0), v[:P + 1].view(np.float16).astype(np.float64).reshape(P + 1, HEADS, ROT)).ravel()
+
+
+@pytest.mark.parametrize("batch,pos", [(64, 0), (50, 60)])
+@pytest.mark.parametrize("size", [1.0, 1e-2, 1e-3, 2.0 ** -14, 30.0, 2.0 ** 12])
+def test_prompt_attention_of_small_and_large_keys(gpu, pkg, rope_table, batch, pos, size):
+    """Keys of any size of f16, with queries that make scores of a few units, are as exact as f32 sums make them: scores of 128 products, the
+    rounding of the table's angles (2^-19 at distances of up to 63) and the sums of the weighted values each leave about 2^-23."""
+    rng = np.random.default_rng(700 + batch)
+    max_ctx = 128
+    k, v = _caches(rng, pos + batch, max_ctx)
+    k = np.zeros((max_ctx, DIM), np.float16)
+    k[:pos + batch] = (rng.standard_normal((pos + batch, DIM)) * size).astype(np.float16)
+    q = (rng.standard_normal((batch, DIM)) / size).astype(np.float32)
+    q[0, :ROT] *= np.float32(1e-30)                         # scores of next to nothing
+    d_out, scratch = gpu.alloc(batch * DIM * 4), gpu.zeros(gpu.lib.lv_attention_scratch_bytes(HEADS, ROT, max_ctx, batch))
+    args = [gpu.upload(a) for a in (q, k.view(np.uint16), v)]
+    pkg.check(gpu.lib.lv_attention_fused(gpu.handle, d_out, *args, u32_dev(gpu, pos), rope_table, scratch, HEADS, ROT, max_ctx, batch))
+    gpu.sync()
+    got = gpu.download(d_out, np.float32, batch * DIM).reshape(batch, DIM)
+    table = gpu.download(rope_table, np.float32, 128 * ROT).reshape(128, ROT // 2, 2)
+    for z in sorted({0, 1, 17, batch // 2, batch - 1}):
+        close(got[z], exact_attention(table, k.view(np.uint16), v, q[z], pos + z), rel_l2=7e-7, max_abs_frac=3e-6)
+    for d in args + [d_out, scratch]:
+        gpu.free(d)
+
+
 @pytest.mark.parametrize("batch,pos,max_ctx", [(64, 0, 128), (50, 100, 256), (64, 448, 512), (70, 90, 256)])
 def test_prompt_attention_rows_do_not_depend_on_later_values(gpu, pkg, rope_table, batch, pos, max_ctx):
     """Values of the cache that are not finite (the append rounds to f16) reach the rows that see them, and no row before: against the same
