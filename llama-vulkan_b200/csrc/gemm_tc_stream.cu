@@ -3,15 +3,15 @@
 //   out[z][r] = sum_k W[r][k] * x[z][k]        z < Z <= 64
 //
 // The work is a list of units: tiles of 128 rows (64 + 64 of a SiLU pair) times groups of 256 columns, tile by tile.  A persistent
-// launch of at most one CTA per SM gives every CTA an equal run of consecutive units, wherever tiles begin and end in it: a run is cut
-// into segments, one per tile that it touches.  A segment that covers a whole tile is finished by its CTA; of the others the partial
+// launch of at most one CTA per SM gives every CTA an equal run of consecutive units, wherever tiles begin and end in it (or an equal share of
+// one tile, see launch_typed): a run is cut into segments, one per tile that it touches.  A segment that covers a whole tile is finished by its CTA; of the others the partial
 // accumulators go to scratch, every CTA reports all of its tiles once at its end, and the last one to report a tile adds the parts
 // in the order of K (deterministic) and applies the epilogue.
 //
 // What bounds it: one CTA per row tile and share of K ran in waves that were filled to 60-80 %, and paid set-up, ring filling and the
 // pass over the parts in every wave; within a wave two raw stages and one barrier hand-over per 64 columns made a group take 1.2 us
-// where the tensor pipe needs 0.5 us (Z = 64) and HBM 0.4 us.  Here those costs are paid once per launch, the weights arrive through four or
-// more raw stages, and activations are handed over 128 columns at a time.
+// where the tensor pipe needs 0.5 us (Z = 64) and HBM 0.4 us.  Here those costs are paid once per launch, the weights arrive through three
+// (q8_0) or four and more raw stages, and activations are handed over 128 columns at a time.
 //
 // Roles (20 warps):
 //   0..15  producers.  A warp reaches only its own quarter of the tensor memory's lanes (= tile rows), so warp w dequantises rows
@@ -24,10 +24,14 @@
 //   19     activation ring: one bulk copy per two tiles of K (q8_0, whose raw stages are larger: one).  The number of stages is even, so that
 //          a stage always belongs to one issuing lane (a parity wait cannot tell a phase from the one two uses later).
 //
-// us per launch, one CTA per tile and share of K -> this, 16 / 64 tokens of q4_0: 11008 x 4096 pair 42.9 -> 35.7 / 47.7 -> 43.6, 4096 x 11008 22.0 ->
-// 17.5 / 24.2 -> 24.1, 4096 x 4096 10.2 -> 10.7 / 12.0 -> 12.5 back to back; behind a smaller kernel the set-up is hidden (a prompt of 1024 tokens,
-// 7B q4_0: 91.5 -> 83.4 ms).  A unit takes about 1700 clocks: 700 of dequantisation, 450 of waiting for and fetching raw words, 90 of tcgen05.st, the
-// rest loop, barriers and drains; the tensor pipe needs 1024 of them at 64 tokens.
+// us per launch, one CTA per tile and share of K -> this, 16 / 64 tokens of q4_0: 11008 x 4096 pair 42.7 -> 35.8 / 47.7 -> 43.5, 4096 x 11008 21.8 ->
+// 17.5 / 24.1 -> 20.3, 4096 x 4096 10.1 -> 10.7 / 11.9 -> 12.4 (q8_0 10.4 -> 12.0 / 12.5 -> 13.7) back to back; behind a smaller kernel the set-up is
+// hidden and four raw stages arrive with it (sessions of 16, eight layers of 4096: 7.6 ms with the old form of this shape, 7.2 with this).  A
+// unit takes about 1700 clocks: 700 of dequantisation, 450 of waiting for and fetching raw words, 90 of tcgen05.st, the rest loop, barriers
+// and drains; the tensor pipe needs 1024 of them at 64 tokens.
+//
+// An accumulator takes a whole segment, up to 16 units of 4096 columns: the error beside the rounding of the weights is 3.7e-6 of a gated pair (2.4e-6
+// with two shares of K), 1.4e-6 of the three attention products (8.5e-7), against 2.1e-4 and 1.8e-4 that the weights leave.
 //
 // Every wait is bounded (common.cuh); a lost wait sets the context's error word, the CTA drains and frees its tensor memory.
 #include <cstdlib>
@@ -51,6 +55,7 @@ template <int QT> __host__ __device__ constexpr uint32_t ts_b_tiles() { return Q
 struct TsPlan {
     uint32_t units, per;       // units of the launch and of a CTA
     uint32_t groups;           // units of a tile
+    uint32_t shares;           // 0: runs of `per` units; otherwise CTAs of a tile, each with an equal part of its units
     uint32_t n_raw, n_b;       // stages of the two rings
 };
 
@@ -200,8 +205,13 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
         row0 = (tile - (mi == 2 ? t1 : (mi == 1 ? t0 : 0))) * rows_per_tile;
         return mi;
     };
-    const uint32_t G = plan.groups, u0 = blockIdx.x * plan.per, n_units = min(plan.units, u0 + plan.per) - u0;
+    const uint32_t G = plan.groups, shares = plan.shares, share = shares != 0 ? blockIdx.x % shares : 0u;
+    const uint32_t u0 = shares != 0 ? blockIdx.x / shares * G + G * share / shares : blockIdx.x * plan.per;
+    const uint32_t n_units = (shares != 0 ? u0 - G * share / shares + G * (share + 1) / shares : min(plan.units, u0 + plan.per)) - u0;
     const uint32_t tile0 = u0 / G, g0 = u0 - tile0 * G;     // where this CTA's run begins
+    // the CTAs that work on tile t
+    auto first_of = [&](uint32_t t) { return shares != 0 ? t * shares : t * G / plan.per; };
+    auto last_of = [&](uint32_t t) { return shares != 0 ? t * shares + shares - 1 : ((t + 1) * G - 1) / plan.per; };
     const uint32_t bank_cols = 2u * p.zpad;
 
     // one barrier per thread (a single thread takes about a microsecond for all of them)
@@ -460,7 +470,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
                 const uint32_t t = threadIdx.x == 0 ? tile0 : last_tile;
                 uint32_t mine = 0;
                 if (threadIdx.x == 0 ? cut_first : cut_last) {
-                    const uint32_t parts = ((t + 1) * G - 1) / plan.per - t * G / plan.per + 1;
+                    const uint32_t parts = last_of(t) - first_of(t) + 1;
                     __threadfence();
                     if (atomicAdd(&p.counters[t], 1u) + 1 == parts) {
                         mine = 1;
@@ -477,7 +487,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
             const uint32_t n_warps = both ? kTsProducers / 2 : kTsProducers;
             if (*reinterpret_cast<volatile uint32_t*>(&s_last[k]) != 0 && ok) {
                 const uint32_t t = k == 0 ? tile0 : last_tile;
-                const uint32_t c_first = t * G / plan.per, c_last = ((t + 1) * G - 1) / plan.per;
+                const uint32_t c_first = first_of(t), c_last = last_of(t);
                 uint32_t row0;
                 const int mi = matrix_of(t, row0);
                 const GemvMatrix& M = p.m[mi];
@@ -489,7 +499,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
                         float4 x[kParts][kTok];
 #pragma unroll
                         for (uint32_t j = 0; j < kParts; ++j) {
-                            const uint32_t c = min(cb + j, c_last), slot = c * plan.per >= t * G ? 0u : 1u;        // its first segment, or its last
+                            const uint32_t c = min(cb + j, c_last), slot = shares != 0 || c * plan.per >= t * G ? 0u : 1u;        // its first segment, or its last
                             const float* q = p.scratch + size_t(2 * c + slot) * p.zpad * kTcRows + 4 * lane;
 #pragma unroll
                             for (uint32_t i = 0; i < kTok; ++i)
@@ -546,15 +556,23 @@ static int launch_typed(lv_ctx* ctx, const GemmTcParams& p, const GemmTcMaps& ma
     const uint32_t sms = uint32_t(ctx->sm_count);
     // equal runs; at least two units each, since a part costs about as much as two units
     plan.per = max((plan.units + sms - 1) / sms, min(2u, plan.groups));
+    // Runs that begin and end inside tiles have two segments, and tiles up to eight parts: about two units more for the CTA that ends last.  Where
+    // equal shares of every tile fit the SMs with no more units than that, each CTA has one segment.  us per launch back to back, q4_0, runs -> shares:
+    //   tokens   2048 x 5632    3 x 2048 x 2048   5120 x 5120    4096 x 11008    1408 x 4096 pair
+    //     16     11.6 -> 10.2   10.3 ->  9.5      13.0 -> 12.3   17.5 -> 17.5    10.9 ->  9.9
+    //     64     18.4 -> 13.1   14.9 -> 11.7      17.7 -> 14.3   24.0 -> 20.3    17.3 -> 12.6
+    // and a prompt of 512 tokens in steps of 64, four layers 2048 wide: 3.31 -> 3.05 ms.
+    const uint32_t most = sms / tiles, n_shares = most == 0 ? 0 : max((plan.groups + most - 1) / most, min(2u, plan.groups));      // units of a CTA
+    if (most > 1 && plan.groups % plan.per != 0 && n_shares <= plan.per + 2) plan.shares = (plan.groups + n_shares - 1) / n_shares;
     // whole tiles only, where the arrival counters or the scratch (two parts per CTA) would not do
     static const char* no_split = getenv("LV_GEMM_TC_NO_SPLIT");
     if (tiles > kTcMaxTiles || size_t(sms) * 2 * p.zpad * kTcRows * sizeof(float) > kTcScratchBytes || (no_split != nullptr && no_split[0] == '1'))
-        plan.per = (tiles + sms - 1) / sms * plan.groups;
+        plan.per = (tiles + sms - 1) / sms * plan.groups, plan.shares = 0;
     // shared memory: up to 128 KB of activations (96 KB beside the larger q8_0 stages) in an even number of stages, the rest raw stages
     const uint32_t b_stage = ts_b_tiles<QT>() * 4u * p.zpad * kTcChunkK;
     plan.n_b = min(uint32_t(kTsMaxB), (QT == T_Q4_0 ? 131072u : 98304u) / b_stage) & ~1u;
     plan.n_raw = min(uint32_t(kTsMaxRaw), (kTsSmemBytes - 1024 - kTsGateBytes - kTsBarBytes - plan.n_b * b_stage) / uint32_t(tc_raw_stage<QT>()));
-    LV_CUDA((launch_pdl(ctx, gemm_tc_stream_kernel<QT>, dim3((plan.units + plan.per - 1) / plan.per), dim3(kTsThreads), kTsSmemBytes, p, plan, maps)));
+    LV_CUDA((launch_pdl(ctx, gemm_tc_stream_kernel<QT>, dim3(plan.shares != 0 ? tiles * plan.shares : (plan.units + plan.per - 1) / plan.per), dim3(kTsThreads), kTsSmemBytes, p, plan, maps)));
     return LV_OK;
 }
 

@@ -289,10 +289,11 @@ def test_gemm_tc_silu_pair_on_the_shards_of_eight_ranks(gpu, pkg, ff, dim, batch
 
 
 @pytest.mark.parametrize("wtype", [qn.Q4_0, qn.Q8_0], ids=["q4_0", "q8_0"])
-@pytest.mark.parametrize("rows,cols,batch", [(32, 256, 64), (160, 256, 17), (4096, 256, 48), (19008, 512, 33), (4096, 2816, 64), (992, 5120, 1), (131200, 256, 6)])
+@pytest.mark.parametrize("rows,cols,batch", [(32, 256, 64), (160, 256, 17), (4096, 256, 48), (19008, 512, 33), (4096, 2816, 64), (992, 5120, 1), (131200, 256, 6),
+                                             (2048, 5632, 37), (608, 4352, 5), (128, 3840, 64)])
 def test_gemm_tc_runs_of_units(gpu, pkg, rows, cols, batch, wtype, form):
     """Every SM takes an equal run of (row tile, 256 columns): tiles of one unit, runs inside a tile, over several whole tiles and over the
-    edges of tiles, more tiles than arrival counters (whole tiles only).  Against float64 with the weights rounded to fp16, which is what
+    edges of tiles, more tiles than arrival counters (whole tiles only), equal shares of every tile.  Against float64 with the weights rounded to fp16, which is what
     this form multiplies: left are 22-bit activations (2^-23 each) and f32 sums, below 1e-5 of the result."""
     if form == "exact":
         pytest.skip("another kernel")
