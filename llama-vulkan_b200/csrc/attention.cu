@@ -417,7 +417,10 @@ int attention_configure(lv_ctx* ctx) {
 //     12          14.2 / 13.9     28.7 / 14.1      50.6 / 16.1      92.3 / 27.9
 //     64          65.7 / 20.8    124.6 / 21.7     237.2 / 24.5     459.6 / 38.0
 // (contexts of up to 128: 8 rows 7.0 / 7.1, 12 rows 10.5 / 7.2, 64 rows 45.6 / 11.7)
-static bool use_prompt_attention(uint32_t batch, uint32_t max_ctx) { return batch >= 12 || (batch >= 8 && max_ctx > 512); }
+// (the products store 16 bytes at a time)
+static bool use_prompt_attention(const void* out, uint32_t batch, uint32_t max_ctx) {
+    return (batch >= 12 || (batch >= 8 && max_ctx > 512)) && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+}
 
 // Grids of at most one CTA per SM stage key rows and the exact table rows in shared memory; larger
 // ones (context beyond ~1280 rows, batches) stage key rows and the compact table, two CTAs per SM.
@@ -546,7 +549,7 @@ extern "C" int lv_attention_fused(lv_ctx* ctx, float* out, const float* q, const
     LV_ENTER(ctx);
     LV_REQUIRE(out && q && k_cache && v_cache && pos && rope_table && scratch, "null argument");
     if (int rc = check_attn_shape(max_ctx, heads, rot, batch)) return rc;
-    if (use_prompt_attention(batch, max_ctx)) return launch_attention_prompt(ctx, out, q, k_cache, v_cache, pos, rope_table, heads, max_ctx, batch);
+    if (use_prompt_attention(out, batch, max_ctx)) return launch_attention_prompt(ctx, out, q, k_cache, v_cache, pos, rope_table, heads, max_ctx, batch);
     const uint32_t nchunks = (max_ctx + kAttnChunk - 1) / kAttnChunk;
     uint32_t* counters = static_cast<uint32_t*>(scratch);
     float* partial = static_cast<float*>(scratch) + attn_counter_words(heads, batch);
@@ -561,7 +564,7 @@ extern "C" int lv_attention_fused_split(lv_ctx* ctx, void* xh_out, const float* 
     LV_REQUIRE(xh_out && q && k_cache && v_cache && pos && rope_table && scratch && (reinterpret_cast<uintptr_t>(xh_out) & 15u) == 0, "null or misaligned argument");
     if (int rc = check_attn_shape(max_ctx, heads, rot, batch)) return rc;
     LV_REQUIRE(batch <= 64, "split activations have at most 64 rows");
-    if (use_prompt_attention(batch, max_ctx)) return launch_attention_prompt(ctx, nullptr, q, k_cache, v_cache, pos, rope_table, heads, max_ctx, batch, xh_out);
+    if (use_prompt_attention(xh_out, batch, max_ctx)) return launch_attention_prompt(ctx, nullptr, q, k_cache, v_cache, pos, rope_table, heads, max_ctx, batch, xh_out);
     const uint32_t nchunks = (max_ctx + kAttnChunk - 1) / kAttnChunk;
     uint32_t* counters = static_cast<uint32_t*>(scratch);
     float* partial = static_cast<float*>(scratch) + attn_counter_words(heads, batch);

@@ -466,6 +466,27 @@ def test_prompt_attention_rows_do_not_depend_on_later_values(gpu, pkg, rope_tabl
         gpu.free(d)
 
 
+@pytest.mark.parametrize("batch,pos,max_ctx", [(12, 30, 128), (64, 300, 512), (64, 1900, 2048)])
+def test_attention_of_rows_that_are_not_aligned(gpu, pkg, rope_table, batch, pos, max_ctx):
+    """Outputs 4 bytes behind a 16-byte boundary were always taken."""
+    rng = np.random.default_rng(900 + batch)
+    k, v = _caches(rng, pos + batch, max_ctx)
+    q = rng.standard_normal((batch, DIM)).astype(np.float32)
+    scratch, d_out = gpu.zeros(gpu.lib.lv_attention_scratch_bytes(HEADS, ROT, max_ctx, batch)), gpu.zeros((batch * DIM + 4) * 4)
+    args = [gpu.upload(a) for a in (q, k, v)]
+    pkg.check(gpu.lib.lv_attention_fused(gpu.handle, pkg.offset(d_out, 4), *args, u32_dev(gpu, pos), rope_table, scratch, HEADS, ROT, max_ctx, batch))
+    gpu.sync()
+    got = gpu.download(d_out, np.float32, batch * DIM + 4)
+    assert got[0] == 0 and not got[-3:].any()
+    backlog = 128
+    while backlog < pos + batch:
+        backlog *= 2
+    for z in (0, batch - 1):
+        close(got[1:-3].reshape(batch, DIM)[z], ob.attention(k, v, q[z], pos + z, backlog, HEADS, ROT), rel_l2=1e-5, max_abs_frac=2e-5)
+    for d in args + [scratch, d_out]:
+        gpu.free(d)
+
+
 def test_prompt_attention_of_several_passes_repeats_itself(gpu, pkg, rope_table):
     """More than 1024 positions: a CTA brings new keys to where it kept probabilities.  The same bits from every launch, and the first
     rows of a step the same bits as in a shorter one."""
