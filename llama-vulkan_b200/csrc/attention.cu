@@ -410,16 +410,22 @@ int attention_configure(lv_ctx* ctx) {
     return LV_OK;
 }
 
-// Whether lv_attention_fused takes the matrix products of attention_prompt.cu.  Measured on the heads of LLaMA-7B, in a chain of launches,
-// one CTA per row, head and 256 positions here / products there, us:
-//   rows    context 200 of 512    500 of 512    1000 of 1024    1950 of 2048
-//      8           9.4 / 13.8     20.5 / 14.0      36.9 / 15.7      64.1 / 27.3
-//     12          14.2 / 13.9     28.7 / 14.1      50.6 / 16.1      92.3 / 27.9
-//     64          65.7 / 20.8    124.6 / 21.7     237.2 / 24.5     459.6 / 38.0
-// (contexts of up to 128: 8 rows 7.0 / 7.1, 12 rows 10.5 / 7.2, 64 rows 45.6 / 11.7)
-// (the products store 16 bytes at a time)
-static bool use_prompt_attention(const void* out, uint32_t batch, uint32_t max_ctx) {
-    return (batch >= 12 || (batch >= 8 && max_ctx > 512)) && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+// Whether lv_attention_fused takes the matrix products of attention_prompt.cu.  us in a chain of launches, one CTA per row, head and 256 positions here /
+// products there:
+//               32 heads                          8 heads                          4 heads
+//   rows    up to 128   450 of 512  1000 of 1024   up to 128   450 of 512  1000 of 1024   up to 128   450 of 512  1000 of 1024
+//      8     7.7          20 / 14     35 / 15       4.7          8 / 11      11 / 12       4.7         8            8 / 11
+//     12    12 / 9        28 / 14     48 / 15       4.9 / 8      11 / 11     17 / 12       4.8 / 8     8 / 11      11 / 11
+//     32    25 / 10       64 / 15    119 / 17       7.9 / 9      20 / 11     36 / 13       4.9 / 8    11 / 11      20 / 12
+//     64    47 / 14      123 / 23    233 / 25        15 / 13     36 / 16     63 / 18       8.1 / 13   20 / 16      36 / 16
+// The kernel here runs up to two CTAs per SM at a time; below that it is as fast or faster, and exact in the angles (grids of one CTA per SM), so the line lies
+// where its CTAs are more than two per SM, three for steps of more than 32 rows, whose products take half as long again, and five where the products
+// take several passes (more than 1024 positions: 12 rows of 4 heads at 1100 of 2048 11 / 20, 16 rows of 8 heads 25 / 20).  (Measured at positions beyond
+// half of the context, as sessions have them; 12 rows of 16 heads at 200 of 512 take 9 / 13.)  Steps of fewer than twelve rows only with more
+// than 512 positions: at 200 of 512, 32 heads, 8 rows take 9.4 / 14.  The products store 16 bytes at a time.
+static bool use_prompt_attention(const lv_ctx* ctx, const void* out, uint32_t heads, uint32_t nchunks, uint32_t max_ctx, uint32_t batch) {
+    if (batch < 8 || (batch < 12 && max_ctx <= 512) || (reinterpret_cast<uintptr_t>(out) & 15u) != 0) return false;
+    return size_t(heads) * nchunks * batch > size_t(max_ctx > 1024 ? 5 : batch > 32 ? 3 : 2) * ctx->sm_count;
 }
 
 // Grids of at most one CTA per SM stage key rows and the exact table rows in shared memory; larger
@@ -549,8 +555,9 @@ extern "C" int lv_attention_fused(lv_ctx* ctx, float* out, const float* q, const
     LV_ENTER(ctx);
     LV_REQUIRE(out && q && k_cache && v_cache && pos && rope_table && scratch, "null argument");
     if (int rc = check_attn_shape(max_ctx, heads, rot, batch)) return rc;
-    if (use_prompt_attention(out, batch, max_ctx)) return launch_attention_prompt(ctx, out, q, k_cache, v_cache, pos, rope_table, heads, max_ctx, batch);
     const uint32_t nchunks = (max_ctx + kAttnChunk - 1) / kAttnChunk;
+    if (use_prompt_attention(ctx, out, heads, nchunks, max_ctx, batch))
+        return launch_attention_prompt(ctx, out, q, k_cache, v_cache, pos, rope_table, heads, max_ctx, batch);
     uint32_t* counters = static_cast<uint32_t*>(scratch);
     float* partial = static_cast<float*>(scratch) + attn_counter_words(heads, batch);
     dim3 grid(heads, nchunks, batch);
@@ -564,8 +571,9 @@ extern "C" int lv_attention_fused_split(lv_ctx* ctx, void* xh_out, const float* 
     LV_REQUIRE(xh_out && q && k_cache && v_cache && pos && rope_table && scratch && (reinterpret_cast<uintptr_t>(xh_out) & 15u) == 0, "null or misaligned argument");
     if (int rc = check_attn_shape(max_ctx, heads, rot, batch)) return rc;
     LV_REQUIRE(batch <= 64, "split activations have at most 64 rows");
-    if (use_prompt_attention(xh_out, batch, max_ctx)) return launch_attention_prompt(ctx, nullptr, q, k_cache, v_cache, pos, rope_table, heads, max_ctx, batch, xh_out);
     const uint32_t nchunks = (max_ctx + kAttnChunk - 1) / kAttnChunk;
+    if (use_prompt_attention(ctx, xh_out, heads, nchunks, max_ctx, batch))
+        return launch_attention_prompt(ctx, nullptr, q, k_cache, v_cache, pos, rope_table, heads, max_ctx, batch, xh_out);
     uint32_t* counters = static_cast<uint32_t*>(scratch);
     float* partial = static_cast<float*>(scratch) + attn_counter_words(heads, batch);
     return launch_attention_fused(ctx, dim3(heads, nchunks, batch), nullptr, q, k_cache, v_cache, pos, rope_table, partial, counters, heads, nchunks, max_ctx, rot,

@@ -405,12 +405,13 @@ def test_prompt_attention(gpu, pkg, rope_table, batch, pos, max_ctx):
 
 def exact_attention(table, k, v, q, P):
     """One row over positions 0 .. P in 64 bits, turned by the rows of the rotation table."""
-    kk = k[:P + 1].view(np.float16).astype(np.float64).reshape(P + 1, HEADS, ROT // 2, 2)
+    heads = q.size // ROT
+    kk = k[:P + 1].view(np.float16).astype(np.float64).reshape(P + 1, heads, ROT // 2, 2)
     t = table[P - np.arange(P + 1)].astype(np.float64)[:, None]
-    turned = np.stack([t[..., 0] * kk[..., 0] + t[..., 1] * kk[..., 1], t[..., 0] * kk[..., 1] - t[..., 1] * kk[..., 0]], -1).reshape(P + 1, HEADS, ROT)
-    s = np.einsum("hd,phd->ph", q.astype(np.float64).reshape(HEADS, ROT), turned) / np.sqrt(ROT)
+    turned = np.stack([t[..., 0] * kk[..., 0] + t[..., 1] * kk[..., 1], t[..., 0] * kk[..., 1] - t[..., 1] * kk[..., 0]], -1).reshape(P + 1, heads, ROT)
+    s = np.einsum("hd,phd->ph", q.astype(np.float64).reshape(heads, ROT), turned) / np.sqrt(ROT)
     e = np.exp(s - s.max(0))
-    return np.einsum("ph,phd->hd", e / e.sum(0), v[:P + 1].view(np.float16).astype(np.float64).reshape(P + 1, HEADS, ROT)).ravel()
+    return np.einsum("ph,phd->hd", e / e.sum(0), v[:P + 1].view(np.float16).astype(np.float64).reshape(P + 1, heads, ROT)).ravel()
 
 
 @pytest.mark.parametrize("batch,pos", [(64, 0), (50, 60)])
@@ -463,6 +464,25 @@ def test_prompt_attention_rows_do_not_depend_on_later_values(gpu, pkg, rope_tabl
     assert not np.isfinite(got[1][sees]).any()
     assert np.array_equal(got[0][~sees].view(np.uint32), got[1][~sees].view(np.uint32))
     for d in (dk, dq, at, scratch, d_out):
+        gpu.free(d)
+
+
+@pytest.mark.parametrize("heads,batch,pos,max_ctx", [(4, 12, 100, 128), (4, 12, 400, 512), (2, 64, 60, 128), (5, 14, 480, 512), (4, 36, 20, 256)])
+def test_attention_of_few_heads_keeps_the_exact_angles(gpu, pkg, rope_table, heads, batch, pos, max_ctx):
+    """Steps whose rows fill no more than an SM each are turned by the table row of every distance: f32 sums are all that is left, 2^-22."""
+    rng = np.random.default_rng(800 + batch)
+    dim = heads * ROT
+    k, v = ((rng.standard_normal((max_ctx, dim))).astype(np.float16) for _ in range(2))
+    q = rng.standard_normal((batch, dim)).astype(np.float32)
+    scratch, d_out = gpu.zeros(gpu.lib.lv_attention_scratch_bytes(heads, ROT, max_ctx, batch)), gpu.alloc(batch * dim * 4)
+    args = [gpu.upload(a) for a in (q, k.view(np.uint16), v.view(np.uint16))]
+    pkg.check(gpu.lib.lv_attention_fused(gpu.handle, d_out, *args, u32_dev(gpu, pos), rope_table, scratch, heads, ROT, max_ctx, batch))
+    gpu.sync()
+    got = gpu.download(d_out, np.float32, batch * dim).reshape(batch, dim)
+    table = gpu.download(rope_table, np.float32, 2048 * ROT).reshape(2048, ROT // 2, 2)
+    for z in (0, batch // 2, batch - 1):
+        close(got[z], exact_attention(table, k.view(np.uint16), v.view(np.uint16), q[z], pos + z), rel_l2=4e-7, max_abs_frac=2e-6)
+    for d in args + [scratch, d_out]:
         gpu.free(d)
 
 
