@@ -70,6 +70,20 @@ def test_gemm_bf16_pairs(gpu, rows, cols, batch, nt, splits):
         assert np.array_equal(got[0].view(np.uint32), other.view(np.uint32))
 
 
+@pytest.mark.parametrize("rows,cols,batch,additions", [(1024, 3072, 60, 16), (1024, 3072, 10, 16), (2048, 512, 100, 16), (2048, 512, 16, 16), (576, 4096, 17, 16), (4640, 1024, 10, 16),
+                                                       (2048, 8448, 16, 60), (300, 64, 20, 4)])
+def test_gemm_bf16_keeps_its_sums_short(gpu, rows, cols, batch, additions):
+    """An accumulator of the tensor core truncates: each of the additions of 16 products that follow one another loses about 2e-8 of the
+    result.  Narrow products have no more of them in a row than shares of at least four chunks of K give (16 shares at most, on 148 SMs)."""
+    rng = np.random.default_rng(rows + batch)
+    w, x = weights(rng, rows, cols), weights(rng, batch, cols, scale=1.0)
+    with Dev(gpu) as d:
+        out = d.zeros(batch * rows * 4)
+        d.call("lv_gemm_bf16", out, pkg.TYPE_F32, rows, d.bf16(w), rows, pad8(cols), cols, d.bf16(x), pad8(cols), batch, 1.0, 0)
+        got = d.get(out, (batch, rows))
+    assert rel(got, x.astype(np.float64) @ w.T.astype(np.float64)) < 2.2e-8 * additions + 4e-8
+
+
 def test_gemm_bf16_from_contexts_on_two_threads(gpu):
     """Launches of one kernel with the large and with the small share of an SM's shared memory, from two contexts at once: none is refused."""
     def launches(rows, cols, failed):
