@@ -72,6 +72,12 @@ void llava_session_group::drop_graph() {
     }
 }
 
+bool llava_session_group::wait() {
+    if (lv_stream_sync(ctx->lv(), 0) != LV_OK) return false;
+    feed_unread = false;
+    return true;
+}
+
 // Checks the members, brings their device state up to date (position words, the pending token in the token log)
 // and uploads the member tables if a member's buffers were (re)created since the step was recorded.
 bool llava_session_group::prepare_members(u32* backlog) {
@@ -104,7 +110,8 @@ bool llava_session_group::prepare_members(u32* backlog) {
         uploaded_table.assign(reinterpret_cast<const u8*>(table.data()), reinterpret_cast<const u8*>(table.data()) + table_bytes);
     }
     // the pending tokens and the positions of members that were moved, in one launch (a copy per member and word took about 6 us each).
-    // Every step before this one has been waited for, so the words are free.
+    // A step that failed between its feed and its end has not been waited for.
+    if (feed_unread && !wait()) return false;
     vector<bool> sampled_now;
     for (u32 i = 0; i < k; ++i) {
         llava_session* s = members[i];
@@ -119,6 +126,7 @@ bool llava_session_group::prepare_members(u32* backlog) {
         sampled_now.push_back(s->sampling_on_device());
     }
     if (lv_group_feed(ctx->lv(), static_cast<const lv_group_member*>(tables->device_ptr()), pinned_feed, k, max_backlog_size + 1) != LV_OK) return false;
+    feed_unread = true;
     for (llava_session* s : members) s->device_pos = s->current_tokens_in_gpu;
     if (sampled_now != sampled) {            // the sampler launches are part of the recorded step
         drop_graph();
@@ -190,7 +198,7 @@ bool llava_session_group::step(vector<u32>* next_tokens) {
     lock_guard<mutex> guard(ctx->queue_mutex);
     u32 backlog = 0;
     if (!prepare_members(&backlog) || !record(backlog)) return false;
-    if (lv_graph_launch(ctx->lv(), graph) != LV_OK || lv_stream_sync(ctx->lv(), 0) != LV_OK) {
+    if (lv_graph_launch(ctx->lv(), graph) != LV_OK || !wait()) {
         cerr << "[!] group step failed: " << lv_last_error_string() << endl;
         return false;
     }
@@ -264,7 +272,7 @@ bool llava_session_group::generate_greedy_on_device(u32 n, vector<vector<u32>>* 
     if (!prepare_members(&backlog) || !record(backlog)) return false;
     for (u32 i = 0; i < n; ++i)
         if (lv_graph_launch(ctx->lv(), graph) != LV_OK) return false;           // each step consumes the previous step's tokens
-    if (lv_stream_sync(ctx->lv(), 0) != LV_OK) {
+    if (!wait()) {
         cerr << "[!] group steps failed: " << lv_last_error_string() << endl;
         return false;
     }

@@ -58,6 +58,7 @@ private:
     bool record(u32 backlog);
     bool prepare_members(u32* backlog);
     void drop_graph();
+    bool wait();
 
     llava_context* const ctx;
     std::vector<llava_session*> members;
@@ -68,6 +69,7 @@ private:
     std::vector<bool> sampled;               // per member: the recorded step ends with its sampler launch
     std::vector<u8> uploaded_table;          // the member tables as the device holds them
     lv_group_feed_item* pinned_feed = nullptr;      // what a step takes from the host
+    bool feed_unread = false;                // a launch that reads it has not been waited for
     u32* pinned_tokens = nullptr;
     lv_graph* graph = nullptr;
     u32 graph_backlog = 0;

@@ -7,6 +7,9 @@ with the default fast tiles rel-L2 <= 3e-3 and the same token unless the oracle'
 logits differ.  The per-member references are the oracle's trajectories.
 """
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -184,6 +187,65 @@ def test_group_members_that_sample_draw_with_their_own_sampler(pkg, world):
     g.close()
     for s in alone + grouped:
         s.close()
+
+
+FAILING_LAUNCH = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stdlib.h>
+/* stands in front of liblv_b200.so: refuses one graph launch, and looks whether a feed follows another one that was not waited for */
+int refuse, early;
+static int unread;
+static void* real(const char* name) { return dlsym(dlopen(getenv("LV_REAL"), RTLD_LAZY | RTLD_NOLOAD), name); }
+int lv_graph_launch(void* c, void* g) {
+    if (refuse) { refuse = 0; return 1; }
+    return ((int (*)(void*, void*))real("lv_graph_launch"))(c, g);
+}
+int lv_stream_sync(void* c, int ms) { unread = 0; return ((int (*)(void*, int))real("lv_stream_sync"))(c, ms); }
+int lv_group_feed(void* c, const void* m, const void* feed, unsigned n, unsigned places) {
+    early += unread;
+    unread = 1;
+    return ((int (*)(void*, const void*, const void*, unsigned, unsigned))real("lv_group_feed"))(c, m, feed, n, places);
+}
+"""
+FAILING_STEP = """
+import ctypes as C, os, sys
+sys.path.insert(0, os.path.dirname(sys.argv[1]))
+from conftest import load_pkg
+pkg = load_pkg()
+front = C.CDLL(os.environ["LD_PRELOAD"])
+ctx = pkg.HostContext(sys.argv[2], 0)
+members = []
+for i in range(3):
+    s = ctx.session()
+    s.set_deterministic(True)
+    for t in range(5 + i):
+        assert s.push_token(100 * i + t)
+    tok = s.predict_next_token()
+    assert s.push_token(tok)
+    members.append(s)
+group = pkg.SessionGroup(ctx, members)
+steps = []
+for fail in (False, True, False):
+    C.c_int.in_dll(front, "refuse").value = int(fail)
+    steps.append(group.step())
+    if steps[-1] is not None and len(steps) == 1:
+        assert all(s.push_token(t) for s, t in zip(members, steps[-1]))
+assert steps[0] is not None and steps[1] is None and steps[2] is not None
+assert C.c_int.in_dll(front, "early").value == 0, "the feed was written while a launch could read it"
+group.close()
+"""
+
+
+def test_a_step_after_a_refused_launch_waits_for_its_feed(tmp_path, pkg):
+    source, front, child, path = (str(tmp_path / n) for n in ("front.c", "front.so", "child.py", "tiny.bin"))
+    open(source, "w").write(FAILING_LAUNCH)
+    open(child, "w").write(FAILING_STEP)
+    subprocess.check_call(["gcc", "-shared", "-fPIC", "-o", front, source, "-ldl"])
+    pkg.write_synthetic_model(path, "7b", n_layers=1, wtype=qn.Q4_0)
+    env = dict(os.environ, LD_PRELOAD=front, LV_REAL=os.path.join(os.path.dirname(pkg.__file__), "liblv_b200.so"))
+    done = subprocess.run([sys.executable, child, os.path.abspath(__file__), path], env=env, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
 
 
 @pytest.mark.parametrize("n", [1, 2, 33, 64])
