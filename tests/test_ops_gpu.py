@@ -547,20 +547,29 @@ def test_prompt_attention_leaves_out_rows_outside_the_cache(gpu, pkg, rope_table
 
 
 def test_fused_attention_shares_one_scratch_between_batches_and_contexts(gpu, pkg, rope_table):
-    """A session clears its scratch once and then launches prompt steps of several sizes, single tokens and growing backlogs on it:
-    what the launches with more than one chunk leave there must not reach the arrival counters of the others."""
+    """A session clears its scratch once and then launches short steps of several sizes, single tokens and growing backlogs on it, a group of
+    sessions one row per member: what the launches with more than one chunk leave there must not reach the arrival counters of the others.
+    (A negative batch: the members of a group.  Prompt steps of many rows take the matrix products, which use no scratch.)"""
     rng = np.random.default_rng(33)
     k, v = _caches(rng, 1100, 2048)
     dk, dv = gpu.upload(k), gpu.upload(v)
     shared = gpu.zeros(gpu.lib.lv_attention_scratch_bytes(HEADS, ROT, 2048, 64))
-    for batch, pos, max_ctx in ((64, 300, 512), (37, 364, 512), (1, 401, 512), (64, 512, 1024), (8, 576, 1024), (5, 584, 1024), (1, 1024, 2048), (2, 1030, 2048)):
+    for batch, pos, max_ctx in ((-64, 300, 512), (-37, 364, 512), (1, 401, 512), (-64, 512, 1024), (7, 576, 1024), (5, 584, 1024), (-12, 700, 1024), (64, 800, 1024), (1, 1024, 2048),
+                                (-50, 1028, 2048), (2, 1030, 2048)):
+        at, members = u32_dev(gpu, pos), None
+        if batch < 0:
+            batch = -batch
+            members = gpu.upload(np.array([[dk.value, dv.value, at.value, 0]] * batch, np.uint64))
         dq = gpu.upload(rng.standard_normal((batch, DIM)).astype(np.float32))
         own = gpu.zeros(gpu.lib.lv_attention_scratch_bytes(HEADS, ROT, max_ctx, batch))
         got = []
         for scratch in (shared, own):
             d_out = gpu.alloc(batch * DIM * 4)
             pkg.check(gpu.lib.lv_memset(gpu.handle, d_out, 0xFF, batch * DIM * 4))
-            pkg.check(gpu.lib.lv_attention_fused(gpu.handle, d_out, dq, dk, dv, u32_dev(gpu, pos), rope_table, scratch, HEADS, ROT, max_ctx, batch))
+            if members is not None:
+                pkg.check(gpu.lib.lv_attention_fused_group(gpu.handle, d_out, dq, members, rope_table, scratch, HEADS, ROT, max_ctx, batch))
+            else:
+                pkg.check(gpu.lib.lv_attention_fused(gpu.handle, d_out, dq, dk, dv, at, rope_table, scratch, HEADS, ROT, max_ctx, batch))
             gpu.sync()
             got.append(gpu.download(d_out, np.float32, batch * DIM))
             gpu.free(d_out)
