@@ -495,7 +495,7 @@ typedef struct lv_expert_args {
 int lv_gemv_bf16_expert_gate_up(lv_ctx* ctx, float* out, uint32_t out_ld, const lv_expert_args* a, const float* x, uint32_t x_ld, uint32_t batch);
 int lv_gemv_bf16_expert_down(lv_ctx* ctx, float* out, uint32_t out_ld, const lv_expert_args* a, const float* x, uint32_t x_ld, uint32_t batch);
 
-/* Products of a batch on the tensor cores: x and W bfloat16, f32 sums, one pass over the weights for up to 128 tokens.
+/* Products of a batch on the tensor cores: x and W bfloat16, f32 sums, one pass over the weights for up to 256 tokens.
  * x [batch][x_ld] with x_ld a multiple of 8; out f32 or bfloat16 [batch][out_ld]. */
 int lv_gemm_bf16(lv_ctx* ctx, void* out, int out_type, uint32_t out_ld, const void* w, uint32_t rows, uint32_t ld, uint32_t cols,
                  const void* x, uint32_t x_ld, uint32_t batch, float factor, int act);

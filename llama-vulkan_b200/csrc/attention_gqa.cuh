@@ -27,6 +27,14 @@ __device__ __forceinline__ float cluster_load(const float* local, uint32_t rank)
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at));
     return v;
 }
+// four of them
+__device__ __forceinline__ float4 cluster_load4(const float* local, uint32_t rank) {
+    uint32_t at;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+    return v;
+}
 
 // 1 / rms of one head's vector, computed by a warp (every lane gets it)
 __device__ __forceinline__ float gqa_rms_factor(const float* v, uint32_t dim, float eps) {

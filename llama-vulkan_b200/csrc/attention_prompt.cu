@@ -72,15 +72,6 @@ __device__ __forceinline__ uint32_t ap_finite(uint32_t w) {
     return w;
 }
 
-// four floats in the shared memory of another CTA of the cluster
-__device__ __forceinline__ float4 ap_cluster_load4(const float* local, uint32_t rank) {
-    uint32_t at;
-    float4 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(local)), "r"(rank));
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
-    return v;
-}
-
 // (cos, sin) of two pairs at the distance d (sin turns its sign with it), from the table
 __device__ __forceinline__ float4 ap_table_row(const float* table, int d, uint32_t dim) {
     float4 w = *reinterpret_cast<const float4*>(table + size_t(abs(d)) * kApHead + dim);
@@ -489,7 +480,7 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f), part[kApMaxCluster];
         const float* mine = s_o + r * kApOStride + 4 * lane;
 #pragma unroll
-        for (uint32_t c = 0; c < kApMaxCluster; ++c) part[c] = c < active ? ap_cluster_load4(mine, c) : sum;
+        for (uint32_t c = 0; c < kApMaxCluster; ++c) part[c] = c < active ? cluster_load4(mine, c) : sum;
 #pragma unroll
         for (uint32_t c = 0; c < kApMaxCluster; ++c) {
             const float f = __shfl_sync(0xffffffffu, w, c);

@@ -77,15 +77,6 @@ __host__ __device__ constexpr uint32_t bg_tmem_cols(int NT, bool pair) {
     return need <= 32 ? 32 : need <= 64 ? 64 : need <= 128 ? 128 : need <= 256 ? 256 : 512;
 }
 
-// four floats in the shared memory of another CTA of the cluster
-__device__ __forceinline__ float4 bg_cluster_load4(const float* local, uint32_t rank) {
-    uint32_t at;
-    float4 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(local)), "r"(rank));
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
-    return v;
-}
-
 // grid (row tiles, token tiles, splits), clusters of (TWO ? 2 : 1, 1, splits)
 template <int NT, bool PAIR, bool GROUPED, bool TWO>
 __global__ void __launch_bounds__(kBgThreads, 2) gemm_bf16_kernel(const GemmBf16Params p, const __grid_constant__ GemmBf16Maps maps) {
@@ -272,10 +263,10 @@ __global__ void __launch_bounds__(kBgThreads, 2) gemm_bf16_kernel(const GemmBf16
 #pragma unroll
                 for (int i = 0; i < kTok; ++i) {
                     const uint32_t z = min(z0 + uint32_t(i) * kWarps, n_tok - 1);
-                    const float4 a = bg_cluster_load4(mine + z * kBgRows, TWO ? 2 * c + half : c);
+                    const float4 a = cluster_load4(mine + z * kBgRows, TWO ? 2 * c + half : c);
                     v[i] = make_float4(v[i].x + a.x, v[i].y + a.y, v[i].z + a.z, v[i].w + a.w);
                     if constexpr (PAIR) {
-                        const float4 b = bg_cluster_load4(mine + (NT + z) * kBgRows, TWO ? 2 * c + half : c);
+                        const float4 b = cluster_load4(mine + (NT + z) * kBgRows, TWO ? 2 * c + half : c);
                         g[i] = make_float4(g[i].x + b.x, g[i].y + b.y, g[i].z + b.z, g[i].w + b.w);
                     }
                 }
