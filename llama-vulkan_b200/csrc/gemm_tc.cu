@@ -716,8 +716,8 @@ void gemm_tc_release(lv_ctx* ctx) {
 
 int gemm_tc_configure(lv_ctx* ctx) {
     LV_CUDA(cudaMalloc(&ctx->tc_scratch, kTcScratchBytes));
-    LV_CUDA(cudaMalloc(&ctx->tc_counters, kTcMaxTiles * sizeof(uint32_t)));
-    LV_CUDA(cudaMemset(ctx->tc_counters, 0, kTcMaxTiles * sizeof(uint32_t)));
+    LV_CUDA(cudaMalloc(&ctx->tc_counters, 4 * kTcMaxTiles * sizeof(uint32_t)));
+    LV_CUDA(cudaMemset(ctx->tc_counters, 0, 4 * kTcMaxTiles * sizeof(uint32_t)));
     LV_REQUIRE(size_t(ctx->max_smem_optin) >= tc_smem_bytes<T_Q4_0>() && size_t(ctx->max_smem_optin) >= tc_smem_bytes<T_Q8_0>(),
                "device has too little shared memory for the batched product");
     constexpr size_t kFastSmem = tc_smem_bytes<T_Q4_0, 1>();

@@ -4,9 +4,10 @@
 //
 // The work is a list of units: tiles of 128 rows (64 + 64 of a SiLU pair) times groups of 256 columns, tile by tile.  A persistent
 // launch of at most one CTA per SM gives every CTA an equal run of consecutive units, wherever tiles begin and end in it (or an equal share of
-// one tile, see launch_typed): a run is cut into segments, one per tile that it touches.  A segment that covers a whole tile is finished by its CTA; of the others the partial
-// accumulators go to scratch, every CTA reports all of its tiles once at its end, and the last one to report a tile adds the parts
-// in the order of K (deterministic) and applies the epilogue.
+// one tile, see launch_typed): a run is cut into segments, one per tile that it touches.  A segment that covers a whole tile is finished by its CTA.  Of the others
+// the partial accumulators go to scratch, each reported as soon as it lies there, and whoever comes last adds the parts in the order of K
+// (deterministic) and applies the epilogue: mostly the CTA whose run ends inside the tile, which then takes its own part from its registers.  The
+// four warps that hold sixteen tokens of a tile do this by themselves.
 //
 // What bounds it: one CTA per row tile and share of K ran in waves that were filled to 60-80 %, and paid set-up, ring filling and the
 // pass over the parts in every wave; within a wave two raw stages and one barrier hand-over per 64 columns made a group take 1.2 us
@@ -24,10 +25,10 @@
 //   19     activation ring: one bulk copy per two tiles of K (q8_0, whose raw stages are larger: one).  The number of stages is even, so that
 //          a stage always belongs to one issuing lane (a parity wait cannot tell a phase from the one two uses later).
 //
-// us per launch, one CTA per tile and share of K -> this, 16 / 64 tokens of q4_0: 11008 x 4096 pair 42.7 -> 35.8 / 47.7 -> 43.5, 4096 x 11008 21.8 ->
-// 17.5 / 24.1 -> 20.3, 4096 x 4096 10.1 -> 10.7 / 11.9 -> 12.4 (q8_0 10.4 -> 12.0 / 12.5 -> 13.7) back to back; behind a smaller kernel the set-up is
-// hidden and four raw stages arrive with it (sessions of 16, eight layers of 4096: 7.6 ms with the old form of this shape, 7.2 with this).  A
-// unit takes about 1700 clocks: 700 of dequantisation, 450 of waiting for and fetching raw words, 90 of tcgen05.st, the rest loop, barriers
+// us per launch back to back, 16 / 64 tokens of q4_0: 11008 x 4096 pair 26.3 / 29.5, 4096 x 11008 16.9 / 19.3, 4096 x 4096 9.5 / 11.9 (q8_0 28.0 / 32.3,
+// 18.5 / 20.7, 10.5 / 12.5).  When every CTA reported its parts at its end, the last one read all of them back, and the epilogues were unrolled code that
+// runs once (instruction fetches: 12 us of a whole pair tile), these took 35.8 / 43.5, 17.5 / 20.3, 10.7 / 12.4 (38.2 / 46.5, 18.9 / 23.4, 12.0 / 13.7).
+// A unit takes about 1700 clocks: 700 of dequantisation, 450 of waiting for and fetching raw words, 90 of tcgen05.st, the rest loop, barriers
 // and drains; the tensor pipe needs 1024 of them at 64 tokens.
 //
 // An accumulator takes a whole segment, up to 16 units of 4096 columns: the error beside the rounding of the weights is 3.7e-6 of a gated pair (2.4e-6
@@ -47,7 +48,7 @@ constexpr int kTsThreads = (kTsProducers + 4) * 32;
 constexpr int kTsMaxRaw = 8, kTsMaxB = 16;
 constexpr uint32_t kTsABase = 256, kTsTileCols = kTcChunkK / 2;      // tensor memory: accumulators in columns 0..255, weights from 256 on
 constexpr uint32_t kTsGateBytes = kTcMaxZ * 64 * sizeof(float);      // the epilogue's gate exchange
-constexpr uint32_t kTsBarBytes = 512;
+constexpr uint32_t kTsBarBytes = 640;
 constexpr uint32_t kTsSmemBytes = 227 * 1024;
 // Tiles of K per activation stage: two, where the raw stages leave room for four stages of 64 tokens (32 KB each).
 template <int QT> __host__ __device__ constexpr uint32_t ts_b_tiles() { return QT == T_Q4_0 ? 2u : 1u; }
@@ -77,46 +78,33 @@ __device__ __forceinline__ __half* ts_cache_row(const GemmTcParams& p, const Gem
     return nullptr;
 }
 
-// Stores one value / four consecutive rows of a token.  (mi: matrix of the launch)
-__device__ __forceinline__ void ts_store(const GemmTcParams& p, const GemvMatrix& M, int mi, uint32_t row, uint32_t z, float v) {
-    if (p.split_out != nullptr) {
-        split_store(p.split_out, p.zpad, z, row, v);
-    } else if (M.epilogue == EPI_STORE_F16_AT_POS) {
-        if (__half* to = ts_cache_row(p, M, mi, z)) to[row] = __float2half_rn(v);
-    } else {
-        float* o = static_cast<float*>(M.out) + size_t(z) * M.rows + row;
-        *o = (M.epilogue == EPI_ADD) ? (*o + v) : v;                                   // matmul.glsl:68-72
-    }
-}
-__device__ __forceinline__ void ts_store4(const GemmTcParams& p, const GemvMatrix& M, int mi, uint32_t row, uint32_t z, float4 v) {
-    if (p.split_out != nullptr) {
-        const float x[4] = {v.x, v.y, v.z, v.w};
-        split_store_n<4>(p.split_out, p.zpad, z, row, x);
-        return;
-    }
+// A thread's 16 finished tokens of one row, tokens z0 .. of which the last is below Z.  All residuals of a thread, or the cache rows of a warp's tokens
+// (lane i looks up token z0 + i), are on their way together: one trip to L2.  Called by whole warps; `live` is false for rows beyond the matrix.
+__device__ __forceinline__ void ts_store16(const GemmTcParams& p, const GemvMatrix& M, int mi, uint32_t row, uint32_t z0, bool live, const float (&v)[16]) {
     if (M.epilogue == EPI_STORE_F16_AT_POS) {
-        __half* to = ts_cache_row(p, M, mi, z);
-        if (to == nullptr) return;
-        to += row;
-        const __half2 a = __floats2half2_rn(v.x, v.y), b = __floats2half2_rn(v.z, v.w);
-        if ((reinterpret_cast<uintptr_t>(to) & 7u) == 0) {
-            *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
-        } else {
-            to[0] = a.x; to[1] = a.y; to[2] = b.x; to[3] = b.y;
+        const uint32_t lane = threadIdx.x & 31u;
+        const __half* at = lane < 16 && z0 + lane < p.Z ? ts_cache_row(p, M, mi, z0 + lane) : nullptr;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            __half* to = reinterpret_cast<__half*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(at), i));
+            if (live && to != nullptr) to[row] = __float2half_rn(v[i]);
         }
         return;
     }
-    float* o = static_cast<float*>(M.out) + size_t(z) * M.rows + row;
-    if ((reinterpret_cast<uintptr_t>(o) & 15u) == 0) {
-        float4* o4 = reinterpret_cast<float4*>(o);
-        if (M.epilogue == EPI_ADD) {
-            const float4 x = *o4;
-            v = make_float4(x.x + v.x, x.y + v.y, x.z + v.z, x.w + v.w);
-        }
-        *o4 = v;
+    if (!live) return;
+    float* o = static_cast<float*>(M.out) + size_t(z0) * M.rows + row;
+    if (M.epilogue == EPI_ADD) {                                                       // matmul.glsl:68-72
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (z0 + i < p.Z) x[i] = o[size_t(i) * M.rows];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (z0 + i < p.Z) o[size_t(i) * M.rows] = x[i] + v[i];
     } else {
-        const float x[4] = {v.x, v.y, v.z, v.w};
-        for (int i = 0; i < 4; ++i) o[i] = (M.epilogue == EPI_ADD) ? (o[i] + x[i]) : x[i];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (z0 + i < p.Z) o[size_t(i) * M.rows] = v[i];
     }
 }
 
@@ -186,12 +174,12 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
     uint64_t* a_empty = a_full + 4;                         // [buffer][half]
     uint64_t* acc_full = a_empty + 4;
     uint64_t* acc_empty = acc_full + 1;
-    uint64_t* gate_full = acc_empty + 1;
-    uint64_t* gate_empty = gate_full + 1;
-    constexpr int kBars = 2 * kTsMaxRaw + 2 * kTsMaxB + 12;
+    uint64_t* group_bar = acc_empty + 1;                    // [4] the four warps of a token group
+    constexpr int kBars = 2 * kTsMaxRaw + 2 * kTsMaxB + 14;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kBars);
-    uint32_t* s_last = tmem_slot + 1;                       // [2]
-    static_assert(kBars * 8 + 12 <= int(kTsBarBytes), "barrier area");
+    volatile uint32_t* s_seen = tmem_slot + 1;              // [4] arrivals at the last tile as the four warps of a token group go by
+    volatile uint32_t* s_late = s_seen + 4;                 // [2][4] this CTA's warps were the last to arrive at the first / last tile
+    static_assert(kBars * 8 + 13 * 4 <= int(kTsBarBytes), "barrier area");
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool pair = p.m[0].w_gate != nullptr;
@@ -224,11 +212,12 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
             if (j < 4) count = kTsProducers / 2;                                        // a_full: the eight warps of a half
             else if (j == 8) count = 2;                                                 // acc_full: both issuing lanes
             else if (j == 9) count = kTsProducers;                                      // acc_empty
-            else if (j >= 10) count = kTsProducers / 2;                                 // gate_full, gate_empty
+            else if (j >= 10) count = 4;                                                // group_bar
         }
         mbar_init(&bars[i], count);
         fence_mbar_init();
     }
+    if (threadIdx.x >= kTsThreads - 8) s_late[threadIdx.x - (kTsThreads - 8)] = 0;
     if (warp == kTsProducers + 1) tc_alloc(tmem_slot, 512);
     tc_fence_before_sync();
     __syncthreads();
@@ -289,12 +278,12 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
         for (uint32_t i = 0; i < n_units && ok; ++i) {
             const uint32_t ab = i & 1u;
             // the accumulators of the previous segment have been read
-            if (first && seg > 0) ok = mbar_wait_elect(acc_empty, (seg - 1) & 1u, p.err);
-            ok = ok && mbar_wait_elect(&a_full[2 * ab + h], (i >> 1) & 1u, p.err);
+            if (first && seg > 0) ok = mbar_wait(acc_empty, (seg - 1) & 1u, p.err);
+            ok = ok && mbar_wait(&a_full[2 * ab + h], (i >> 1) & 1u, p.err);
             const uint32_t a_tmem = tmem_base + kTsABase + (4u * ab + 2u * h) * kTsTileCols;
 #pragma unroll
             for (uint32_t st = 0; st < 2 / kBT; ++st) {
-                ok = ok && mbar_wait_elect(&b_full[bs], b_phase, p.err);
+                ok = ok && mbar_wait(&b_full[bs], b_phase, p.err);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint64_t b_desc = b_desc0 + ((bs * b_stage) >> 4);
@@ -329,15 +318,94 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
         const uint32_t tr = quarter * 32u + uint32_t(lane);             // tile row
         const uint32_t lanes_at = (quarter * 32u) << 16;
 
-        uint32_t n_pairs = 0;
-        // reads the accumulators of segment `seg` (16 tokens per warp) and stores or parks them
-        auto drain = [&](uint32_t seg, uint32_t tile, bool whole, uint32_t slot) {
+        // Sixteen tokens of a tile belong to the four warps of one `tt`, a thread has one row of them.  These four warps finish a tile whose
+        // parts come from several CTAs on their own: the counter of (tile, tt) counts warps.
+        const uint32_t z0 = 16u * tt;
+        const bool active = z0 < p.zpad;
+        uint32_t met = 0;
+        auto group_sync = [&]() {                                        // (a bounded wait: a warp may have given up elsewhere)
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&group_bar[tt]);
+            ok = ok && mbar_wait(&group_bar[tt], met & 1u, p.err);
+            ++met;
+            return ok;
+        };
+        auto part_of = [&](uint32_t c, uint32_t t) {                     // CTA c's part of tile t: its first segment, or its last
+            const uint32_t slot = shares != 0 || c * plan.per >= t * G ? 0u : 1u;
+            return p.scratch + (size_t(2 * c + slot) * p.zpad + z0) * kTcRows + tr;
+        };
+        auto arrive = [&](uint32_t t, uint32_t which) {                  // this warp's share of a part is in memory
+            __threadfence();
+            __syncwarp();
+            if (lane == 0 && atomicAdd(&p.counters[4 * t + tt], 1u) + 1 == 4 * (last_of(t) - first_of(t) + 1)) s_late[4 * which + tt] = 1;
+        };
+        // adds the parts of tile t in the order of K (`own` of them from v, none when it is no CTA) and leaves the counter ready for the next launch
+        auto add_parts = [&](uint32_t t, uint32_t own, float (&v)[16]) {
+            const uint32_t c_last = last_of(t);
+            float sum[16] = {};
+#pragma unroll 1
+            for (uint32_t c = first_of(t); c <= c_last; ++c) {
+                float x[16];
+                const float* q = part_of(c, t);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) x[i] = c == own ? v[i] : __ldcg(q + size_t(i) * kTcRows);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) sum[i] += x[i];
+            }
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = sum[i];
+            if (quarter == 0 && lane == 0) p.counters[4 * t + tt] = 0;
+        };
+        auto store = [&](uint32_t t, float (&v)[16]) {
+            uint32_t row0;
+            const int mi = matrix_of(t, row0);
+            const GemvMatrix& M = p.m[mi];
+            if (!pair) {
+                ts_store16(p, M, mi, row0 + tr, z0, row0 + tr < M.rows, v);
+                return;
+            }
+            // Tile rows 64..127 carry the gate (w1) of rows 0..63.  The two warps of a row hand each other eight tokens of what they have and finish
+            // eight each, four at a time in a loop that stays one: this code runs once or twice per launch, and unrolled it took 12 us (11008 x 4096, 16
+            // tokens), nearly all of it instruction fetches.
+            const bool gate = quarter >= 2;
+            float* swap = gate_s + z0 * 64 + (tr & 63u);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) swap[(gate ? i : i + 8) * 64] = gate ? v[i] : v[i + 8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = gate ? v[i + 8] : v[i];
+            if (!group_sync()) return;
+            const uint32_t row = row0 + (tr & 63u), from = gate ? 8 : 0;
+            if (row < M.rows) {
+#pragma unroll 1
+                for (uint32_t at = from; at < from + 8 && z0 + at < p.Z; at += 4) {
+#pragma unroll
+                    for (uint32_t i = 0; i < 4; ++i) {
+                        const float other = swap[(at + i) * 64], y = ts_silu(gate ? other : v[i], gate ? v[i] : other);
+                        const uint32_t z = z0 + at + i;
+                        if (z >= p.Z) break;
+                        if (p.split_out != nullptr) split_store(p.split_out, p.zpad, z, row, y);
+                        else static_cast<float*>(M.out)[size_t(z) * M.rows + row] = y;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v[i] = v[i + 4];
+                }
+            }
+            group_sync();
+        };
+
+        // Reads the accumulators of segment `seg` and stores them, or parks them as a part.  The CTA whose last segment completes a tile (the parts
+        // of the others having arrived long ago, as first segments do) adds them to the values that it holds and leaves nothing behind.  Returns whether a
+        // part was parked whose arrival has still to be reported.
+        auto drain = [&](uint32_t seg, uint32_t tile, bool whole, uint32_t slot, bool final) {
+            pdl_wait();                                        // (outputs, parts and counters may still be in use by the previous kernel)
+            uint32_t seen = 0;
+            const uint32_t parts = last_of(tile) - first_of(tile) + 1;
+            if (!whole && final && active && quarter == 0 && lane == 0) seen = ld_acquire_gpu(&p.counters[4 * tile + tt]);
             ok = mbar_wait_warp_tc(acc_full, seg & 1u, p.err);
-            if (!ok) return;
+            if (!ok) return false;
             tc_fence_after_sync();
-            const uint32_t z0 = 16u * tt;
             float v[16];
-            if (z0 < p.zpad) {
+            if (active) {
                 uint32_t a[16], b[16];
                 tc_load16(a, tmem_base + lanes_at + z0);
                 tc_load16(b, tmem_base + lanes_at + p.zpad + z0);
@@ -353,48 +421,31 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty);
-            pdl_wait();                                        // (outputs may still be read by the previous kernel)
+            if (!active) return false;
             if (!whole) {
-                if (z0 < p.zpad) {
+                bool last = false;
+                if (final) {
+                    if (quarter == 0 && lane == 0) s_seen[tt] = seen;
+                    if (!group_sync()) return false;
+                    last = s_seen[tt] == 4 * (parts - 1);
+                }
+                if (!last) {
                     float* part = p.scratch + (size_t(2 * blockIdx.x + slot) * p.zpad + z0) * kTcRows + tr;
 #pragma unroll
                     for (int i = 0; i < 16; ++i) __stcg(part + size_t(i) * kTcRows, v[i]);
+                    if (!final) return true;
+                    arrive(tile, 1);
+                    if (!group_sync() || s_late[4 + tt] == 0) return false;
+                    __threadfence();
                 }
-                return;
+                add_parts(tile, blockIdx.x, v);
             }
-            uint32_t row0;
-            const int mi = matrix_of(tile, row0);
-            const GemvMatrix& M = p.m[mi];
-            if (pair) {
-                // tile rows 64..127 carry the gate (w1) of rows 0..63
-                if (quarter >= 2 && n_pairs > 0) ok = mbar_wait_warp(gate_empty, (n_pairs - 1) & 1u, p.err);
-                if (tr >= 64 && z0 < p.zpad) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) gate_s[(z0 + i) * 64 + tr - 64] = v[i];
-                }
-                if (quarter < 2) {
-                    ok = mbar_wait_warp(gate_full, n_pairs & 1u, p.err);
-                    if (ok && z0 < p.zpad && row0 + tr < M.rows) {
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            if (z0 + i < p.Z) ts_store(p, M, mi, row0 + tr, z0 + i, ts_silu(v[i], gate_s[(z0 + i) * 64 + tr]));
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(gate_empty);
-                } else {
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(gate_full);
-                }
-                ++n_pairs;
-            } else if (z0 < p.zpad && row0 + tr < M.rows) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (z0 + i < p.Z) ts_store(p, M, mi, row0 + tr, z0 + i, v[i]);
-            }
+            store(tile, v);
+            return false;
         };
 
         uint32_t tile = tile0, g = g0, seg = 0, seg_begin = g0, rs = 0, raw_phase = 0;
-        bool pending = false, pend_whole = false;
+        bool pending = false, pend_whole = false, parked = false;
         uint32_t pend_tile = 0, pend_slot = 0, pend_seg = 0;
         // the raw words of a unit are fetched while the one before it is dequantised (rows are 9 / 17 chunks of 16 bytes apart, so a
         // quarter warp's loads fall into different banks)
@@ -442,8 +493,12 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&a_full[2 * ab + half]);
+            if (parked) {                      // one unit after its stores
+                arrive(tile0, 0);
+                parked = false;
+            }
             if (pending) {
-                drain(pend_seg, pend_tile, pend_whole, pend_slot);
+                parked = drain(pend_seg, pend_tile, pend_whole, pend_slot, false);
                 pending = false;
             }
             if (++g == G || i + 1 == n_units) {
@@ -459,78 +514,14 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
         }
         // (the warps of a CTA may disagree about `ok` only after a lost wait, whose error word ends every later wait; barriers below
         // are reached by all of them)
-        if (ok && pending) drain(pend_seg, pend_tile, pend_whole, pend_slot);
-
-        // ---- tiles that other CTAs work on as well ----
-        const uint32_t u_end = u0 + n_units, last_tile = (u_end - 1) / G;
-        const bool cut_first = g0 != 0 || u_end < (tile0 + 1) * G, cut_last = last_tile != tile0 && u_end < (last_tile + 1) * G;
-        if (cut_first || cut_last) {
-            asm volatile("bar.sync 2, 512;" ::: "memory");
-            if (threadIdx.x < 2) {
-                const uint32_t t = threadIdx.x == 0 ? tile0 : last_tile;
-                uint32_t mine = 0;
-                if (threadIdx.x == 0 ? cut_first : cut_last) {
-                    const uint32_t parts = last_of(t) - first_of(t) + 1;
-                    __threadfence();
-                    if (atomicAdd(&p.counters[t], 1u) + 1 == parts) {
-                        mine = 1;
-                        __threadfence();
-                        p.counters[t] = 0;                          // ready for the next launch
-                    }
-                }
-                s_last[threadIdx.x] = mine;
-            }
-            asm volatile("bar.sync 2, 512;" ::: "memory");
-            // (two tiles are finished side by side)
-            const bool both = *reinterpret_cast<volatile uint32_t*>(&s_last[0]) != 0 && *reinterpret_cast<volatile uint32_t*>(&s_last[1]) != 0;
-            const uint32_t k = both ? uint32_t(warp) / (kTsProducers / 2) : (*reinterpret_cast<volatile uint32_t*>(&s_last[0]) != 0 ? 0u : 1u);
-            const uint32_t n_warps = both ? kTsProducers / 2 : kTsProducers;
-            if (*reinterpret_cast<volatile uint32_t*>(&s_last[k]) != 0 && ok) {
-                const uint32_t t = k == 0 ? tile0 : last_tile;
-                const uint32_t c_first = first_of(t), c_last = last_of(t);
-                uint32_t row0;
-                const int mi = matrix_of(t, row0);
-                const GemvMatrix& M = p.m[mi];
-                // a warp has whole tokens, a lane four rows of them; the parts of four tokens and three CTAs are on their way together
-                constexpr uint32_t kTok = 4, kParts = 3;
-                for (uint32_t zb = uint32_t(warp) % n_warps; zb < p.Z; zb += kTok * n_warps) {
-                    float4 sum[kTok] = {};
-                    for (uint32_t cb = c_first; cb <= c_last; cb += kParts) {
-                        float4 x[kParts][kTok];
-#pragma unroll
-                        for (uint32_t j = 0; j < kParts; ++j) {
-                            const uint32_t c = min(cb + j, c_last), slot = shares != 0 || c * plan.per >= t * G ? 0u : 1u;        // its first segment, or its last
-                            const float* q = p.scratch + size_t(2 * c + slot) * p.zpad * kTcRows + 4 * lane;
-#pragma unroll
-                            for (uint32_t i = 0; i < kTok; ++i)
-                                x[j][i] = __ldcg(reinterpret_cast<const float4*>(q + size_t(min(zb + i * n_warps, p.Z - 1)) * kTcRows));
-                        }
-#pragma unroll
-                        for (uint32_t j = 0; j < kParts; ++j)
-#pragma unroll
-                            for (uint32_t i = 0; i < kTok; ++i)
-                                if (cb + j <= c_last) {
-                                    sum[i].x += x[j][i].x;
-                                    sum[i].y += x[j][i].y;
-                                    sum[i].z += x[j][i].z;
-                                    sum[i].w += x[j][i].w;
-                                }
-                    }
-#pragma unroll
-                    for (uint32_t i = 0; i < kTok; ++i) {
-                        const uint32_t z = zb + i * n_warps, row = row0 + 4 * uint32_t(lane);
-                        if (z >= p.Z) break;
-                        float4 v = sum[i];
-                        if (pair) {                                // lanes 16 .. 31 hold the gate
-                            const float4 gate = make_float4(__shfl_down_sync(0xffffffffu, v.x, 16), __shfl_down_sync(0xffffffffu, v.y, 16),
-                                                            __shfl_down_sync(0xffffffffu, v.z, 16), __shfl_down_sync(0xffffffffu, v.w, 16));
-                            v = make_float4(ts_silu(v.x, gate.x), ts_silu(v.y, gate.y), ts_silu(v.z, gate.z), ts_silu(v.w, gate.w));
-                            if (lane >= 16) continue;
-                        }
-                        if (row < M.rows) ts_store4(p, M, mi, row, z, v);          // (rows come in multiples of 32)
-                    }
-                }
-            }
+        if (ok && parked) arrive(tile0, 0);
+        if (ok && pending) drain(pend_seg, pend_tile, pend_whole, pend_slot, true);
+        // the part of the first tile was the last one after all
+        if (ok && active && group_sync() && s_late[tt] != 0) {
+            __threadfence();
+            float v[16];
+            add_parts(tile0, 0xffffffffu, v);
+            store(tile0, v);
         }
     }
     tc_fence_before_sync();
