@@ -24,8 +24,9 @@
 // The softmax of a CTA's keys needs the maximum over its eight warps (one exchange), the CTAs of the cluster meet once at the end
 // through distributed shared memory, each finishing its share of the rows.  No scratch, no counters.
 //
-// Bound by latency: 64 rows at 964 positions of 1024 take 25.3 us (233 before; 22.7 with one long chain of sums and a table row of any distance), of
-// which the matrix products are 5; 2 are the query preparation, 3 the softmax's exchanges, 4 the meeting of the cluster.  Two CTAs per SM hide some of it behind each other.
+// Bound by latency.  Between the launches of a 7B session (32 heads, 64 rows, 1024 positions) a launch takes 20 to 24 us, 38 where a CTA has a second chunk
+// of keys: 5 to the queries in fragments, 7 for the scores, 2.5 softmax, 3 values, 4 the meeting of the cluster.  It took 40 to 48: of 32 clusters of 8 CTAs two ran
+// after the others (see launch_attention_prompt), the queries took 7 (unrolled code, rows of the table from HBM).  Two CTAs per SM hide some of it behind each other.
 #include <math.h>
 
 #include <algorithm>
@@ -70,6 +71,10 @@ __device__ __forceinline__ uint32_t ap_finite(uint32_t w) {
     if ((w & 0x7c00u) == 0x7c00u) w &= 0xffff0000u;
     if ((w & 0x7c000000u) == 0x7c000000u) w &= 0x0000ffffu;
     return w;
+}
+
+__device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {        // multiples of 16 bytes
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
 // (cos, sin) of two pairs at the distance d (sin turns its sign with it), from the table
@@ -119,6 +124,17 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
         s_m[threadIdx.x] = -INFINITY;
         s_l[threadIdx.x] = 0.f;
     }
+    const uint32_t c_max = (max_ctx - 1) >> 5;
+    {
+        // Table rows, keys and values are in HBM more often than not (a layer's weights pass through L2 between two of its steps): what this CTA will
+        // read is on its way to L2 before the previous kernel has ended.  A hint: the position may be that of an earlier step.
+        const uint32_t guess = min(__ldcg(pos), max_ctx - 1) + z0, p0 = rank * kApKeys, i = threadIdx.x & (kApKeys - 1);
+        if (p0 + i <= guess && p0 + i < max_ctx) l2_prefetch((threadIdx.x < kApKeys ? kc : vc) + size_t(p0 + i) * dim + h * kApHead, kApHead * sizeof(__half));
+        if (threadIdx.x == 0) l2_prefetch(table, min(17u, max_ctx) * kApHead * 4);
+        const uint32_t c0 = guess >> 5, c = (p0 + 16 * warp + 16) >> 5;
+        if (lane == 0) l2_prefetch(table + size_t(32 * min(c0 > c ? c0 - c : c - c0, c_max)) * kApHead, kApHead * 4);
+        if (lane == 1 && warp < 3) l2_prefetch(table + size_t(32 * min(uint32_t(warp), c_max)) * kApHead, kApHead * 4);
+    }
     __syncthreads();
     pdl_wait();
     const uint32_t P = *pos + z0;                                   // position of this tile's first row
@@ -142,7 +158,7 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
     // Angles: position 32 c + d, |d| <= 16 where the table has the rows, is turned from 32 c0 by the table rows of 32 (c - c0) and of d, queries forwards
     // and keys backwards.  (The table's angles are rounded products of distance and frequency: rows of few distances, mostly small or powers
     // of two times 32, keep that error below that of a row of any distance.)
-    const uint32_t c0 = P >> 5, c_max = (max_ctx - 1) >> 5;
+    const uint32_t c0 = P >> 5;
     float4 far[4];                                                  // of this warp's 32 positions, four steps ahead
     auto load_far = [&](uint32_t p0, uint32_t ks, int i) {
         far[i] = ap_table_row(table, int(32 * c0) - int(32 * min((p0 + 16 * warp + 16) >> 5, c_max)), ap_first_dim(ks, t));
@@ -155,9 +171,10 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
     if (rank < n_chunks) {
         load_rows(rank * kApKeys);
         // ---- queries: turned by their row, scaled by a power of two so that the largest value of a row is in [1024, 2048) --------
-        constexpr int kRows = 4;                                    // rows of a warp at a time, all loads before the first use
-        for (uint32_t r0 = warp; r0 < 16 * n_mt; r0 += kRows * kApWarps) {
-            float4 x[kRows], near[kRows], far[kRows];
+        // Two rows of a warp at a time, the next two on their way: all rows at once are unrolled code that runs once (6 us, most of it instruction fetches).
+        constexpr int kRows = 2;
+        float4 x[kRows], near[kRows], far[kRows];
+        auto fetch = [&](uint32_t r0) {
 #pragma unroll
             for (int i = 0; i < kRows; ++i) {
                 const uint32_t r = r0 + i * kApWarps;
@@ -168,19 +185,27 @@ __global__ void __launch_bounds__(kApThreads, 2) attention_prompt_kernel(float* 
                 near[i] = ap_table_row(table, int(P + r) - int(32 * c), 4 * lane);
                 far[i] = ap_table_row(table, int(32 * (c - c0)), 4 * lane);
             }
+        };
+        fetch(warp);
+#pragma unroll 1
+        for (uint32_t r0 = warp; r0 < 16 * n_mt; r0 += kRows * kApWarps) {
+            float4 v[kRows];
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) {
+                const float4 w = ap_add_angles(far[i], near[i]);
+                v[i] = make_float4(w.x * x[i].x - w.y * x[i].y, w.y * x[i].x + w.x * x[i].y, w.z * x[i].z - w.w * x[i].w, w.w * x[i].z + w.z * x[i].w);
+            }
+            fetch(r0 + kRows * kApWarps);
 #pragma unroll
             for (int i = 0; i < kRows; ++i) {
                 const uint32_t r = r0 + i * kApWarps;
-                if (r >= 16 * n_mt) break;
-                const float4 w = ap_add_angles(far[i], near[i]);
-                const float4 v = make_float4(w.x * x[i].x - w.y * x[i].y, w.y * x[i].x + w.x * x[i].y, w.z * x[i].z - w.w * x[i].w, w.w * x[i].z + w.z * x[i].w);
-                const float top = warp_max(fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+                const float top = warp_max(fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
                 const uint32_t e = max(__float_as_uint(top) >> 23, 11u);
                 const float up = __uint_as_float((264u - e) << 23), down = __uint_as_float((e - 10u) << 23);      // 2^(137 - e), 2^(e - 137)
                 if (lane == 0) s_qf[r] = down * scale * kApLog2e;
                 uint32_t hi0, lo0, hi1, lo1;
-                ap_split(v.x * up, v.y * up, hi0, lo0);
-                ap_split(v.z * up, v.w * up, hi1, lo1);
+                ap_split(v[i].x * up, v[i].y * up, hi0, lo0);
+                ap_split(v[i].z * up, v[i].w * up, hi1, lo1);
                 // ap_first_dim(ks, t4) == 4 lane; rows 8 .. 15 of a tile are words 1 and 3 of a fragment
                 const uint32_t ks = 4 * (lane >> 4) + 2 * ((lane >> 1) & 1) + (lane & 1), t4 = (lane >> 2) & 3;
                 uint32_t* at = reinterpret_cast<uint32_t*>(s_q + (((r >> 4) * 8 + ks) * 32 + (r & 7) * 4 + t4) * 16) + ((r >> 3) & 1);
@@ -500,14 +525,39 @@ int attention_prompt_configure(lv_ctx* ctx) {
     LV_REQUIRE(size_t(ctx->max_smem_optin) >= kApSmemBytes + 1024, "device has too little shared memory for the prompt attention kernel");
     LV_CUDA(cudaFuncSetAttribute(attention_prompt_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kApSmemBytes)));
     LV_CUDA(cudaFuncSetAttribute(attention_prompt_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kApSmemBytes)));
+    for (uint32_t c = 1; c <= kApMaxCluster; ++c) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(1, c);
+        cfg.blockDim = dim3(kApThreads);
+        cfg.dynamicSmemBytes = kApSmemBytes;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1;
+        attr[0].val.clusterDim.y = c;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        LV_CUDA(cudaOccupancyMaxActiveClusters(&n, attention_prompt_kernel<false>, &cfg));
+        ctx->ap_clusters[c] = uint32_t(n);
+    }
     return LV_OK;
 }
 
 int launch_attention_prompt(lv_ctx* ctx, float* out, const float* q, const void* k_cache, const void* v_cache, const uint32_t* pos,
                             const float* rope_table, uint32_t heads, uint32_t max_ctx, uint32_t batch, void* xh) {
-    const uint32_t chunks = (max_ctx + kApKeys - 1) / kApKeys, C = std::min(kApMaxCluster, chunks);
+    const uint32_t chunks = (max_ctx + kApKeys - 1) / kApKeys, tiles = (batch + kApQ - 1) / kApQ;
+    // Clusters so small that all of them run at a time, where that is possible: of 32 clusters of 8 two had to wait for the others to end (40 us where 24
+    // were needed), and in clusters of 7 only the last of 1024 positions take a second pass (10 us).  Next to other kernels a tenth fewer find room
+    // than the device holds on its own.
+    uint32_t C = std::min(kApMaxCluster, chunks);
+    for (uint32_t c = C; c >= 4; --c)
+        if (10 * heads * tiles <= 9 * ctx->ap_clusters[c]) {
+            C = c;
+            break;
+        }
     auto* kernel = chunks <= C ? attention_prompt_kernel<true> : attention_prompt_kernel<false>;
-    LV_CUDA(launch_pdl_cluster(ctx, kernel, dim3(heads, C, (batch + kApQ - 1) / kApQ), dim3(kApThreads), dim3(1, C), kApSmemBytes, out, q,
+    LV_CUDA(launch_pdl_cluster(ctx, kernel, dim3(heads, C, tiles), dim3(kApThreads), dim3(1, C), kApSmemBytes, out, q,
                                static_cast<const __half*>(k_cache), static_cast<const __half*>(v_cache), pos, rope_table, heads, batch, max_ctx,
                                1.0f / sqrtf(float(kApHead)), ctx->d_err, static_cast<__half*>(xh), (batch + 15u) & ~15u));
     return LV_OK;

@@ -24,6 +24,7 @@ struct lv_ctx {
     bool peer_ready = false;
     void* tc_scratch = nullptr;       // partial accumulators of the K-split tensor-core products
     void* tc_counters = nullptr;
+    uint32_t ap_clusters[9] = {};     // clusters of 1 .. 8 CTAs that the device holds at a time (attention_prompt.cu)
     uint32_t bg_clusters[9] = {};     // clusters of 2 .. 8 CTAs that the device holds at a time (gemm_bf16.cu)
     bool tc_exact = false;            // batched q4_0 products with the exact hi/lo weight planes instead of one fp16 plane
     // exchange roles that lv_tp_arm_push / lv_tp_arm_pull set for the next GEMV-family launch

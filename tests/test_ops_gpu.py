@@ -438,7 +438,7 @@ def test_prompt_attention_of_small_and_large_keys(gpu, pkg, rope_table, batch, p
         gpu.free(d)
 
 
-@pytest.mark.parametrize("batch,pos,max_ctx", [(64, 0, 128), (50, 100, 256), (64, 448, 512), (70, 90, 256)])
+@pytest.mark.parametrize("batch,pos,max_ctx", [(64, 0, 128), (50, 100, 256), (64, 448, 512), (70, 90, 256), (64, 960, 1024)])
 def test_prompt_attention_rows_do_not_depend_on_later_values(gpu, pkg, rope_table, batch, pos, max_ctx):
     """Values of the cache that are not finite (the append rounds to f16) reach the rows that see them, and no row before: against the same
     caches with 0 in their place every other output has the same bits."""
