@@ -20,8 +20,9 @@ namespace lv {
 
 constexpr int kAttnThreads = 256;  // the three separate ops
 constexpr int kFusedThreads = 512;  // 128 registers per thread: room to keep every load of a step in flight
-constexpr int kAttnChunk = 256;    // cache rows per CTA of the fused kernel (16 per warp)
-constexpr int kScoreIters = kAttnChunk / (kFusedThreads / 32) / 4;   // row batches per warp: four rows at a time, 8 lanes each
+constexpr int kAttnChunk = 256;    // cache rows per CTA of the fused kernel
+constexpr int kScoreRows = kFusedThreads / 8;                    // rows of a pass of the scores, four per warp, 8 lanes each
+constexpr int kScoreIters = kAttnChunk / kScoreRows;
 constexpr int kValueRows = kAttnChunk / (kFusedThreads / 16);        // rows per thread in the value pass
 constexpr int kRowGroups = kFusedThreads / 16;   // 16 threads x 8 dims cover a row of one head
 constexpr int kRot = 128;        // head size; the reference supports only 128 (dim 4096/5120)
@@ -137,8 +138,8 @@ __host__ __device__ inline size_t attn_partial_floats(uint32_t heads, uint32_t n
 // step): scores with 8 lanes per cache row (16 elements each, both of a warp's
 // row batches in flight together), values with 16 threads per row (8 dims each)
 // and four rows per thread in flight.
-// Shared-memory staging of the score inputs: the chunk's key rows and the rows of the rotation table
-// it needs are brought in by bulk (TMA) copies and the scores are computed from shared memory.  With
+// Shared-memory staging of the score inputs: the rows of the rotation table that the chunk needs are brought in by bulk (TMA)
+// copies, its key rows 16 bytes per thread, and the scores are computed from shared memory.  With
 // plain loads the kernel spent a fifth of its samples throttled on the load/store queue (28 16-byte
 // loads per thread).
 //   STAGED = 2 (grids of at most one CTA per SM): the table rows of the chunk's distances, one
@@ -149,6 +150,8 @@ __host__ __device__ inline size_t attn_partial_floats(uint32_t heads, uint32_t n
 //     cos/sin((32 A + B) theta) from the angle-addition formulas (exact for A = 0, else a few units
 //     in the last place beside the table's own rounding); key rows unpadded.
 //   STAGED = 0: plain loads.
+// us per launch in a step, key rows by bulk copies and all passes of 256 rows -> this: 50 members of 32 heads at 120 positions 45 -> 32, 16 members at 200
+// 19.8 -> 17.0, one row at 1100 positions 14.3 -> 13.4; 40 heads at 210 positions (STAGED = 2) 6.3 -> 6.0.
 constexpr int kStagedKeyStride = 320;
 constexpr size_t kStagedTableBytes = size_t(kAttnChunk) * kRot * sizeof(float);              // 131072
 constexpr size_t kStagedSmemBytes = kStagedTableBytes + size_t(kAttnChunk) * kStagedKeyStride;  // + 81920
@@ -201,13 +204,16 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
     auto load_values = [&]() {
 #pragma unroll
         for (int j = 0; j < kValueRows; ++j) {
+            if (STAGED != 2 && uint32_t(kRowGroups * j) >= n) break;
             const uint32_t i = min(uint32_t(rg + kRowGroups * j), n - 1);
             vraw[j] = *reinterpret_cast<const uint4*>(vc + size_t(p0 + i) * dim + h * kRot + d8);
         }
     };
     if constexpr (STAGED == 2) load_values();
 
-    // ---- scores: warp w owns rows 16w .. 16w+15, lane group g = lane / 8 one row per pass -----
+    // ---- scores: warp w has rows 4w .. 4w+3 of every 64, lane group g = lane / 8 one of them; passes beyond the last row are left out where many
+    // CTAs share an SM (not with one CTA per SM: there the four passes overlap, and branches between them cost 0.6 us at 200 positions) -----
+    if (threadIdx.x >= n && threadIdx.x < kAttnChunk) s_e[threadIdx.x] = -INFINITY;
     if constexpr (STAGED != 0) {
         const int sub = lane & 7, g = lane >> 3;
         constexpr bool kCompact = STAGED == 1;
@@ -221,12 +227,15 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
             mbar_init(&s_bar, 1);
             fence_mbar_init();
             const uint32_t table_bytes = kCompact ? (32u + a_count) * kRot * uint32_t(sizeof(float)) : n * kRot * uint32_t(sizeof(float));
-            mbar_expect_tx(&s_bar, n * kRot * uint32_t(sizeof(__half)) + table_bytes);
+            mbar_expect_tx(&s_bar, table_bytes);
         }
+        // key row p0 + t -> ktile row t, 16 bytes per thread (a bulk copy per row keeps the copy unit busy for 13 clocks or more per row, 1.7 us at 256 rows)
+        for (uint32_t c = threadIdx.x; c < 16 * n; c += kFusedThreads)
+            cp_async16(ktile + (c >> 4) * kKeyStride + (c & 15u) * 16, kc + size_t(p0 + (c >> 4)) * dim + h * kRot + (c & 15u) * 8);
         __syncthreads();
-        // key row p0 + t -> ktile row t
-        if (threadIdx.x < n)
-            bulk_g2s(ktile + threadIdx.x * kKeyStride, kc + size_t(p0 + threadIdx.x) * dim + h * kRot, kRot * sizeof(__half), &s_bar);
+        // values that are fetched after the scores are on their way from HBM meanwhile
+        if (kCompact && threadIdx.x >= 256 && threadIdx.x - 256 < n)
+            l2_prefetch(vc + size_t(p0 + threadIdx.x - 256) * dim + h * kRot, kRot * sizeof(__half));
         if constexpr (kCompact) {
             // table rows 0..31 -> ttile rows 0..31; rows 32 (a_first + t) -> ttile row 32 + t
             if (threadIdx.x == 0) bulk_g2s(ttile, table, 32 * kRot * sizeof(float), &s_bar);
@@ -240,10 +249,13 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
         float4 qv[4];
 #pragma unroll
         for (int m = 0; m < 4; ++m) qv[m] = *reinterpret_cast<const float4*>(q + size_t(z) * dim + h * kRot + (sub + 8 * m) * 4);
+        asm volatile("cp.async.wait_all;" ::: "memory");
         const bool ok = mbar_wait(&s_bar, 0u, err);
+        __syncthreads();                                              // every thread's part of the keys is there
 #pragma unroll
         for (int it = 0; it < kScoreIters; ++it) {
-            const uint32_t i = warp * (4 * kScoreIters) + it * 4 + g;
+            if (kCompact && uint32_t(it * kScoreRows + 4 * warp) >= n) break;
+            const uint32_t i = it * kScoreRows + 4 * warp + g;
             const uint32_t ic = min(i, n - 1);                        // rows past n are computed and discarded
             const uint8_t* krow = ktile + ic * kKeyStride;
             const uint32_t d = d_min + (n - 1 - ic);
@@ -274,7 +286,7 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
             sacc += __shfl_xor_sync(0xffffffffu, sacc, 4);
             sacc += __shfl_xor_sync(0xffffffffu, sacc, 2);
             sacc += __shfl_xor_sync(0xffffffffu, sacc, 1);
-            if (sub == 0) s_e[i] = (i < n && ok) ? sacc * scale : -INFINITY;
+            if (sub == 0 && i < n) s_e[i] = ok ? sacc * scale : -INFINITY;
         }
     } else {
         const int sub = lane & 7, g = lane >> 3;
@@ -286,7 +298,8 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
         float4 cs[kScoreIters][4];
 #pragma unroll
         for (int it = 0; it < kScoreIters; ++it) {
-            const uint32_t i = warp * (4 * kScoreIters) + it * 4 + g;
+            if (uint32_t(it * kScoreRows + 4 * warp) >= n) break;
+            const uint32_t i = it * kScoreRows + 4 * warp + g;
             const uint32_t p = p0 + min(i, n - 1);                 // clamped: rows past n are computed and discarded
             const __half* krow = kc + size_t(p) * dim + h * kRot + sub * 16;
             kraw[it][0] = *reinterpret_cast<const uint4*>(krow);
@@ -297,7 +310,8 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
         }
 #pragma unroll
         for (int it = 0; it < kScoreIters; ++it) {
-            const uint32_t i = warp * (4 * kScoreIters) + it * 4 + g;
+            if (uint32_t(it * kScoreRows + 4 * warp) >= n) break;
+            const uint32_t i = it * kScoreRows + 4 * warp + g;
             const __half2* k2 = reinterpret_cast<const __half2*>(&kraw[it][0]);      // 8 (even, odd) pairs
             float sacc = 0.f;
 #pragma unroll
@@ -313,7 +327,7 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
             sacc += __shfl_xor_sync(0xffffffffu, sacc, 4);
             sacc += __shfl_xor_sync(0xffffffffu, sacc, 2);
             sacc += __shfl_xor_sync(0xffffffffu, sacc, 1);
-            if (sub == 0) s_e[i] = i < n ? sacc * scale : -INFINITY;
+            if (sub == 0 && i < n) s_e[i] = sacc * scale;
         }
     }
     // ---- weighted values: thread = (8 dims, one of 32 row groups), rows rg, rg+32, ... -----------
@@ -328,6 +342,7 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
     float lsum = 0.f;
 #pragma unroll
     for (int j = 0; j < kValueRows; ++j) {
+        if (STAGED != 2 && uint32_t(kRowGroups * j) >= n) break;
         const uint32_t i = rg + kRowGroups * j;
         const float e = i < n ? expf(s_e[i] - m) : 0.f;
         lsum += e;

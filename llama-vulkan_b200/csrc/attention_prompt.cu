@@ -73,10 +73,6 @@ __device__ __forceinline__ uint32_t ap_finite(uint32_t w) {
     return w;
 }
 
-__device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {        // multiples of 16 bytes
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
 // (cos, sin) of two pairs at the distance d (sin turns its sign with it), from the table
 __device__ __forceinline__ float4 ap_table_row(const float* table, int d, uint32_t dim) {
     float4 w = *reinterpret_cast<const float4*>(table + size_t(abs(d)) * kApHead + dim);

@@ -120,6 +120,16 @@ __device__ __forceinline__ void bulk_g2s_stream(void* smem_dst, const void* gsrc
         : "memory");
 }
 
+// 16 bytes global -> shared by this thread (cp.async.wait_all, then a barrier for the others to see them).
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
+}
+
+// A hint: brings global bytes to L2 (16-byte aligned, a multiple of 16).
+__device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // 2-D tiled TMA load: one instruction fetches a box of rows x bytes described by a tensor
 // map (tile coordinates x = inner element index, y = row) and counts the box on `bar`.
 // The inner coordinate times the element size must be a multiple of 16 bytes.
