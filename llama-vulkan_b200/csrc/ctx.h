@@ -15,6 +15,7 @@ struct lv_ctx {
     cudaStream_t stream = nullptr;
     uint32_t* d_err = nullptr;        // device error word, see lv::ERR_* in common.cuh
     uint32_t* h_err = nullptr;        // pinned mirror used by lv_ctx_check
+    void* h_bounce = nullptr;         // pinned, kBounceBytes: lv_download's way to ordinary memory (used under api_mutex)
     cudaGraph_t capture_graph = nullptr;
     bool capturing = false;
     std::recursive_mutex api_mutex;   // see LV_ENTER
@@ -36,6 +37,8 @@ struct lv_ctx {
 };
 
 namespace lv {
+
+constexpr size_t kBounceBytes = 256 * 1024;
 
 // Records a message retrievable through lv_last_error_string (thread local).
 int fail(int code, const std::string& msg);

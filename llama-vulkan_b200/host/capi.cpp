@@ -259,10 +259,7 @@ int llava_session_collect_greedy_on_device(void* s, uint32_t* out, uint32_t cap)
 }
 
 int llava_session_get_logits(void* s, float* out, uint32_t cap) {
-    std::vector<float> v;
-    if (!S(s)->get_logits(&v) || v.size() > cap) return 0;
-    std::memcpy(out, v.data(), v.size() * sizeof(float));
-    return 1;
+    return S(s)->read_logits(out, cap) ? 1 : 0;
 }
 
 uint32_t llava_session_get_backlog_size(void* s) { return S(s)->get_backlog_size(); }
@@ -383,10 +380,7 @@ int llava_session_group_generate_greedy_on_device(void* group, uint32_t n, uint3
     return 1;
 }
 int llava_session_group_get_logits(void* group, uint32_t member, float* out, uint32_t n) {
-    std::vector<float> v;
-    if (!static_cast<llava_session_group*>(group)->get_logits(member, &v) || v.size() != n) return 0;
-    std::memcpy(out, v.data(), size_t(n) * sizeof(float));
-    return 1;
+    return static_cast<llava_session_group*>(group)->read_logits(member, out, n) ? 1 : 0;
 }
 uint32_t llava_session_group_kernel_launches(void* group) { return static_cast<llava_session_group*>(group)->kernel_launches(); }
 

@@ -342,7 +342,13 @@ u32 llava_session::step_kernel_launches() const {
 bool llava_session::get_logits(vector<float>* out) {
     if (output_probs == nullptr) return false;
     out->resize(model->get_header().vocab_size);
-    return output_probs->read_raw(0, out->data(), out->size() * sizeof(float));
+    return read_logits(out->data(), u32(out->size()));
+}
+
+bool llava_session::read_logits(float* out, u32 room) {
+    if (output_probs == nullptr) return false;
+    const u32 vocab = model->get_header().vocab_size;
+    return vocab <= room && output_probs->read_raw(0, out, size_t(vocab) * sizeof(float));
 }
 
 u32 llava_session::get_last_predicted_token(bool want_deterministic) {

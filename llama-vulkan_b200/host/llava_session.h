@@ -82,6 +82,7 @@ public:
     bool evaluate_pending(const std::vector<u32>& wanted, std::vector<float>* logits);
     // logits of the last evaluated token (vocab floats)
     bool get_logits(std::vector<float>* out);
+    bool read_logits(float* out, u32 room);                    // the same into the caller's memory, room floats of it
     u32 get_backlog_size() const { return backlog_size; }
     u32 get_tokens_in_gpu() const { return current_tokens_in_gpu; }
     // timeline of the one-launch token step (lv_step_plan_set_trace); false when the session has no such step

@@ -292,7 +292,12 @@ bool llava_session_group::generate_greedy_on_device(u32 n, vector<vector<u32>>* 
 
 bool llava_session_group::get_logits(u32 member, vector<float>* out) {
     if (!valid || member >= size()) return false;
+    out->resize(ctx->get_model()->get_header().vocab_size);
+    return read_logits(member, out->data(), u32(out->size()));
+}
+
+bool llava_session_group::read_logits(u32 member, float* out, u32 n) {
+    if (!valid || member >= size()) return false;
     const u32 vocab = ctx->get_model()->get_header().vocab_size;
-    out->resize(vocab);
-    return logits->read_raw(size_t(member) * vocab * sizeof(float), out->data(), size_t(vocab) * sizeof(float));
+    return n == vocab && logits->read_raw(size_t(member) * vocab * sizeof(float), out, size_t(vocab) * sizeof(float));
 }

@@ -52,6 +52,7 @@ public:
     const std::vector<llava_session*>& get_members() const { return members; }
     // logits of member i from the last step (vocab floats)
     bool get_logits(u32 member, std::vector<float>* out);
+    bool read_logits(u32 member, float* out, u32 n);          // n: the vocabulary's size
     u32 kernel_launches() const { return launches; }
 
 private:

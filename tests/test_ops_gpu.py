@@ -73,6 +73,15 @@ def test_norm(gpu, pkg, dim, batch):
         close(got[z], ob.norm(x[z], w), rel_l2=2e-6, max_abs_frac=2e-6)
 
 
+@pytest.mark.parametrize("nbytes", [1, 4099, 128000, 256 * 1024, 256 * 1024 + 1, 1 << 20])
+def test_download_through_either_way(gpu, pkg, nbytes):
+    data = np.random.default_rng(nbytes).integers(0, 256, nbytes + 1, dtype=np.uint8)
+    d, got = gpu.upload(data), np.full(nbytes + 2, 7, np.uint8)
+    pkg.check(gpu.lib.lv_download(gpu.handle, C.c_void_p(got.ctypes.data + 1), pkg.offset(d, 1), nbytes))
+    assert np.array_equal(got[1:-1], data[1:]) and got[0] == 7 and got[-1] == 7
+    gpu.free(d)
+
+
 GEMV_SHAPES = [
     (qn.Q4_0, 4096, 4096), (qn.Q4_0, 4096, 11008), (qn.Q4_0, 5120, 13824), (qn.Q4_0, 5120, 5120),
     (qn.Q4_0, 32000, 4096), (qn.Q8_0, 4096, 4096), (qn.Q8_0, 4096, 11008), (qn.Q8_0, 1024, 5120),
