@@ -67,8 +67,10 @@ __device__ __forceinline__ void nc_store(const lv_norm_conv_args& a, uint32_t t,
 }
 
 // CTA b: token a.first + b.  A thread holds NV vectors of VEC channels.
-template <int VEC, int NV, typename OutT>
-__global__ void __launch_bounds__(1024) norm_rows_kernel(const NormConvParams p) {
+// HT > 0: one token with 1 .. HT taps.  Their weights are fetched before the previous kernel has ended and the state with the token's row, in registers:
+// fetched one tap after the other behind the sums they took 1.8 of the launch's 4.8 us (2048 channels, 4 taps).
+template <int VEC, int NV, typename OutT, int HT = 0>
+__global__ void __launch_bounds__(HT > 0 ? 512 : 1024) norm_rows_kernel(const NormConvParams p) {
     pdl_launch_dependents();
     const lv_norm_conv_args& a = p.a;
     __shared__ float scratch[64];
@@ -83,8 +85,29 @@ __global__ void __launch_bounds__(1024) norm_rows_kernel(const NormConvParams p)
             if (a.y != nullptr) post[k].load(a.post_w + i);
         }
     }
+    // taps and state right-aligned: the current token's tap is the last of HT, the state's newest entry the last of HT - 1
+    NcVec<VEC> tap[HT > 0 ? HT : 1][NV], old[HT > 1 ? HT - 1 : 1][NV];
+    const int tap0 = HT - int(a.taps);
+    if constexpr (HT > 0) {
+#pragma unroll
+        for (int j = 0; j < HT; ++j)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                const uint32_t i = (threadIdx.x + k * blockDim.x) * VEC;
+                if (j >= tap0 && i < W) tap[j][k].load(a.conv_w + size_t(j - tap0) * W + i);
+            }
+    }
     const float w0 = a.plain_w ? 0.f : 1.f;
     pdl_wait();
+    if constexpr (HT > 1) {
+#pragma unroll
+        for (int j = 0; j + 1 < HT; ++j)
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                const uint32_t i = (threadIdx.x + k * blockDim.x) * VEC;
+                if (j >= tap0 && i < W) old[j][k].load(a.history + size_t(j - tap0) * W + i);
+            }
+    }
     const uint32_t pos = *a.pos;
     NcVec<VEC> x[NV], y[NV];
     if (a.x == nullptr) {
@@ -209,7 +232,22 @@ __global__ void __launch_bounds__(1024) norm_rows_kernel(const NormConvParams p)
         NcVec<VEC> h, out;
 #pragma unroll
         for (int e = 0; e < VEC; ++e) out.v[e] = h.v[e] = x[k].v[e] * r * (w0 + pre[k].v[e]);
-        if (a.taps) {
+        if constexpr (HT > 0) {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) out.v[e] = fmaf(tap[HT - 1][k].v[e], h.v[e], out.v[e]);
+#pragma unroll
+            for (int j = 0; j + 1 < HT; ++j) {                      // as below
+                if (j < tap0) continue;
+                if (pos + uint32_t(j - tap0) < keep) {
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) old[j][k].v[e] = 0.f;
+                }
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) out.v[e] = fmaf(tap[j][k].v[e], old[j][k].v[e], out.v[e]);
+                if (j > tap0) old[j][k].store(a.history + size_t(j - tap0 - 1) * W + i);
+            }
+            if (keep) h.store(a.history + size_t(keep - 1) * W + i);
+        } else if (a.taps) {
             NcVec<VEC> w, old;
             w.load(a.conv_w + size_t(keep) * W + i);
 #pragma unroll
@@ -319,7 +357,10 @@ static int norm_conv_launch(lv_ctx* ctx, const lv_norm_conv_args& a) {
     if (vec && units >= 512 && nv == 1) nv = 2;           // fewer warps to sum over
     const uint32_t threads = ((units + nv - 1) / nv + 31) / 32 * 32;
     auto rows = [&](auto kernel) { return launch_pdl(ctx, kernel, dim3(count), dim3(threads), 0, p); };
-    if (!vec) LV_CUDA(rows(norm_rows_kernel<1, 16, OutT>));
+    const bool held = vec && a.batch == 1 && a.taps != 0 && a.taps <= 4 && threads <= 512;
+    if (held && nv == 1) LV_CUDA(rows(norm_rows_kernel<4, 1, OutT, 4>));
+    else if (held && nv == 2) LV_CUDA(rows(norm_rows_kernel<4, 2, OutT, 4>));
+    else if (!vec) LV_CUDA(rows(norm_rows_kernel<1, 16, OutT>));
     else if (nv == 1) LV_CUDA(rows(norm_rows_kernel<4, 1, OutT>));
     else if (nv == 2) LV_CUDA(rows(norm_rows_kernel<4, 2, OutT>));
     else LV_CUDA(rows(norm_rows_kernel<4, 4, OutT>));

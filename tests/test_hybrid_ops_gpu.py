@@ -221,7 +221,7 @@ def test_experts_chosen_by_token(gpu, width, ff, n, top, batch):
 
 # ---- norm, residual and convolution -----------------------------------------------------------
 
-@pytest.mark.parametrize("width,taps,cuts", [(64, 4, [1] * 9), (72, 4, [9]), (2056, 3, [2, 1, 5, 1]), (100, 6, [3, 2, 1, 1, 13]), (64, 1, [4, 1]),
+@pytest.mark.parametrize("width,taps,cuts", [(64, 4, [1] * 9), (72, 4, [9]), (2056, 3, [2, 1, 5, 1]), (4096, 4, [1, 1, 1, 3, 1]), (5000, 4, [1, 2, 1]), (100, 6, [3, 2, 1, 1, 13]), (64, 1, [4, 1]),
                                              (40, 9, [2, 2, 1, 20]), (64, 2, [7])])
 def test_norm_conv_in_portions(gpu, width, taps, cuts):
     rng = np.random.default_rng(width * taps)
