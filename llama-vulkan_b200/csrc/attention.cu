@@ -433,6 +433,8 @@ int attention_configure(lv_ctx* ctx) {
 //     12    12 / 9        28 / 14     48 / 15       4.9 / 8      11 / 11     17 / 12       4.8 / 8     8 / 11      11 / 11
 //     32    25 / 10       64 / 15    119 / 17       7.9 / 9      20 / 11     36 / 13       4.9 / 8    11 / 11      20 / 12
 //     64    47 / 14      123 / 23    233 / 25        15 / 13     36 / 16     63 / 18       8.1 / 13   20 / 16      36 / 16
+// (Taken with launches back to back, clusters of 8 and key rows by bulk copies.  Since then 64 rows of 32 heads at 1000 of 1024 take a second pass in clusters of 7:
+// 38 us between the launches of a session, where clusters of 8 took 44; the kernel here is 5 to 30 % faster, most with many CTAs.)
 // The kernel here runs up to two CTAs per SM at a time; below that it is as fast or faster, and exact in the angles (grids of one CTA per SM), so the line lies
 // where its CTAs are more than two per SM, three for steps of more than 32 rows, whose products take half as long again, and five where the products
 // take several passes (more than 1024 positions: 12 rows of 4 heads at 1100 of 2048 11 / 20, 16 rows of 8 heads 25 / 20).  (Measured at positions beyond
