@@ -102,6 +102,13 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, u
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
+// After a lost wait: lets what is on its way to the barrier arrive (bounded), whatever the error word says.
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+    const long long t0 = clock64();
+    while (!mbar_test(bar, parity))
+        if (clock64() - t0 > 20000000ll) break;
+}
+
 // 1-D bulk copy global -> shared, completion counted in bytes on `bar`.
 // Both addresses must be 16-byte aligned and `bytes` a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {

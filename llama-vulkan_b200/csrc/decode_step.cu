@@ -178,13 +178,6 @@ __device__ __forceinline__ bool ll_wait4(const uint64_t* __restrict__ buf, uint3
     return false;
 }
 
-// Lets the outstanding copies of a warp's ring land (bounded), whatever the error word says.
-__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
-    const long long t0 = clock64();
-    while (!mbar_test(bar, parity))
-        if (clock64() - t0 > 20000000ll) break;
-}
-
 // emit_block_record out of line: the step kernel calls it from a dozen places and its code size matters more than a call
 __device__ __noinline__ void emit_record(uint8_t* __restrict__ xrec, float4 v, uint32_t e, int lane) { emit_block_record(xrec, v, e, lane); }
 

@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
     constexpr uint32_t tmem_base = 0;                       // the allocation is all of the tensor memory
 
     bool ok = true;
+    uint32_t issued = 0;                                    // stages that a ring or issuing warp has asked for
 
     if (warp == kTsProducers) {
         // ---------------- raw ring: weights do not depend on the previous kernel ----------------
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
                 } else {
                     tma_load_2d_plain(dst, mi == 0 ? &maps.w[0] : (mi == 1 ? &maps.w[1] : &maps.w[2]), x, int(row0), &raw_full[rs]);
                 }
+                ++issued;
                 if (++rs == plan.n_raw) { rs = 0; phase ^= 1u; }
                 if (++g == G) { g = 0; mi = matrix_of(++tile, row0); }
             }
@@ -260,6 +262,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
                 const uint32_t j = i % kStages, t = kBT == 2 ? 2 * j : 2 * (j & 1u) + (j >> 1);       // first tile of the stage
                 mbar_expect_tx(&b_full[bs], b_stage);
                 bulk_g2s(bring + bs * b_stage, xh + size_t(4 * g + t) * b_tile, b_stage, &b_full[bs]);
+                ++issued;
                 if (++bs == plan.n_b) { bs = 0; phase ^= 1u; }
                 if (j + 1 == kStages && ++g == G) g = 0;
             }
@@ -297,6 +300,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
                     tc_commit(&b_empty[bs]);
                 }
                 __syncwarp();
+                ++issued;
                 bs += 2;
                 if (bs >= plan.n_b) { bs -= plan.n_b; b_phase ^= 1u; }
             }
@@ -525,7 +529,19 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
         }
     }
     tc_fence_before_sync();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) {
+        // a wait was lost: copies and products that are on their way end before shared and tensor memory are given back
+        auto drain_ring = [&](uint64_t* full, uint32_t n) {
+            for (uint32_t s = 0; s < min(issued, n); ++s) mbar_drain(&full[s], ((issued - 1 - s) / n) & 1u);
+        };
+        if (lane == 0 && warp == kTsProducers) drain_ring(raw_full, plan.n_raw);
+        else if (lane == 0 && warp == kTsProducers + 3) drain_ring(b_full, plan.n_b);
+        else if (lane == 0 && warp > kTsProducers && issued != 0) {
+            const uint32_t own = plan.n_b / 2, last = issued - 1;          // the last stage of this issuing lane's half of the ring
+            mbar_drain(&b_empty[2 * (last % own) + uint32_t(warp) - (kTsProducers + 1)], (last / own) & 1u);
+        }
+        __syncthreads();
+    }
     if (warp == kTsProducers + 1) {
         tc_fence_after_sync();
         tc_free(tmem_base, 512);
