@@ -109,6 +109,13 @@ __device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
         if (clock64() - t0 > 20000000ll) break;
 }
 
+// For a whole warp, every lane of which looks at the barrier itself: what it guards is ordered for all without a lane that tells the others.  Whether
+// the wait was lost is put to the vote, since each lane finds out on its own and what follows (elections, shuffles, tcgen05 .sync) needs the whole
+// warp: lanes that went on alone would wait for the others without a limit.
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, uint32_t* err) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err));
+}
+
 // 1-D bulk copy global -> shared, completion counted in bytes on `bar`.
 // Both addresses must be 16-byte aligned and `bytes` a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {

@@ -281,12 +281,12 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
         for (uint32_t i = 0; i < n_units && ok; ++i) {
             const uint32_t ab = i & 1u;
             // the accumulators of the previous segment have been read
-            if (first && seg > 0) ok = mbar_wait(acc_empty, (seg - 1) & 1u, p.err);
-            ok = ok && mbar_wait(&a_full[2 * ab + h], (i >> 1) & 1u, p.err);
+            if (first && seg > 0) ok = mbar_wait_all(acc_empty, (seg - 1) & 1u, p.err);
+            ok = ok && mbar_wait_all(&a_full[2 * ab + h], (i >> 1) & 1u, p.err);
             const uint32_t a_tmem = tmem_base + kTsABase + (4u * ab + 2u * h) * kTsTileCols;
 #pragma unroll
             for (uint32_t st = 0; st < 2 / kBT; ++st) {
-                ok = ok && mbar_wait(&b_full[bs], b_phase, p.err);
+                ok = ok && mbar_wait_all(&b_full[bs], b_phase, p.err);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint64_t b_desc = b_desc0 + ((bs * b_stage) >> 4);
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
         auto group_sync = [&]() {                                        // (a bounded wait: a warp may have given up elsewhere)
             __syncwarp();
             if (lane == 0) mbar_arrive(&group_bar[tt]);
-            ok = ok && mbar_wait(&group_bar[tt], met & 1u, p.err);
+            ok = ok && mbar_wait_all(&group_bar[tt], met & 1u, p.err);
             ++met;
             return ok;
         };
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
         // quarter warp's loads fall into different banks)
         uint32_t L[4 * ts_load_chunks<QT>()];
         auto fetch = [&]() {
-            ok = mbar_wait(&raw_full[rs], raw_phase, p.err);
+            ok = mbar_wait_all(&raw_full[rs], raw_phase, p.err);
             if (!ok) return;
             const uint4* src = reinterpret_cast<const uint4*>(rawring + rs * kRawStage + tr * kRawRowBytes) + (QT == T_Q4_0 ? 2u : 4u) * tt;
 #pragma unroll
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
             if (!ok) break;
             const uint32_t ab = i & 1u;
             if (i >= 2) {
-                ok = mbar_wait(&a_empty[2 * ab + half], ((i >> 1) - 1) & 1u, p.err);
+                ok = mbar_wait_all(&a_empty[2 * ab + half], ((i >> 1) - 1) & 1u, p.err);
                 if (!ok) break;
                 tc_fence_after_sync();
             }

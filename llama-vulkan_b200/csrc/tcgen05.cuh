@@ -53,14 +53,6 @@ __device__ __forceinline__ bool tc_elect() {
     return yes != 0;
 }
 
-// Waits like mbar_wait_warp, for a warp whose elected lane alone goes on to use what the barrier guards: that lane looks at the barrier itself, so the
-// others need no ordering behind it.
-__device__ __forceinline__ bool mbar_wait_elect(uint64_t* bar, uint32_t parity, uint32_t* err) {
-    bool ok = false;
-    if (tc_elect()) ok = mbar_wait(bar, parity, err);
-    return __any_sync(0xffffffffu, ok);
-}
-
 // mbar_wait_warp for a warp whose next step is tc_load16, an instruction of the whole warp that the fence in front of it orders: without the
 // ordering of ordinary loads by other lanes (0.1 us for each of the ends of a segment in gemm_tc_stream.cu).
 __device__ __forceinline__ bool mbar_wait_warp_tc(uint64_t* bar, uint32_t parity, uint32_t* err) {

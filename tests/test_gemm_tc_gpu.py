@@ -386,3 +386,25 @@ def test_act_split_takes_the_weights_of_the_launch_before(gpu, pkg, form):
     close(hi[:batch] + lo[:batch], want, rel_l2=1e-5, max_abs_frac=1e-5)
     for d in (out, row, ones, dx, xh):
         gpu.free(d)
+
+
+@pytest.mark.parametrize("wtype", [qn.Q4_0, qn.Q8_0], ids=["q4_0", "q8_0"])
+def test_gemm_tc_that_gives_up_returns(gpu, pkg, wtype, form):
+    """An index out of range sets the error word, behind which long waits are given up: those of a product whose activations wait for a long launch.  Its thread
+    blocks end without their rows, the synchronisation reports the error."""
+    if form == "exact":
+        pytest.skip("another kernel")
+    rows, cols, batch, lib, h = 23680, 1024, 40, gpu.lib, gpu.handle       # 148 runs of five units over tiles of four
+    rng = np.random.default_rng(70)
+    W = np.tile(matrix(rng, 32, cols, wtype=wtype).reshape(32, -1), (rows // 32, 1))
+    dW, xh = gpu.upload(W), split(gpu, pkg, rng.standard_normal((batch, cols)).astype(np.float32))
+    n = 1 << 23
+    long_row, norm, cache, word = gpu.zeros(n * 4), gpu.alloc(n * 4), gpu.zeros(64 * 2), gpu.upload(np.full(1, 8, np.uint32))
+    out = gpu.upload(np.full((batch, rows), np.nan, np.float32))
+    pkg.check(lib.lv_kv_append_f16(h, cache, long_row, word, 64, 1, 1))      # row 8 of a cache of one row
+    pkg.check(lib.lv_norm_f32(h, norm, long_row, long_row, n, 1))        # one thread block
+    pkg.check(lib.lv_gemm_tc(h, out, dW, wtype, xh, rows, cols, batch, 0))
+    assert lib.lv_stream_sync(h, 0) == pkg.LV_ERR_DEVICE_WAIT
+    assert np.isnan(gpu.download(out, np.float32, batch * rows)).any()       # (or nothing was given up)
+    for d in (dW, xh, long_row, norm, cache, word, out):
+        gpu.free(d)
