@@ -338,10 +338,14 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
             const uint32_t slot = shares != 0 || c * plan.per >= t * G ? 0u : 1u;
             return p.scratch + (size_t(2 * c + slot) * p.zpad + z0) * kTcRows + tr;
         };
-        auto arrive = [&](uint32_t t, uint32_t which) {                  // this warp's share of a part is in memory
-            __threadfence();
+        // This warp's share of a part is in memory.  One lane orders what the warp has stored before the addition and, where it is the last, the addition
+        // before the flag that sends the group to the other parts.
+        auto arrive = [&](uint32_t t, uint32_t which) {
             __syncwarp();
-            if (lane == 0 && atomicAdd(&p.counters[4 * t + tt], 1u) + 1 == 4 * (last_of(t) - first_of(t) + 1)) s_late[4 * which + tt] = 1;
+            if (lane == 0 && atom_add_release_gpu(&p.counters[4 * t + tt], 1u) + 1 == 4 * (last_of(t) - first_of(t) + 1)) {
+                __threadfence();
+                s_late[4 * which + tt] = 1;
+            }
         };
         // adds the parts of tile t in the order of K (`own` of them from v, none when it is no CTA) and leaves the counter ready for the next launch
         auto add_parts = [&](uint32_t t, uint32_t own, float (&v)[16]) {
@@ -440,7 +444,6 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
                     if (!final) return true;
                     arrive(tile, 1);
                     if (!group_sync() || s_late[4 + tt] == 0) return false;
-                    __threadfence();
                 }
                 add_parts(tile, blockIdx.x, v);
             }
@@ -522,7 +525,6 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
         if (ok && pending) drain(pend_seg, pend_tile, pend_whole, pend_slot, true);
         // the part of the first tile was the last one after all
         if (ok && active && group_sync() && s_late[tt] != 0) {
-            __threadfence();
             float v[16];
             add_parts(tile0, 0xffffffffu, v);
             store(tile0, v);

@@ -12,6 +12,7 @@ tight tolerances against the product with fp16-rounded weights -- the kernel doe
 pair): what the rounding of the weights costs.  Both forms exist for q4_0 and q8_0 matrices.
 """
 import ctypes as C
+import time
 
 import numpy as np
 import pytest
@@ -313,6 +314,83 @@ def test_gemm_tc_runs_of_units(gpu, pkg, rows, cols, batch, wtype, form):
 
 
 @pytest.mark.parametrize("wtype", [qn.Q4_0, qn.Q8_0], ids=["q4_0", "q8_0"])
+@pytest.mark.parametrize("kind,rows,cols,batch", [("plain", 14208, 1024, 64), ("plain", 23680, 1024, 33), ("plain", 19008, 512, 17), ("plain", 4096, 2816, 37), ("plain", 608, 4352, 64),
+                                                  ("silu", 11008, 4096, 16), ("silu", 1376, 4096, 64), ("group", 4096, 1024, 50), ("group", 2048, 1280, 1)])
+def test_gemm_tc_parts_in_any_order(gpu, pkg, kind, rows, cols, batch, wtype, form):
+    """Whoever reports the last part of a tile finishes it: mostly the thread block whose run ends there, the one whose run begins there when its launch came late.
+    Launches beside a norm of another context that keeps 0, 3, 63 or 139 SMs for some milliseconds, so that the last thread blocks begin when the others have ended, give the
+    same bits."""
+    if form == "exact":
+        pytest.skip("another kernel")
+    lib, h, rng = gpu.lib, gpu.handle, np.random.default_rng(rows + batch)
+    keep = []
+
+    def up(a):
+        keep.append(gpu.upload(a))
+        return keep[-1]
+
+    def zeros(nbytes):
+        keep.append(gpu.zeros(nbytes))
+        return keep[-1]
+
+    mats = [np.tile(matrix(rng, 32, cols, wtype=wtype).reshape(32, -1), (rows // 32, 1))[rng.permutation(rows)] for _ in range({"plain": 1, "silu": 2, "group": 3}[kind])]
+    x = rng.standard_normal((batch, cols)).astype(np.float32)
+    d, xh, out = [up(m) for m in mats], split(gpu, pkg, x), zeros(batch * rows * 4)
+    n = 1 << 20
+    wide, normed = zeros(n * 4 * 139), gpu.alloc(n * 4 * 139)
+    keep.append(normed)
+    ctx_rows = 64
+    if kind == "group":
+        at = rng.permutation(ctx_rows)[:batch].astype(np.uint32)
+        caches = zeros(2 * batch * ctx_rows * rows * 2)
+        members = np.zeros((batch, 4), np.uint64)
+        for z in range(batch):
+            members[z] = (caches.value + 2 * z * ctx_rows * rows * 2, caches.value + (2 * z + 1) * ctx_rows * rows * 2, up(np.full(4, at[z], np.uint32)).value, 0)
+        members = up(members)
+
+    def launch():
+        if kind == "plain":
+            pkg.check(lib.lv_gemm_tc(h, out, d[0], wtype, xh, rows, cols, batch, 0))
+        elif kind == "silu":
+            pkg.check(lib.lv_gemm_tc_silu(h, out, d[0], d[1], wtype, xh, rows, cols, batch))
+        else:
+            pkg.check(lib.lv_gemm_tc_qkv_kvappend_group(h, out, *d, wtype, xh, members, rows, cols, batch, ctx_rows))
+
+    def result():
+        got = [gpu.download(out, np.float32, batch * rows).reshape(batch, rows)]
+        if kind == "group":
+            for half in range(2):
+                got.append(np.stack([gpu.download(pkg.offset(caches, ((2 * z + half) * ctx_rows + int(at[z])) * rows * 2), np.float16, rows) for z in range(batch)]))
+        return got
+
+    launch()
+    gpu.sync()
+    first = result()
+    with pkg.Context(0) as other:
+        for late in (0, 3, 63, 139):
+            pkg.check(lib.lv_memset(h, out, 255, batch * rows * 4))
+            gpu.sync()
+            if late:
+                pkg.check(lib.lv_norm_f32(other.handle, normed, wide, wide, n, late))
+                time.sleep(1e-4)
+            for _ in range(4):
+                launch()
+            gpu.sync()
+            other.sync()
+            assert all(np.array_equal(a.view(np.uint8), b.view(np.uint8)) for a, b in zip(result(), first)), late
+    if kind == "silu":
+        up_rows, gate = (rounded_weights_product(m.reshape(-1), x, rows, cols, wtype) for m in mats)
+        close(first[0], up_rows * gate / (np.exp(-gate) + 1), rel_l2=2e-5, max_abs_frac=2e-5)
+    else:
+        want = [rounded_weights_product(m.reshape(-1), x, rows, cols, wtype) for m in mats]      # wq alone, or wq, wk, wv
+        close(first[0], want[0], rel_l2=1e-5, max_abs_frac=1e-5)
+        for got, w in zip(first[1:], want[1:]):
+            close(got, w, rel_l2=6e-4, max_abs_frac=1e-3)
+    for b in keep + [xh]:
+        gpu.free(b)
+
+
+@pytest.mark.parametrize("wtype", [qn.Q4_0, qn.Q8_0], ids=["q4_0", "q8_0"])
 @pytest.mark.parametrize("ff,dim,batch", [(64, 256, 1), (192, 512, 16), (11008, 4096, 37), (2048, 1024, 64)])
 def test_gemm_tc_silu_split_is_the_split_of_its_rows(gpu, pkg, ff, dim, batch, wtype, form):
     rng = np.random.default_rng(ff + batch)
@@ -391,7 +469,7 @@ def test_act_split_takes_the_weights_of_the_launch_before(gpu, pkg, form):
 @pytest.mark.parametrize("wtype", [qn.Q4_0, qn.Q8_0], ids=["q4_0", "q8_0"])
 def test_gemm_tc_that_gives_up_returns(gpu, pkg, wtype, form):
     """An index out of range sets the error word, behind which long waits are given up: those of a product whose activations wait for a long launch.  Its thread
-    blocks end without their rows, the synchronisation reports the error."""
+    blocks end without their rows, except for the one that found no SM before, and the synchronisation reports the error."""
     if form == "exact":
         pytest.skip("another kernel")
     rows, cols, batch, lib, h = 23680, 1024, 40, gpu.lib, gpu.handle       # 148 runs of five units over tiles of four
@@ -405,6 +483,7 @@ def test_gemm_tc_that_gives_up_returns(gpu, pkg, wtype, form):
     pkg.check(lib.lv_norm_f32(h, norm, long_row, long_row, n, 1))        # one thread block
     pkg.check(lib.lv_gemm_tc(h, out, dW, wtype, xh, rows, cols, batch, 0))
     assert lib.lv_stream_sync(h, 0) == pkg.LV_ERR_DEVICE_WAIT
-    assert np.isnan(gpu.download(out, np.float32, batch * rows)).any()       # (or nothing was given up)
+    written = ~np.isnan(gpu.download(out, np.float32, batch * rows))
+    assert written.any() and not written.all()                               # (or nothing was given up, or everything)
     for d in (dW, xh, long_row, norm, cache, word, out):
         gpu.free(d)
