@@ -260,6 +260,7 @@ extern "C" int lv_stream_sync(lv_ctx* ctx, int timeout_ms) {
     if (*ctx->h_err != 0) {
         const uint32_t word = *ctx->h_err;
         cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream);
+        gemm_tc_reset(ctx);
         return fail(LV_ERR_DEVICE_WAIT, "device error word " + std::to_string(word) +
                                             " (1 = copy wait lost, 2 = grid barrier lost, 4 = peer wait lost, 8 = index out of range)");
     }

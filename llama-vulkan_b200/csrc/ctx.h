@@ -50,6 +50,7 @@ int launch_attention_prompt(lv_ctx* ctx, float* out, const float* q, const void*
                             const float* rope_table, uint32_t heads, uint32_t max_ctx, uint32_t batch, void* xh = nullptr);      // attention_prompt.cu
 int gemm_tc_configure(lv_ctx* ctx);
 void gemm_tc_release(lv_ctx* ctx);
+void gemm_tc_reset(lv_ctx* ctx);       // after an error, on a drained stream
 int gemm_bf16_configure(lv_ctx* ctx);
 uint32_t* peer_step_counter(lv_ctx* ctx);
 bool peer_windows(lv_ctx* ctx, float** windows, int* n_ranks, int* rank, uint32_t* capacity);   // the connected peer windows, if any          // device word counting evaluation steps, or null without a peer window

@@ -714,10 +714,14 @@ void gemm_tc_release(lv_ctx* ctx) {
     ctx->tc_counters = nullptr;
 }
 
+// Thread blocks that give a wait up (behind any error that is not yet reported) leave without their arrivals, and the counters of their tiles would
+// stay where the others have brought them.
+void gemm_tc_reset(lv_ctx* ctx) { cudaMemsetAsync(ctx->tc_counters, 0, kTcCounterBytes, ctx->stream); }
+
 int gemm_tc_configure(lv_ctx* ctx) {
     LV_CUDA(cudaMalloc(&ctx->tc_scratch, kTcScratchBytes));
-    LV_CUDA(cudaMalloc(&ctx->tc_counters, 4 * kTcMaxTiles * sizeof(uint32_t)));
-    LV_CUDA(cudaMemset(ctx->tc_counters, 0, 4 * kTcMaxTiles * sizeof(uint32_t)));
+    LV_CUDA(cudaMalloc(&ctx->tc_counters, kTcCounterBytes));
+    LV_CUDA(cudaMemset(ctx->tc_counters, 0, kTcCounterBytes));
     LV_REQUIRE(size_t(ctx->max_smem_optin) >= tc_smem_bytes<T_Q4_0>() && size_t(ctx->max_smem_optin) >= tc_smem_bytes<T_Q8_0>(),
                "device has too little shared memory for the batched product");
     constexpr size_t kFastSmem = tc_smem_bytes<T_Q4_0, 1>();

@@ -23,6 +23,7 @@ template <int QT> __host__ __device__ constexpr int tc_raw_stage() { return kTcR
 
 constexpr size_t kTcScratchBytes = size_t(32) << 20;
 constexpr uint32_t kTcMaxTiles = 1024;
+constexpr size_t kTcCounterBytes = 4 * kTcMaxTiles * sizeof(uint32_t);
 
 struct GemmTcParams {
     GemvMatrix m[3];         // same meaning as in the GEMV; w_gate set = SiLU pair (64 + 64 rows per CTA)
@@ -35,7 +36,7 @@ struct GemmTcParams {
     const __half* xh;        // split activations, one contiguous pre-swizzled B tile per 64 columns of K (act_split_kernel)
     uint32_t splits;         // CTAs that share one tile of rows, each taking a contiguous range of K
     float* scratch;          // splits > 1: partial accumulators [tile][split][zpad][128]; gemm_tc_stream.cu: [CTA][first, last tile][zpad][128]
-    uint32_t* counters;      // arrivals per tile; gemm_tc_stream.cu: per tile and sixteen tokens (zero between launches)
+    uint32_t* counters;      // arrivals per tile; gemm_tc_stream.cu: per tile and sixteen tokens (zero between launches; after an error gemm_tc_reset sees to it)
     uint32_t* err;
     __half* split_out;       // SiLU pairs, gemm_tc_stream.cu: finished rows go there as the split activations of the next product, not to m[0].out
     const lv_group_member* group;   // non-null: token z is member z of a group step; cache rows go to its own caches at its own position

@@ -519,8 +519,8 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_tc_stream_kernel(const Gem
                 g = seg_begin = 0;
             }
         }
-        // (the warps of a CTA may disagree about `ok` only after a lost wait, whose error word ends every later wait; barriers below
-        // are reached by all of them)
+        // (After a lost wait, whose error word ends every later one, arrivals stay out and the warps of a CTA may disagree about `ok`: every wait of theirs for one
+        // another is bounded, and gemm_tc_reset takes the counters back to 0 when the error is reported.)
         if (ok && parked) arrive(tile0, 0);
         if (ok && pending) drain(pend_seg, pend_tile, pend_whole, pend_slot, true);
         // the part of the first tile was the last one after all
