@@ -276,6 +276,34 @@ def test_norm_conv_in_portions(gpu, width, taps, cuts):
             at += n
 
 
+@pytest.mark.parametrize("width,taps,batch", [(256, 4, 1), (256, 9, 1), (2048, 3, 1), (100, 2, 1), (256, 4, 5), (98, 6, 3)])
+@pytest.mark.parametrize("which", ["pre_w", "post_w", "conv_w"])
+def test_norm_conv_takes_the_weights_of_the_launch_before(gpu, which, width, taps, batch):
+    """The array is the end of a long row that one thread block normalises in the launch just before.  A normalised value carries a few units of 2^-24 and the long
+    row's factor 1e-6 or so."""
+    n, size = 1 << 22, width * (taps if which == "conv_w" else 1)
+    rng = np.random.default_rng(width + taps)
+    long_row = rng.standard_normal(n).astype(np.float32)
+    x, y = rng.standard_normal((2, batch, width)).astype(np.float32)
+    w = {"pre_w": rng.standard_normal(width), "post_w": rng.standard_normal(width), "conv_w": rng.standard_normal((taps, width))}
+    state = rng.standard_normal((taps - 1, width)).astype(np.float32)
+    with Dev(gpu) as d:
+        row, ones, normed = d.f32(long_row), d.f32(np.ones(n)), d.zeros(n * 4)
+        at = {k: d.f32(v).value for k, v in w.items()}
+        at[which] = pkg.offset(normed, (n - size) * 4).value
+        out = d.zeros(batch * width * 4)
+        a = pkg.NormConvArgs(x=d.f32(x).value, y=d.f32(y).value, pos=d.u32([50] * 4).value, y_rows=1, mult=0.5, eps=EPS, x_out=d.zeros(batch * width * 4).value,
+                             row_factor=d.zeros(batch * 4).value, history=d.f32(state).value, taps=taps, out=out.value, out_type=pkg.TYPE_F32, out_ld=width, width=width,
+                             batch=batch, **at)
+        pkg.check(gpu.lib.lv_norm_f32(gpu.handle, normed, row, ones, n, 1))
+        d.call("lv_norm_conv", C.byref(a))
+        w[which] = (long_row[n - size:] / long_row.astype(np.float64).std()).reshape(w[which].shape)
+        h = sp.norm_one_plus(x + 0.5 * sp.norm_one_plus(y.astype(np.float64), w["post_w"], EPS), w["pre_w"], EPS)
+        past = np.concatenate([state, h])
+        want = h + sum(w["conv_w"][j] * past[j:j + batch] for j in range(taps))
+        assert rel(d.get(out, (batch, width)), want) < 1e-5
+
+
 def test_norm_without_convolution_of_the_last_row(gpu):
     rng = np.random.default_rng(5)
     n, width = 6, 96
