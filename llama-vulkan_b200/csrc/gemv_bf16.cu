@@ -54,10 +54,10 @@ struct GbSettled {
 };
 
 // Partial dot products of NR rows with x over this lane's share of K.  WAIT: the rows are known before the previous kernel
-// has finished and their first 1024 elements are requested before waiting for it; ahead: and the next 2048 are on their way to L2.  settle: called after the wait; true: it has changed the rows
+// has finished and their first elements are requested before waiting for it.  settle: called after the wait; true: it has changed the rows
 // (which were only a guess) and their first elements are requested again.
 template <int NR, bool WAIT, typename Settle = GbSettled>
-__device__ __forceinline__ void gb_dot(float (&acc)[NR], const __nv_bfloat16* const (&row)[NR], const float* x, uint32_t K, bool ahead = false, Settle settle = Settle()) {
+__device__ __forceinline__ void gb_dot(float (&acc)[NR], const __nv_bfloat16* const (&row)[NR], const float* x, uint32_t K, Settle settle = Settle()) {
     const uint32_t lane8 = (threadIdx.x & 31u) * 8u;
     uint4 w[kGbUnroll][NR];
     auto fetch = [&](uint32_t k0) {
@@ -69,13 +69,7 @@ __device__ __forceinline__ void gb_dot(float (&acc)[NR], const __nv_bfloat16* co
         }
     };
     fetch(0);
-    if constexpr (WAIT) {
-        const uint32_t next = 256u * kGbUnroll + 8u * lane8;                     // a line of 64 elements per lane
-#pragma unroll
-        for (int r = 0; r < NR; ++r)
-            if (ahead && next < K) asm volatile("prefetch.global.L2 [%0];" ::"l"(row[r] + next));
-        pdl_wait();
-    }
+    if constexpr (WAIT) pdl_wait();
     if (settle()) fetch(0);
     for (uint32_t k0 = 0; k0 < K; k0 += 256u * kGbUnroll) {
 #pragma unroll
@@ -102,7 +96,6 @@ struct GemvBf16Params {
     uint32_t out_ld;
     float factor;
     int act;
-    bool ahead;
 };
 
 // SPLIT: warps that share two rows
@@ -115,11 +108,11 @@ __global__ void __launch_bounds__(kGbThreads) gemv_bf16_kernel(const GemvBf16Par
     if constexpr (SPLIT == 1) {
         if (u >= p.rows) return;
         const __nv_bfloat16* row[2] = {p.w[0] + size_t(u) * p.ld, p.w[0] + size_t(min(u + 1, p.rows - 1)) * p.ld};
-        gb_dot<2, true>(acc, row, p.x + size_t(blockIdx.y) * p.x_ld, p.K, p.ahead);
+        gb_dot<2, true>(acc, row, p.x + size_t(blockIdx.y) * p.x_ld, p.K);
     } else {
         const uint32_t per = (p.K + SPLIT * 256 - 1) / (SPLIT * 256) * 256, first = warp % SPLIT * per, count = u < p.rows && first < p.K ? min(per, p.K - first) : 0;
         const __nv_bfloat16* row[2] = {p.w[0] + size_t(min(u, p.rows - 1)) * p.ld + first, p.w[0] + size_t(min(u + 1, p.rows - 1)) * p.ld + first};
-        gb_dot<2, true>(acc, row, p.x + size_t(blockIdx.y) * p.x_ld + first, count, p.ahead);
+        gb_dot<2, true>(acc, row, p.x + size_t(blockIdx.y) * p.x_ld + first, count);
     }
     float a0 = warp_sum(acc[0]), a1 = warp_sum(acc[1]);
     if constexpr (SPLIT > 1) {
@@ -141,7 +134,7 @@ __global__ void __launch_bounds__(kGbThreads) gemv_bf16_mingru_kernel(const Gemv
     if (c >= p.rows) return;
     const __nv_bfloat16* row[3] = {p.w[0] + size_t(c) * p.ld, p.w[1] + size_t(c) * p.ld, p.w[2] + size_t(c) * p.ld};
     float acc[3] = {0.f, 0.f, 0.f};
-    gb_dot<3, true>(acc, row, p.x, p.K, p.ahead);
+    gb_dot<3, true>(acc, row, p.x, p.K);
     const float az = warp_sum(acc[0]), ax = warp_sum(acc[1]), ag = warp_sum(acc[2]);
     if ((threadIdx.x & 31u) == 0) p.out[c] = mingru_step(az + bz[c], ax + bx[c], ag, *pos == 0 ? 0.f : state[c], &state[c]);
 }
@@ -194,7 +187,7 @@ __global__ void __launch_bounds__(kGbThreads) gemv_bf16_expert_gate_up_kernel(co
     if (p.log_places != 0) {
         const uint32_t guess = gb_expert_guess(p, slot);
         rows_of(guess);
-        gb_dot<2, true>(acc, row, p.x, p.K, false, [&]() {
+        gb_dot<2, true>(acc, row, p.x, p.K, [&]() {
             const uint32_t e = gb_expert(p, 0, slot);
             if (e == guess) return false;
             rows_of(e);
@@ -229,7 +222,7 @@ __global__ void __launch_bounds__(kGbThreads) gemv_bf16_expert_down_kernel(const
     if (p.log_places != 0) {
         const uint32_t guess = gb_expert_guess(p, s);
         rows_of(guess);
-        gb_dot<2, true>(acc, row, x + size_t(s) * p.x_ld, p.K, false, [&]() {
+        gb_dot<2, true>(acc, row, x + size_t(s) * p.x_ld, p.K, [&]() {
             const uint32_t e = gb_expert(p, 0, s);
             if (e == guess) return false;
             rows_of(e);
@@ -255,12 +248,6 @@ __global__ void __launch_bounds__(kGbThreads) gemv_bf16_expert_down_kernel(const
     if (lane < 2 && r + lane < p.rows) p.out[size_t(t) * p.out_ld + r + lane] = (lane ? a1 : a0) / float(p.top);
 }
 
-// Whether a launch brings the second part of its rows to L2 while it waits.  Up to 24 MB it is bound by latency, often behind a norm that leaves HBM idle:
-// products of 2048 x 2048 and 3072 x 2048 3.97 -> 2.87 us.  Larger ones keep HBM busy anyway, and the prefetch takes it from what the previous launch waits
-// for: with it for all, a request of the state-space design 4096 wide (34 MB and more) took 14.3 ms, without 13.65, with this rule 13.5.  Nor for
-// experts (46 MB of gate and up 12.5 -> 11.7, but 23 MB of down 9.6 -> 10.5 and the norm before them 3.0 -> 3.5).
-static bool gb_ahead(uint64_t weights) { return weights * 2 <= (uint64_t(24) << 20); }
-
 static bool gb_aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 }  // namespace lv
@@ -277,7 +264,6 @@ extern "C" int lv_gemv_bf16(lv_ctx* ctx, float* out, uint32_t out_ld, const void
     p.w[0] = static_cast<const __nv_bfloat16*>(w);
     p.rows = rows;
     p.ld = ld; p.K = cols; p.x = x; p.x_ld = x_ld; p.out = out; p.out_ld = out_ld; p.factor = factor; p.act = act;
-    p.ahead = gb_ahead(uint64_t(rows) * ld);
     // three or more CTAs per SM, at least 512 columns per warp
     uint32_t split = 1;
     while (split < 8 && uint64_t(rows) * batch * split < uint64_t(48) * uint32_t(ctx->sm_count) && cols >= 512 * 2 * split) split *= 2;
@@ -298,7 +284,6 @@ extern "C" int lv_gemv_bf16_mingru(lv_ctx* ctx, float* out, const void* wz, cons
     p.w[2] = static_cast<const __nv_bfloat16*>(wg);
     p.rows = channels;
     p.ld = ld; p.K = cols; p.x = x; p.out = out;
-    p.ahead = gb_ahead(uint64_t(3) * channels * ld);
     LV_CUDA(launch_pdl(ctx, gemv_bf16_mingru_kernel, dim3((channels + kGbWarps - 1) / kGbWarps), dim3(kGbThreads), 0, p, bz, bx, state, pos));
     return LV_OK;
 }
