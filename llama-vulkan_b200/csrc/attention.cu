@@ -11,6 +11,7 @@
 #include <cstdlib>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -150,8 +151,9 @@ __host__ __device__ inline size_t attn_partial_floats(uint32_t heads, uint32_t n
 //     cos/sin((32 A + B) theta) from the angle-addition formulas (exact for A = 0, else a few units
 //     in the last place beside the table's own rounding); key rows unpadded.
 //   STAGED = 0: plain loads.
-// us per launch in a step, key rows by bulk copies and all passes of 256 rows -> this: 50 members of 32 heads at 120 positions 45 -> 32, 16 members at 200
-// 19.8 -> 17.0, one row at 1100 positions 14.3 -> 13.4; 40 heads at 210 positions (STAGED = 2) 6.3 -> 6.0.
+// us per launch behind a copy that passes through L2, 32 heads, key rows by bulk copies and all passes of 256 rows -> this: 50 members at 120 / 500 / 1000 positions
+// 47.4 / 124 / 231 -> 34.5 / 110 / 202, 16 members at 200 21.8 -> 20.5; rows of one sequence: 16 at 240 18.2 -> 17.4, one at 1100 / 1900 of 2048 13.0 / 14.8 ->
+// 11.8 / 14.5; one row of 40 heads at 210 positions in a step (STAGED = 2) 6.3 -> 6.0.
 constexpr int kStagedKeyStride = 320;
 constexpr size_t kStagedTableBytes = size_t(kAttnChunk) * kRot * sizeof(float);              // 131072
 constexpr size_t kStagedSmemBytes = kStagedTableBytes + size_t(kAttnChunk) * kStagedKeyStride;  // + 81920
@@ -212,7 +214,8 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
     if constexpr (STAGED == 2) load_values();
 
     // ---- scores: warp w has rows 4w .. 4w+3 of every 64, lane group g = lane / 8 one of them; passes beyond the last row are left out where many
-    // CTAs share an SM (not with one CTA per SM: there the four passes overlap, and branches between them cost 0.6 us at 200 positions) -----
+    // CTAs share an SM and the chunk is not full (without branches the four passes overlap: with them one CTA per SM took 0.6 us more at 200 positions, one row at
+    // 1900 of 2048 positions 15.3 us instead of 14.5, 50 rows 353 instead of 323) -----
     if (threadIdx.x >= n && threadIdx.x < kAttnChunk) s_e[threadIdx.x] = -INFINITY;
     if constexpr (STAGED != 0) {
         const int sub = lane & 7, g = lane >> 3;
@@ -233,8 +236,8 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
         for (uint32_t c = threadIdx.x; c < 16 * n; c += kFusedThreads)
             cp_async16(ktile + (c >> 4) * kKeyStride + (c & 15u) * 16, kc + size_t(p0 + (c >> 4)) * dim + h * kRot + (c & 15u) * 8);
         __syncthreads();
-        // values that are fetched after the scores are on their way from HBM meanwhile
-        if (kCompact && threadIdx.x >= 256 && threadIdx.x - 256 < n)
+        // values that are fetched after the scores are on their way from HBM meanwhile (rows that share the caches: asked for by the first)
+        if (kCompact && (group != nullptr || z == 0) && threadIdx.x >= 256 && threadIdx.x - 256 < n)
             l2_prefetch(vc + size_t(p0 + threadIdx.x - 256) * dim + h * kRot, kRot * sizeof(__half));
         if constexpr (kCompact) {
             // table rows 0..31 -> ttile rows 0..31; rows 32 (a_first + t) -> ttile row 32 + t
@@ -252,42 +255,46 @@ __global__ void __launch_bounds__(kFusedThreads, MIN_CTAS_PER_SM) attention_fuse
         asm volatile("cp.async.wait_all;" ::: "memory");
         const bool ok = mbar_wait(&s_bar, 0u, err);
         __syncthreads();                                              // every thread's part of the keys is there
+        auto scores = [&](auto all) {
 #pragma unroll
-        for (int it = 0; it < kScoreIters; ++it) {
-            if (kCompact && uint32_t(it * kScoreRows + 4 * warp) >= n) break;
-            const uint32_t i = it * kScoreRows + 4 * warp + g;
-            const uint32_t ic = min(i, n - 1);                        // rows past n are computed and discarded
-            const uint8_t* krow = ktile + ic * kKeyStride;
-            const uint32_t d = d_min + (n - 1 - ic);
-            const float* trow = kCompact ? ttile + size_t(d & 31u) * kRot : ttile + size_t(n - 1 - ic) * kRot;
-            const float* arow = ttile + size_t(32u + (d >> 5) - a_first) * kRot;          // compact only
-            float sacc = 0.f;
+            for (int it = 0; it < kScoreIters; ++it) {
+                if (!decltype(all)::value && uint32_t(it * kScoreRows + 4 * warp) >= n) break;
+                const uint32_t i = it * kScoreRows + 4 * warp + g;
+                const uint32_t ic = min(i, n - 1);                        // rows past n are computed and discarded
+                const uint8_t* krow = ktile + ic * kKeyStride;
+                const uint32_t d = d_min + (n - 1 - ic);
+                const float* trow = kCompact ? ttile + size_t(d & 31u) * kRot : ttile + size_t(n - 1 - ic) * kRot;
+                const float* arow = ttile + size_t(32u + (d >> 5) - a_first) * kRot;          // compact only
+                float sacc = 0.f;
 #pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int f = sub + 8 * m;
-                const uint2 kk = *reinterpret_cast<const uint2*>(krow + f * 8);           // 4 halves = 2 pairs
-                float4 t = *reinterpret_cast<const float4*>(trow + f * 4);                // (cos, sin) of the two pairs
-                if constexpr (kCompact) {
-                    // (cos, sin)((32 A + B) theta) from the rows of 32 A and of B
-                    const float4 a = *reinterpret_cast<const float4*>(arow + f * 4);
-                    const float c0 = fmaf(a.x, t.x, -(a.y * t.y)), s0 = fmaf(a.y, t.x, a.x * t.y);
-                    const float c1 = fmaf(a.z, t.z, -(a.w * t.w)), s1 = fmaf(a.w, t.z, a.z * t.w);
-                    t = make_float4(c0, s0, c1, s1);
+                for (int m = 0; m < 4; ++m) {
+                    const int f = sub + 8 * m;
+                    const uint2 kk = *reinterpret_cast<const uint2*>(krow + f * 8);           // 4 halves = 2 pairs
+                    float4 t = *reinterpret_cast<const float4*>(trow + f * 4);                // (cos, sin) of the two pairs
+                    if constexpr (kCompact) {
+                        // (cos, sin)((32 A + B) theta) from the rows of 32 A and of B
+                        const float4 a = *reinterpret_cast<const float4*>(arow + f * 4);
+                        const float c0 = fmaf(a.x, t.x, -(a.y * t.y)), s0 = fmaf(a.y, t.x, a.x * t.y);
+                        const float c1 = fmaf(a.z, t.z, -(a.w * t.w)), s1 = fmaf(a.w, t.z, a.z * t.w);
+                        t = make_float4(c0, s0, c1, s1);
+                    }
+                    const float2 ka = __half22float2(*reinterpret_cast<const __half2*>(&kk.x));
+                    const float2 kb = __half22float2(*reinterpret_cast<const __half2*>(&kk.y));
+                    const float4 qq = qv[m];
+                    // mhsa.comp:42-57
+                    const float rx0 = t.x * ka.x + t.y * ka.y, ry0 = -t.y * ka.x + t.x * ka.y;
+                    const float rx1 = t.z * kb.x + t.w * kb.y, ry1 = -t.w * kb.x + t.z * kb.y;
+                    sacc += qq.x * rx0 + qq.y * ry0;
+                    sacc += qq.z * rx1 + qq.w * ry1;
                 }
-                const float2 ka = __half22float2(*reinterpret_cast<const __half2*>(&kk.x));
-                const float2 kb = __half22float2(*reinterpret_cast<const __half2*>(&kk.y));
-                const float4 qq = qv[m];
-                // mhsa.comp:42-57
-                const float rx0 = t.x * ka.x + t.y * ka.y, ry0 = -t.y * ka.x + t.x * ka.y;
-                const float rx1 = t.z * kb.x + t.w * kb.y, ry1 = -t.w * kb.x + t.z * kb.y;
-                sacc += qq.x * rx0 + qq.y * ry0;
-                sacc += qq.z * rx1 + qq.w * ry1;
+                sacc += __shfl_xor_sync(0xffffffffu, sacc, 4);
+                sacc += __shfl_xor_sync(0xffffffffu, sacc, 2);
+                sacc += __shfl_xor_sync(0xffffffffu, sacc, 1);
+                if (sub == 0 && i < n) s_e[i] = ok ? sacc * scale : -INFINITY;
             }
-            sacc += __shfl_xor_sync(0xffffffffu, sacc, 4);
-            sacc += __shfl_xor_sync(0xffffffffu, sacc, 2);
-            sacc += __shfl_xor_sync(0xffffffffu, sacc, 1);
-            if (sub == 0 && i < n) s_e[i] = ok ? sacc * scale : -INFINITY;
-        }
+        };
+        if (!kCompact || n == uint32_t(kAttnChunk)) scores(std::true_type());
+        else scores(std::false_type());
     } else {
         const int sub = lane & 7, g = lane >> 3;
         const float* qh = q + size_t(z) * dim + h * kRot + sub * 16;
