@@ -543,9 +543,12 @@ int attention_prompt_configure(lv_ctx* ctx) {
 int launch_attention_prompt(lv_ctx* ctx, float* out, const float* q, const void* k_cache, const void* v_cache, const uint32_t* pos,
                             const float* rope_table, uint32_t heads, uint32_t max_ctx, uint32_t batch, void* xh) {
     const uint32_t chunks = (max_ctx + kApKeys - 1) / kApKeys, tiles = (batch + kApQ - 1) / kApQ;
-    // Clusters so small that all of them run at a time, where that is possible: of 32 clusters of 8 two had to wait for the others to end (40 us where 24
-    // were needed), and in clusters of 7 only the last of 1024 positions take a second pass (10 us).  Next to other kernels a tenth fewer find room
-    // than the device holds on its own.
+    // Clusters so small that all of them run at a time, where that is possible: between the launches of a session two of 32 clusters of 8 had to wait for the others
+    // to end (40 us where 24 were needed), and in clusters of 7 only the last of 1024 positions take a second pass (10 us).  Next to other kernels a tenth
+    // fewer find room than the device holds on its own (there 32 clusters of 8 do run at a time: 27 us at 960 positions, 40 in clusters of 7).
+    // ms of a prompt of six layers, clusters of 8 / 7 / 6 / 5 / 4: 32 heads, 1984 tokens in steps of 64 28.3 / 25.0 / 25.5 / 25.9 / 27.0; 40 heads, 1024 tokens 16.5 /
+    // 16.6 / 15.2 / 15.2 / 15.5, 1984 tokens 34.8 / 35.0 / 30.8 / 31.3 / 32.2; 16 heads, 1984 tokens 17.0 / 17.5 / 17.9 / 18.6 / 19.5.  A launch of 52 heads on its
+    // own, 64 rows at 960 of 1024 / 1900 of 2048 positions: 48.8 / 79.2 us in clusters of 8, 40.4 / 68.2 in clusters of 4.
     uint32_t C = std::min(kApMaxCluster, chunks);
     for (uint32_t c = C; c >= 4; --c)
         if (10 * heads * tiles <= 9 * ctx->ap_clusters[c]) {

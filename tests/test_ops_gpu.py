@@ -495,6 +495,28 @@ def test_attention_of_few_heads_keeps_the_exact_angles(gpu, pkg, rope_table, hea
         gpu.free(d)
 
 
+@pytest.mark.parametrize("heads", [24, 40, 44, 52, 60])
+@pytest.mark.parametrize("batch,pos,max_ctx", [(64, 960, 1024), (20, 700, 1024), (50, 1890, 2048), (64, 1984, 2048), (33, 1000, 2048)])
+def test_prompt_attention_in_clusters_of_every_size(gpu, pkg, rope_table, heads, batch, pos, max_ctx):
+    """Clusters are so small that all of them run at a time: 8, 6, 5, 4 and 4 CTAs for these heads on 148 SMs, with one to four passes of which the last is
+    partial.  Bounds as in test_prompt_attention."""
+    rng = np.random.default_rng(heads + pos)
+    dim = heads * ROT
+    k, v = (rng.standard_normal((max_ctx, dim), dtype=np.float32).astype(np.float16).view(np.uint16) for _ in range(2))
+    q = rng.standard_normal((batch, dim)).astype(np.float32)
+    scratch, d_out = gpu.zeros(gpu.lib.lv_attention_scratch_bytes(heads, ROT, max_ctx, batch)), gpu.zeros((batch + 1) * dim * 4)
+    args = [gpu.upload(a) for a in (q, k, v)]
+    pkg.check(gpu.lib.lv_attention_fused(gpu.handle, d_out, *args, u32_dev(gpu, pos), rope_table, scratch, heads, ROT, max_ctx, batch))
+    gpu.sync()
+    got = gpu.download(d_out, np.float32, (batch + 1) * dim).reshape(batch + 1, dim)
+    table = gpu.download(rope_table, np.float32, 2048 * ROT).reshape(2048, ROT // 2, 2)
+    for z in (0, 9, batch // 2 + 1, batch - 1):
+        close(got[z], exact_attention(table, k, v, q[z], pos + z), rel_l2=1e-5, max_abs_frac=2e-5)
+    assert not got[batch].any() and np.isfinite(got).all()
+    for d in args + [scratch, d_out]:
+        gpu.free(d)
+
+
 @pytest.mark.parametrize("batch,pos,max_ctx", [(12, 30, 128), (64, 300, 512), (64, 1900, 2048)])
 def test_attention_of_rows_that_are_not_aligned(gpu, pkg, rope_table, batch, pos, max_ctx):
     """Outputs 4 bytes behind a 16-byte boundary were always taken."""
