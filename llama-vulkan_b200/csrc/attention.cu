@@ -432,24 +432,23 @@ int attention_configure(lv_ctx* ctx) {
     return LV_OK;
 }
 
-// Whether lv_attention_fused takes the matrix products of attention_prompt.cu.  us in a chain of launches, one CTA per row, head and 256 positions here /
-// products there:
-//               32 heads                          8 heads                          4 heads
-//   rows    up to 128   450 of 512  1000 of 1024   up to 128   450 of 512  1000 of 1024   up to 128   450 of 512  1000 of 1024
-//      8     7.7          20 / 14     35 / 15       4.7          8 / 11      11 / 12       4.7         8            8 / 11
-//     12    12 / 9        28 / 14     48 / 15       4.9 / 8      11 / 11     17 / 12       4.8 / 8     8 / 11      11 / 11
-//     32    25 / 10       64 / 15    119 / 17       7.9 / 9      20 / 11     36 / 13       4.9 / 8    11 / 11      20 / 12
-//     64    47 / 14      123 / 23    233 / 25        15 / 13     36 / 16     63 / 18       8.1 / 13   20 / 16      36 / 16
-// (Taken with launches back to back, clusters of 8 and key rows by bulk copies.  Since then 64 rows of 32 heads at 1000 of 1024 take a second pass in clusters of 7:
-// 38 us between the launches of a session, where clusters of 8 took 44; the kernel here is 5 to 30 % faster, most with many CTAs.)
+// Whether lv_attention_fused takes the matrix products of attention_prompt.cu.  us behind a copy that passes through L2, one CTA per row, head and 256 positions
+// here / products there, at positions beyond half of the context, as sessions have them:
+//               32 heads                                16 heads                                8 heads
+//   rows    100 of 128  200 of 256  450 of 512  937 of 1024   of 128      of 256      of 512      of 1024     of 128      of 256      of 512      of 1024
+//      8     6.1 / 11    8.6 / 13    20 / 15     33 / 25       5.3 / 11    5.8 / 12    11 / 13     19 / 15     5.0 / 11    5.6 / 12    8.1 / 12    11 / 13
+//     12     9.5 / 12     13 / 13    27 / 15     46 / 25       5.9 / 11    8.3 / 13    18 / 13     27 / 15     5.1 / 11    5.6 / 12    10 / 12     17 / 13
+//     16      11 / 12     16 / 14    34 / 15     59 / 25       6.1 / 11    8.6 / 13    19 / 14     33 / 15     5.1 / 11    5.7 / 12    11 / 13     19 / 14
+//     32      20 / 13     28 / 15    61 / 16    111 / 27        11 / 13     16 / 14    34 / 14     59 / 16     6.3 / 12    8.8 / 14    19 / 14     33 / 14
+//     64      34 / 19     53 / 22   117 / 24    215 / 39        19 / 18     28 / 21    62 / 22    112 / 24      11 / 17     16 / 20    35 / 19     59 / 22
 // The kernel here runs up to two CTAs per SM at a time; below that it is as fast or faster, and exact in the angles (grids of one CTA per SM), so the line lies
-// where its CTAs are more than two per SM, three for steps of more than 32 rows, whose products take half as long again, and five where the products
-// take several passes (more than 1024 positions: 12 rows of 4 heads at 1100 of 2048 11 / 20, 16 rows of 8 heads 25 / 20).  (Measured at positions beyond
-// half of the context, as sessions have them; 12 rows of 16 heads at 200 of 512 take 9 / 13.)  Steps of fewer than twelve rows only with more
-// than 512 positions: at 200 of 512, 32 heads, 8 rows take 9.4 / 14.  The products store 16 bytes at a time.
+// where its CTAs are more than two per SM, and three for steps of more than 32 rows, whose products take half as long again.  One more of each in contexts of up to
+// 256 positions, where its CTAs are short (a third of an SM's time at 100 positions), and five where the products take several passes (more than 1024: 24 rows of 4
+// heads at 1500 of 2048 21 / 23, 16 rows of 8 heads 28 / 24).  Steps of fewer than twelve rows only with more than 512 positions: at 450 of 512 eight rows of 32
+// heads would gain, at 200 of 512 they take 9.4 / 14.  The products store 16 bytes at a time.
 static bool use_prompt_attention(const lv_ctx* ctx, const void* out, uint32_t heads, uint32_t nchunks, uint32_t max_ctx, uint32_t batch) {
     if (batch < 8 || (batch < 12 && max_ctx <= 512) || (reinterpret_cast<uintptr_t>(out) & 15u) != 0) return false;
-    return size_t(heads) * nchunks * batch > size_t(max_ctx > 1024 ? 5 : batch > 32 ? 3 : 2) * ctx->sm_count;
+    return size_t(heads) * nchunks * batch > size_t(max_ctx > 1024 ? 5 : (batch > 32 ? 3 : 2) + (nchunks == 1 ? 1 : 0)) * ctx->sm_count;
 }
 
 // Grids of at most one CTA per SM stage key rows and the exact table rows in shared memory; larger

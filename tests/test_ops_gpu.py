@@ -386,7 +386,8 @@ def test_fused_attention_batch_is_causal(gpu, pkg, rope_table):
 
 
 @pytest.mark.parametrize("batch,pos,max_ctx", [(12, 0, 128), (64, 0, 128), (16, 120, 256), (17, 111, 128), (64, 64, 128), (33, 300, 512), (64, 512, 1024), (50, 974, 1024),
-                                               (9, 1015, 2048), (64, 1984, 2048), (63, 1985, 2048), (70, 90, 256), (130, 640, 1024), (12, 19, 31)])
+                                               (9, 1015, 2048), (64, 1984, 2048), (63, 1985, 2048), (70, 90, 256), (130, 640, 1024), (12, 19, 31),
+                                               (13, 100, 128), (14, 0, 128), (14, 16, 31), (18, 238, 256), (19, 1, 257)])
 def test_prompt_attention(gpu, pkg, rope_table, batch, pos, max_ctx):
     """Steps of many rows go through the matrix products of attention_prompt.cu: chunks of 128 keys that end inside a block of 16, one or
     several CTAs and passes per head, one or several tiles of 64 rows.  Bounds as for the compact table of test_fused_attention: the angle of
