@@ -79,6 +79,14 @@ def test_download_through_either_way(gpu, pkg, nbytes):
     d, got = gpu.upload(data), np.full(nbytes + 2, 7, np.uint8)
     pkg.check(gpu.lib.lv_download(gpu.handle, C.c_void_p(got.ctypes.data + 1), pkg.offset(d, 1), nbytes))
     assert np.array_equal(got[1:-1], data[1:]) and got[0] == 7 and got[-1] == 7
+    pinned = C.c_void_p()
+    pkg.check(gpu.lib.lv_host_alloc(gpu.handle, nbytes + 2, C.byref(pinned)))
+    got = np.frombuffer((C.c_uint8 * (nbytes + 2)).from_address(pinned.value), np.uint8)
+    got[:] = 7
+    pkg.check(gpu.lib.lv_download(gpu.handle, pkg.offset(pinned, 1), pkg.offset(d, 1), nbytes))
+    assert np.array_equal(got[1:-1], data[1:]) and got[0] == 7 and got[-1] == 7
+    del got
+    pkg.check(gpu.lib.lv_host_free(gpu.handle, pinned))
     gpu.free(d)
 
 
