@@ -136,9 +136,9 @@ __host__ __device__ inline size_t attn_partial_floats(uint32_t heads, uint32_t n
 //
 // The kernel is a short chain of dependent steps on little data, so each step
 // issues all of its global loads before using any of them (one trip to L2 per
-// step): scores with 8 lanes per cache row (16 elements each, both of a warp's
-// row batches in flight together), values with 16 threads per row (8 dims each)
-// and four rows per thread in flight.
+// step): scores with 8 lanes per cache row (16 elements each, four passes of four
+// rows per warp), values with 16 threads per row (8 dims each) and up to eight rows
+// per thread in flight.
 // Shared-memory staging of the score inputs: the rows of the rotation table that the chunk needs are brought in by bulk (TMA)
 // copies, its key rows 16 bytes per thread, and the scores are computed from shared memory.  With
 // plain loads the kernel spent a fifth of its samples throttled on the load/store queue (28 16-byte

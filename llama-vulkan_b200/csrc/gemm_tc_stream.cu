@@ -25,9 +25,10 @@
 //   19     activation ring: one bulk copy per two tiles of K (q8_0, whose raw stages are larger: one).  The number of stages is even, so that
 //          a stage always belongs to one issuing lane (a parity wait cannot tell a phase from the one two uses later).
 //
-// us per launch back to back, 16 / 64 tokens of q4_0: 11008 x 4096 pair 26.3 / 29.5, 4096 x 11008 16.9 / 19.3, 4096 x 4096 9.5 / 11.9 (q8_0 28.0 / 32.3,
-// 18.5 / 20.7, 10.5 / 12.5).  When every CTA reported its parts at its end, the last one read all of them back, and the epilogues were unrolled code that
-// runs once (instruction fetches: 12 us of a whole pair tile), these took 35.8 / 43.5, 17.5 / 20.3, 10.7 / 12.4 (38.2 / 46.5, 18.9 / 23.4, 12.0 / 13.7).
+// us per launch back to back, 16 / 64 tokens of q4_0: 11008 x 4096 pair 27.3 / 30.5, 4096 x 11008 17.2 / 19.7, 4096 x 4096 9.5 / 11.8 (q8_0 28.6 / 33.7,
+// 18.5 / 20.7, 10.5 / 12.4).  When every CTA reported its parts at its end, the last one read all of them back, and the epilogues were unrolled code that
+// runs once (instruction fetches: 12 us of a whole pair tile), these took 35.8 / 43.5, 17.4 / 20.2, 10.7 / 12.5 (38.0 / 46.5, 18.9 / 22.9, 12.0 / 13.7).
+// 1.7 % (0 to 4) of the present times is the price of giving a wait up in order: a producer's two votes per unit 1.1, the last barrier that collects them 0.6.
 // A unit takes about 1700 clocks: 700 of dequantisation, 450 of waiting for and fetching raw words, 90 of tcgen05.st, the rest loop, barriers
 // and drains; the tensor pipe needs 1024 of them at 64 tokens.
 //
@@ -563,14 +564,14 @@ static int launch_typed(lv_ctx* ctx, const GemmTcParams& p, const GemmTcMaps& ma
     plan.groups = p.K / (4 * kTcChunkK);
     plan.units = tiles * plan.groups;
     const uint32_t sms = uint32_t(ctx->sm_count);
-    // equal runs; at least two units each, since a part costs about as much as two units
+    // Equal runs; at least two units each (one instead of two: 2048 x 2048 6.7 -> 8.4 us, 512 x 5632 9.9 -> 13.3).
     plan.per = max((plan.units + sms - 1) / sms, min(2u, plan.groups));
     // Runs that begin and end inside tiles have two segments, and tiles up to eight parts: about two units more for the CTA that ends last.  Where
     // equal shares of every tile fit the SMs with no more units than that, each CTA has one segment.  us per launch back to back, q4_0, runs -> shares:
-    //   tokens   2048 x 5632    3 x 2048 x 2048   5120 x 5120    4096 x 11008    1408 x 4096 pair
-    //     16     11.6 -> 10.2   10.3 ->  9.5      13.0 -> 12.3   17.5 -> 17.5    10.9 ->  9.9
-    //     64     18.4 -> 13.1   14.9 -> 11.7      17.7 -> 14.3   24.0 -> 20.3    17.3 -> 12.6
-    // and a prompt of 512 tokens in steps of 64, four layers 2048 wide: 3.31 -> 3.05 ms.
+    //   tokens   2048 x 5632    3 x 2048 x 2048   5120 x 5120    4096 x 11008    1408 x 4096 pair   8192 x 4096     (three units more:) 5120 x 13824   6656 x 6656
+    //     16     10.4 ->  9.7    9.2 ->  8.9      12.3 -> 12.1   17.6 -> 17.3    10.2 ->  9.9       13.9 -> 13.6                        22.9 -> 24.2    16.6 -> 18.1
+    //     64     13.6 -> 12.6   11.5 -> 10.8      14.8 -> 14.3   20.9 -> 19.8    13.1 -> 12.5       16.7 -> 15.6                        26.3 -> 26.8    19.7 -> 20.2
+    // and the same in q8_0.
     const uint32_t most = sms / tiles, n_shares = most == 0 ? 0 : max((plan.groups + most - 1) / most, min(2u, plan.groups));      // units of a CTA
     if (most > 1 && plan.groups % plan.per != 0 && n_shares <= plan.per + 2) plan.shares = (plan.groups + n_shares - 1) / n_shares;
     // whole tiles only, where the arrival counters or the scratch (two parts per CTA) would not do
