@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
     };
 
     bool ok = true;
+    uint32_t raw_issued = 0, b_issued = 0;                 // the TMA lane's copies; b_issued of the MMA lane: stages whose products it has issued
 
     if (warp == kTcProducerWarps) {
         // ---------------- TMA warp: one lane feeds the raw ring and the B tiles ----------------
@@ -233,6 +234,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
                     else if (clock64() - t_idle > kWaitCycleLimit) { atomicOr(p.err, ERR_MBAR_TIMEOUT); ok = false; }
                 }
             }
+            raw_issued = g_next;
+            b_issued = c_next;
         }
     } else if (warp == kTcProducerWarps + 1) {
         // ---------------- MMA warp: one lane issues all tensor-core work ---------------------------
@@ -263,6 +266,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
                             tc_mma_f16(bank, a_desc + 2u * k, b_desc + 2u * k, idesc_wide, acc);
                         }
                         tc_commit(&b_empty[bs]);
+                        ++b_issued;
                         a_desc += uint32_t(kTcTileBytes) >> 4;
                         if (++bs == nb) { bs = 0; b_phase ^= 1u; }
                     }
@@ -286,6 +290,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
                 }
                 tc_commit(&slot_empty[s]);                                   // arrive when these MMAs have read the tiles
                 tc_commit(&b_empty[bs]);
+                ++b_issued;
                 if (++bs == nb) { bs = 0; b_phase ^= 1u; }
             }
             }
@@ -593,7 +598,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
         }
     }
     tc_fence_before_sync();
-    __syncthreads();
+    if (__syncthreads_or(!ok)) {
+        // a wait was lost: copies and products that are on their way end before shared and tensor memory are given back
+        if (lane == 0 && warp == kTcProducerWarps) {
+            for (uint32_t s = 0; s < min(raw_issued, uint32_t(kTcRawStages)); ++s) mbar_drain(&raw_full[s], ((raw_issued - 1 - s) / kTcRawStages) & 1u);
+            for (uint32_t s = 0; s < min(b_issued, nb); ++s) mbar_drain(&b_full[s], ((b_issued - 1 - s) / nb) & 1u);
+        } else if (lane == 0 && warp == kTcProducerWarps + 1 && b_issued != 0) {
+            mbar_drain(&b_empty[(b_issued - 1) % nb], ((b_issued - 1) / nb) & 1u);
+        }
+        __syncthreads();
+    }
     if (warp == kTcProducerWarps + 1) {
         tc_fence_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
