@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
             const uint32_t fr = uint32_t(warp) * 8u + (uint32_t(lane) & 7u), ft = uint32_t(lane) >> 3;
             for (uint32_t g = 0; g < n_groups && ok; ++g) {
                 const int rs = int(g % kTcRawStages);
-                ok = mbar_wait(&raw_full[rs], (g / kTcRawStages) & 1u, p.err);
+                ok = mbar_wait_all(&raw_full[rs], (g / kTcRawStages) & 1u, p.err);
                 if (!ok) break;
                 uint32_t w[9];
                 {
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
                 if (lane == 0) mbar_arrive(&raw_empty[rs]);
                 const uint32_t ab = g % kTcFastBufs;
                 if (g >= uint32_t(kTcFastBufs)) {
-                    ok = mbar_wait(&slot_empty[ab], ((g / kTcFastBufs) - 1) & 1u, p.err);
+                    ok = mbar_wait_all(&slot_empty[ab], ((g / kTcFastBufs) - 1) & 1u, p.err);
                     if (!ok) break;
                 }
                 uint8_t* a_tile = slots + ab * kTcFastBufBytes + ft * kTcTileBytes;
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
         const uint32_t jpar = threadIdx.x >> 8;               // producer group: even or odd tiles of K
         for (uint32_t g = 0; g < n_groups && ok; ++g) {
             const int rs = int(g % kTcRawStages);
-            ok = mbar_wait(&raw_full[rs], (g / kTcRawStages) & 1u, p.err);
+            ok = mbar_wait_all(&raw_full[rs], (g / kTcRawStages) & 1u, p.err);
             if (!ok) break;
             // the two tiles of this group that the thread's producer group owns (tiles jpar and jpar + 2 of the
             // four): kTileWords words each, taken out of the row with 16-byte loads
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
                 const uint32_t c = g * 4 + jpar + 2 * jj;
                 const int s = int(c % kTcSlots);
                 if (c >= kTcSlots) {
-                    ok = mbar_wait(&slot_empty[s], ((c / kTcSlots) - 1) & 1u, p.err);
+                    ok = mbar_wait_all(&slot_empty[s], ((c / kTcSlots) - 1) & 1u, p.err);
                     if (!ok) break;
                 }
                 // even block of the tile: scale in the low half of word 0, payload shifted by two bytes;
@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const GemmTcPara
         uint32_t* s_last = tmem_slot + 1;
         if (warp < 4) {
             pdl_wait();
-            if (ok) ok = mbar_wait(acc_full, 0u, p.err);
+            if (ok) ok = mbar_wait_all(acc_full, 0u, p.err);
             tc_fence_after_sync();
             float* gate_s = reinterpret_cast<float*>(slots);      // [64][17] floats, free once the accumulator is complete
             const uint32_t tr = uint32_t(warp * 32 + lane);       // tile row
